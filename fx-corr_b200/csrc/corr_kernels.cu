@@ -351,19 +351,66 @@ __global__ void __launch_bounds__(FPC * N / 16, MINB) corr_batch_kernel(const Ba
 // Fixed-order sum of the per-CTA partials.  The multipliers (exact powers of
 // two) undo the two-for-one 2x factor of each spectrum and the per-station
 // level scaling.  Writes acf11, acf22, xcf (re,im) and zeroes the phased slot.
-// A 256-thread block covers 32 bins: each of its 8 warps sums one contiguous
-// eighth of the slots in slot order (coalesced 256-byte rows), then the eight
-// warp sums are added in warp order; the order depends only on nblk, so the
-// result is deterministic.
-constexpr int kRedBins = 32, kRedGroups = 8;
+// A block covers 32 bins: each of its warps sums a contiguous share of the
+// slots in slot order (coalesced 256-byte rows), then the warp sums are added
+// in warp order; the order depends only on nblk, so the result is
+// deterministic.  Bound by the latency of the slots' loads, a serial chain per
+// warp: many slots take 32 warps and a block per column, so that a warp has all
+// its loads (ten of 296 slots) in flight at once.  8 warps with all four
+// columns took 40 us at the 296 slots of FFT 1024..4096 and 21 us at the 148 of
+// FFT 8192; 32 warps take 7.4 and 10.1 us.  At the 33 slots of FFT 65536 it is
+// the other way round: 9.4 us with 8 warps, 15 us with a block per column.
+constexpr int kRedBins = 32;
+constexpr int kRedWideSlots = 64;
 
-__global__ void __launch_bounds__(kRedBins * kRedGroups)
+// The sum of this thread's column and bin; in warp 0 only.
+template <int WARPS>
+__device__ __forceinline__ double reduce_column(const double* __restrict__ part, int nblk,
+                                                size_t stride, int k, bool in,
+                                                double (&sm)[WARPS][kRedBins]) {
+  const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
+  const int b0 = (nblk * grp) / WARPS, b1 = (nblk * (grp + 1)) / WARPS;
+  double s = 0.0;
+  if (in) {
+    const double* q = part + (size_t)b0 * stride + k;
+#pragma unroll 10
+    for (int b = b0; b < b1; ++b, q += stride) s += *q;
+  }
+  sm[grp][lane] = s;
+  __syncthreads();
+  double t = 0.0;
+  if (grp == 0) {
+#pragma unroll
+    for (int g = 0; g < WARPS; ++g) t += sm[g][lane];
+  }
+  return t;
+}
+
+__device__ __forceinline__ void reduce_store(int v, int k, int h, double t, double m11, double m22,
+                                             double m12, double* __restrict__ out) {
+  if (v < 2) out[(size_t)v * h + k] = (v ? m22 : m11) * t;
+  else out[2 * (size_t)h + 2 * k + (v - 2)] = m12 * t;
+  if (v == 0) out[4 * (size_t)h + k] = 0.0;
+}
+
+// One column per block (blockIdx.y), 32 warps.
+__global__ void __launch_bounds__(kRedBins * 32)
+reduce_partials_wide_kernel(const double* __restrict__ part, int nblk, int h, double m11,
+                            double m22, double m12, double* __restrict__ out) {
+  __shared__ double sm[32][kRedBins];
+  const int k = blockIdx.x * kRedBins + (threadIdx.x & 31), v = blockIdx.y;
+  const double t = reduce_column<32>(part + (size_t)v * h, nblk, (size_t)4 * h, k, k < h, sm);
+  if (threadIdx.x < kRedBins && k < h) reduce_store(v, k, h, t, m11, m22, m12, out);
+}
+
+// All four columns per block, 8 warps.
+__global__ void __launch_bounds__(kRedBins * 8)
 reduce_partials_kernel(const double* __restrict__ part, int nblk, int h, double m11, double m22,
                        double m12, double* __restrict__ out) {
-  __shared__ double sm[kRedGroups][4][kRedBins];
+  __shared__ double sm[8][4][kRedBins];
   const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
   const int k = blockIdx.x * kRedBins + lane;
-  const int b0 = (nblk * grp) / kRedGroups, b1 = (nblk * (grp + 1)) / kRedGroups;
+  const int b0 = (nblk * grp) / 8, b1 = (nblk * (grp + 1)) / 8;
   double s[4] = {0, 0, 0, 0};
   if (k < h) {
     for (int b = b0; b < b1; ++b) {
@@ -376,16 +423,23 @@ reduce_partials_kernel(const double* __restrict__ part, int nblk, int h, double 
   for (int v = 0; v < 4; ++v) sm[grp][v][lane] = s[v];
   __syncthreads();
   if (grp != 0 || k >= h) return;
-  double t[4] = {0, 0, 0, 0};
 #pragma unroll
-  for (int g = 0; g < kRedGroups; ++g)
+  for (int v = 0; v < 4; ++v) {
+    double t = 0.0;
 #pragma unroll
-    for (int v = 0; v < 4; ++v) t[v] += sm[g][v][lane];
-  out[k] = m11 * t[0];
-  out[h + k] = m22 * t[1];
-  out[2 * h + 2 * k] = m12 * t[2];
-  out[2 * h + 2 * k + 1] = m12 * t[3];
-  out[4 * h + k] = 0.0;
+    for (int g = 0; g < 8; ++g) t += sm[g][v][lane];
+    reduce_store(v, k, h, t, m11, m22, m12, out);
+  }
+}
+
+// Fixed-order sum of the per-CTA phased partials into acc[4H, 5H).
+template <int WARPS>
+__global__ void __launch_bounds__(kRedBins * WARPS)
+reduce_phased_kernel(const double* __restrict__ part, int nblk, int h, double* __restrict__ out) {
+  __shared__ double sm[WARPS][kRedBins];
+  const int k = blockIdx.x * kRedBins + (threadIdx.x & 31);
+  const double t = reduce_column<WARPS>(part, nblk, (size_t)h, k, k < h, sm);
+  if (threadIdx.x < kRedBins && k < h) out[4 * (size_t)h + k] = t;
 }
 
 __global__ void delay_entries_kernel(const DelayParams p, uint64_t first, uint64_t nf,
@@ -628,8 +682,21 @@ cudaError_t launch_batch_reduce(const BatchArgs& a, int grid, cudaStream_t s) {
 
 cudaError_t launch_reduce(const double* part, int nblk, int h, double m11, double m22, double m12,
                           double* out, cudaStream_t s) {
-  reduce_partials_kernel<<<(h + kRedBins - 1) / kRedBins, kRedBins * kRedGroups, 0, s>>>(
-      part, nblk, h, m11, m22, m12, out);
+  const int grid = (h + kRedBins - 1) / kRedBins;
+  if (nblk >= kRedWideSlots)
+    reduce_partials_wide_kernel<<<dim3(grid, 4), kRedBins * 32, 0, s>>>(part, nblk, h, m11, m22,
+                                                                        m12, out);
+  else
+    reduce_partials_kernel<<<grid, kRedBins * 8, 0, s>>>(part, nblk, h, m11, m22, m12, out);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_reduce_phased(const double* part, int nblk, int h, double* out, cudaStream_t s) {
+  const int grid = (h + kRedBins - 1) / kRedBins;
+  if (nblk >= kRedWideSlots)
+    reduce_phased_kernel<32><<<grid, kRedBins * 32, 0, s>>>(part, nblk, h, out);
+  else
+    reduce_phased_kernel<8><<<grid, kRedBins * 8, 0, s>>>(part, nblk, h, out);
   return cudaGetLastError();
 }
 

@@ -331,28 +331,6 @@ phased_batch_kernel(const BatchArgs a, int grp) {
   phased_cta_drain(smem, L);
 }
 
-// Fixed-order sum of the per-CTA phased partials into acc[4H, 5H).
-// (32 bins per block; each of 8 warps sums a contiguous eighth of the slots in
-// slot order, the warp sums are added in warp order: deterministic.)
-__global__ void __launch_bounds__(256) reduce_phased_kernel(const double* __restrict__ part,
-                                                            int nblk, int h,
-                                                            double* __restrict__ out) {
-  __shared__ double sm[8][32];
-  const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
-  const int k = blockIdx.x * 32 + lane;
-  const int b0 = (nblk * grp) / 8, b1 = (nblk * (grp + 1)) / 8;
-  double s = 0.0;
-  if (k < h)
-    for (int b = b0; b < b1; ++b) s += part[(size_t)b * h + k];
-  sm[grp][lane] = s;
-  __syncthreads();
-  if (grp != 0 || k >= h) return;
-  double t = 0.0;
-#pragma unroll
-  for (int g = 0; g < 8; ++g) t += sm[g][lane];
-  out[4 * h + k] = t;
-}
-
 template <int N, int FPC>
 static cudaError_t launch_phased_one(const PhasedParams& p, int grid, cudaStream_t stream) {
   const uint32_t smem = smem_layout<N, FPC>(p.stage_bytes).total + 1024 + 4096;
@@ -439,11 +417,6 @@ cudaError_t launch_phased_batch(uint32_t n, const BatchArgs& a, int grp, int gri
     case 16384: return launch_phased_pair_batch(a, grp, grid, s);
     default: return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
-}
-
-cudaError_t launch_reduce_phased(const double* part, int nblk, int h, double* out, cudaStream_t s) {
-  reduce_phased_kernel<<<(h + 31) / 32, 256, 0, s>>>(part, nblk, h, out);
   return cudaGetLastError();
 }
 
