@@ -6,7 +6,8 @@
 // of `item_frames` frames (at most one per persistent CTA), uploads the
 // tables in one copy and runs
 //   batch_frame_info_kernel  the FP64 delay records of every frame,
-//   one persistent kernel per FFT length present (tickets over its items),
+//   one persistent kernel per FFT length present (tickets over its items), side
+//   by side,
 //   batch_reduce_kernel      every sector's partials in item order,
 // either launched directly or as a CUDA graph captured once per set of FFT
 // lengths (the kernels read every count from the uploaded header, so one
@@ -72,6 +73,7 @@ struct Shape {
   int ctas = 0;  // resident CTAs per SM of the variant
   double gsps = 0.0;
   bool tuned = false;
+  bool pinned = false;  // the caller's item size: kept for every sector
 };
 
 }  // namespace
@@ -100,6 +102,8 @@ struct fxc_batch {
   uint64_t charged = 0;
   cudaEvent_t ev_done = nullptr;    // the last call's device work
   cudaStream_t cap_stream = nullptr;
+  cudaStream_t side[kBatchGroups] = {};  // a call's groups run side by side
+  cudaEvent_t ev_fork = nullptr, ev_join[kBatchGroups] = {};
   std::map<uint64_t, cudaGraphExec_t> execs;  // by group set and variants
   std::mutex mu;
   uint64_t launches = 0;
@@ -208,10 +212,24 @@ struct Entry {
 };
 
 // Frames per item of a sector: the group's item size, enlarged so that a
-// sector has at most one item per resident CTA, rounded to whole CTA iterations.
-uint64_t item_len(const Shape& sh, int sms, uint64_t nf) {
+// sector has at most one item per resident CTA and, unless the caller set it,
+// reduced to a part of a short sector (but at least 2^15 samples per station),
+// rounded to whole CTA iterations.  A call takes at least as long as its
+// longest item: 128 frames of FFT 4096 phased are 1.8 ms on one CTA while the
+// rest of the GPU has run out of items.  An item costs 2-4 us beyond its frames
+// (tables, first copy) and writes 16 N bytes of partials, which the reduction
+// reads.  24 sectors of 2^21 samples, FFT 1024 / 4096 / 16384, correlation and
+// phased: 4820 us a call with 128-frame items one group after another, 736 us
+// with 16 items a sector and the groups side by side, 583 with 24, 519 with 32;
+// 64 sectors of FFT 8192, 125-2000 frames: 2766 us with 64-frame items, 2776
+// with 16, 2753 with 24, 2792 with 32 (the partials).  So 24 for correlation
+// and, four times smaller partials, 32 for phased sectors.  Only the sector's
+// own length counts, so that its sums do not depend on what else is in the call.
+uint64_t item_len(const Shape& sh, int g, int sms, uint64_t nf, bool exact) {
   const uint64_t maxn = (uint64_t)std::max(1, sms * sh.ctas);
   uint64_t per = sh.item_frames;
+  const uint64_t parts = phased_group(g) ? 32 : 24;
+  if (!exact) per = std::min(per, std::max<uint64_t>((nf + parts - 1) / parts, 32768 / kGroupN[g]));
   if ((nf + per - 1) / per > maxn) per = (nf + maxn - 1) / maxn;
   return align_up(per, (uint64_t)sh.fpc);
 }
@@ -396,6 +414,10 @@ fxc_status run_batch(fxc_batch* b, fxc_scan* const* scans, const uint8_t* const*
       fxc_status st = set_shape(b, g, b->shape[g].fpc, b->shape[g].item_frames);
       if (st != FXC_OK) return st;
     }
+    if (!b->side[g]) {
+      BCK(cudaStreamCreateWithFlags(&b->side[g], cudaStreamNonBlocking));
+      BCK(cudaEventCreateWithFlags(&b->ev_join[g], cudaEventDisableTiming));
+    }
   }
   // table order: by group, then call order; items follow the same order
   std::stable_sort(ents.begin(), ents.end(),
@@ -410,7 +432,7 @@ fxc_status run_batch(fxc_batch* b, fxc_scan* const* scans, const uint8_t* const*
       if (e.group != g) continue;
       const Shape& sh = b->shape[g];
       const uint64_t n = e.bs.p.nf;
-      const uint64_t per = item_len(sh, b->sms, n);
+      const uint64_t per = item_len(sh, g, b->sms, n, sh.pinned || b->tuning[g]);
       const uint32_t nparts = (uint32_t)((n + per - 1) / per);
       const uint64_t h = e.bs.h;
       const uint64_t slot = phased_group(g) ? h : 4 * h;  // partial doubles per item
@@ -466,18 +488,28 @@ fxc_status run_batch(fxc_batch* b, fxc_scan* const* scans, const uint8_t* const*
       const uint64_t fgrid = full ? (uint64_t)grid_aux
                                   : std::min<uint64_t>((uint64_t)grid_aux, (hdr.nframes + 127) / 128);
       BCK(launch_batch_frame_info(a, (int)std::max<uint64_t>(fgrid, 1), s));
-      for (int g = 0; g < kBatchGroups; ++g) {
+      // The groups' kernels are independent: one stream each, so that the end
+      // of one (its last items on a few SMs) runs beside the next instead of
+      // before it.  The slowest per frame first: phased, then by FFT length.
+      const bool fork = (mask & (mask - 1u)) != 0;
+      if (fork) BCK(cudaEventRecord(b->ev_fork, s));
+      for (int g = kBatchGroups - 1; g >= 0; --g) {
         if (!(mask & (1u << g))) continue;
         const Shape& sh = b->shape[g];
         uint64_t grid = (uint64_t)b->sms * sh.ctas;
         if (!full) grid = std::min<uint64_t>(grid, hdr.nitems[g]);
+        const cudaStream_t gs = fork ? b->side[g] : s;
+        if (fork) BCK(cudaStreamWaitEvent(gs, b->ev_fork, 0));
         if (phased_group(g))
-          BCK(launch_phased_batch(kGroupN[g], a, g, (int)std::max<uint64_t>(grid, 1), s));
+          BCK(launch_phased_batch(kGroupN[g], a, g, (int)std::max<uint64_t>(grid, 1), gs));
         else
-          BCK(launch_batch_group(g, sh.fpc, a, (int)std::max<uint64_t>(grid, 1), s));
+          BCK(launch_batch_group(g, sh.fpc, a, (int)std::max<uint64_t>(grid, 1), gs));
+        if (fork) BCK(cudaEventRecord(b->ev_join[g], gs));
       }
+      for (int g = 0; fork && g < kBatchGroups; ++g)
+        if (mask & (1u << g)) BCK(cudaStreamWaitEvent(s, b->ev_join[g], 0));
       const uint64_t rgrid = full ? (uint64_t)grid_aux
-                                  : std::min<uint64_t>((uint64_t)grid_aux, (hdr.nbins + 255) / 256);
+                                  : std::min<uint64_t>((uint64_t)grid_aux, (4 * hdr.nbins + 255) / 256);
       BCK(launch_batch_reduce(a, (int)std::max<uint64_t>(rgrid, 1), s));
       return FXC_OK;
     };
@@ -559,6 +591,7 @@ fxc_status fxc_batch_create(fxc_engine* e, const fxc_batch_opts* opts, fxc_batch
   for (int g = 0; g < kBatchGroups; ++g) {
     b->shape[g].fpc = kDefaultFpc[g];
     b->shape[g].item_frames = b->item_override ? b->item_override : kDefaultItems[g];
+    b->shape[g].pinned = b->item_override != 0;
   }
   DeviceGuardB dg(b->device);
   auto bail = [&](cudaError_t err) {
@@ -571,6 +604,7 @@ fxc_status fxc_batch_create(fxc_engine* e, const fxc_batch_opts* opts, fxc_batch
   if ((err = cudaEventCreateWithFlags(&b->arena[0].staged, cudaEventDisableTiming)) != cudaSuccess ||
       (err = cudaEventCreateWithFlags(&b->arena[1].staged, cudaEventDisableTiming)) != cudaSuccess ||
       (err = cudaEventCreateWithFlags(&b->ev_done, cudaEventDisableTiming)) != cudaSuccess ||
+      (err = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming)) != cudaSuccess ||
       (err = cudaStreamCreateWithFlags(&b->cap_stream, cudaStreamNonBlocking)) != cudaSuccess)
     return bail(err);
   engine_track_batch(e, b, true);
@@ -592,6 +626,11 @@ fxc_status fxc_batch_destroy(fxc_batch* b) {
   cudaFree(b->d_part);
   engine_release(b->eng, b->charged);
   if (b->ev_done) cudaEventDestroy(b->ev_done);
+  if (b->ev_fork) cudaEventDestroy(b->ev_fork);
+  for (int g = 0; g < kBatchGroups; ++g) {
+    if (b->side[g]) cudaStreamDestroy(b->side[g]);
+    if (b->ev_join[g]) cudaEventDestroy(b->ev_join[g]);
+  }
   if (b->cap_stream) cudaStreamDestroy(b->cap_stream);
   delete b;
   return FXC_OK;
@@ -668,6 +707,7 @@ fxc_status fxc_batch_set_shape(fxc_batch* b, uint32_t fft_len, int32_t fpc,
   fxc_status st = set_shape(b, g, fpc, item_frames);
   if (st != FXC_OK) return st;
   b->shape[g].tuned = true;  // pinned: the first-use tuner leaves it
+  b->shape[g].pinned = true;
   b->shape[g].gsps = 0.0;
   return FXC_OK;
 }

@@ -447,6 +447,7 @@ template <int ROWS>
 __global__ void __launch_bounds__(kT, 1) corr_fold_batch_kernel(const BatchArgs a, int grp) {
   extern __shared__ __align__(128) uint8_t smem[];
   const FoldLayout L = fold_layout(2u * (uint32_t)(kN * ROWS));
+  if (blockIdx.x >= a.hdr->nitems[grp]) return;  // a graph launches the full grid
   uint32_t* ticket = reinterpret_cast<uint32_t*>(smem + kOffFlag + 4);
   FoldCta<ROWS> c;
   fold_cta_init<ROWS>(smem, c);

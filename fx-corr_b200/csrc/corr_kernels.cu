@@ -327,6 +327,7 @@ template <int N, int FPC, int MINB>
 __global__ void __launch_bounds__(FPC * N / 16, MINB) corr_batch_kernel(const BatchArgs a, int grp) {
   extern __shared__ __align__(128) uint8_t smem[];
   const SmemLayout L = smem_layout<N, FPC>(2u * FPC * N);
+  if (blockIdx.x >= a.hdr->nitems[grp]) return;  // a graph launches the full grid
   uint32_t* ticket = reinterpret_cast<uint32_t*>(smem + L.off_flag + 4);
   Twiddles<N> tw;
   corr_cta_init<N, FPC>(L, smem, tw);
@@ -501,41 +502,35 @@ __global__ void batch_frame_info_kernel(const BatchArgs a) {
   }
 }
 
-// Fixed-order sum of each sector's item partials (grid-stride over all bins
-// of the batch), with the same multipliers and output layout as
-// reduce_partials_kernel (a phased sector: its power in [4H, 5H), the
+// Fixed-order sum of each sector's item partials (grid-stride over all columns
+// and bins of the batch, one thread each: a serial chain of loads per thread,
+// so the more threads the better), with the same multipliers and output layout
+// as reduce_partials_kernel (a phased sector: its power in [4H, 5H), the
 // correlation columns zero, as reduce_phased_kernel after a zeroed block).
 __global__ void batch_reduce_kernel(const BatchArgs a) {
   const uint32_t ns = a.hdr->nscans;
-  const uint64_t total = a.hdr->nbins;
+  const uint64_t total = 4 * a.hdr->nbins;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; x < total; x += stride) {
-    const BatchScan& b = a.hdr->scans[batch_find(a.hdr->scans, ns, x, true)];
-    const uint64_t k = x - b.bin0;
-    const uint64_t h = b.h;
-    const double* q = a.partials + b.part + k;
+    const BatchScan& b = a.hdr->scans[batch_find(a.hdr->scans, ns, x >> 2, true)];
+    const uint32_t h = b.h, r = (uint32_t)(x - 4 * b.bin0);
+    const uint32_t v = r / h, k = r % h;
     double* out = b.acc;
+    const size_t slot = b.phased ? h : 4 * (size_t)h;
+    const double* q = a.partials + b.part + (b.phased ? k : r);
+    double t = 0.0;
+    if (!b.phased || v == 0) {
+#pragma unroll 8
+      for (uint32_t i = 0; i < b.nparts; ++i, q += slot) t += *q;
+    }
     if (b.phased) {
-      // phased power: H partials per item, summed in item order
-      double t = 0.0;
-      for (uint32_t i = 0; i < b.nparts; ++i, q += h) t += *q;
-      out[k] = 0.0;
-      out[h + k] = 0.0;
-      out[2 * h + 2 * k] = 0.0;
-      out[2 * h + 2 * k + 1] = 0.0;
-      out[4 * h + k] = t;
-      continue;
+      // phased power: H partials per item
+      if (v == 0) out[4 * (size_t)h + k] = t;
+      else if (v == 1) out[k] = out[h + k] = 0.0;
+      else if (v == 2) out[2 * (size_t)h + 2 * k] = out[2 * (size_t)h + 2 * k + 1] = 0.0;
+    } else {
+      reduce_store((int)v, (int)k, (int)h, t, b.m11, b.m22, b.m12, out);
     }
-    double s[4] = {0, 0, 0, 0};
-    for (uint32_t i = 0; i < b.nparts; ++i, q += 4 * h) {
-#pragma unroll
-      for (int v = 0; v < 4; ++v) s[v] += q[(size_t)v * h];
-    }
-    out[k] = b.m11 * s[0];
-    out[h + k] = b.m22 * s[1];
-    out[2 * h + 2 * k] = b.m12 * s[2];
-    out[2 * h + 2 * k + 1] = b.m12 * s[3];
-    out[4 * h + k] = 0.0;
   }
 }
 

@@ -313,6 +313,7 @@ __global__ void __launch_bounds__(FPC * N / 16, (N >= 8192 ? 1 : 2))
 phased_batch_kernel(const BatchArgs a, int grp) {
   extern __shared__ __align__(128) uint8_t smem[];
   const SmemLayout L = smem_layout<N, FPC>(2u * FPC * N);
+  if (blockIdx.x >= a.hdr->nitems[grp]) return;  // a graph launches the full grid
   uint32_t* ticket = reinterpret_cast<uint32_t*>(smem + L.off_flag + 4);
   PhasedCta<N> c;
   phased_cta_init<N, FPC>(smem, L, c);

@@ -413,6 +413,7 @@ __global__ void __launch_bounds__(kT, 1) phased_pair_kernel(const __grid_constan
 // every bit depth, and every frame is computed exactly as by phased_pair_kernel.
 __global__ void __launch_bounds__(kT, 1) phased_pair_batch_kernel(const BatchArgs a, int grp) {
   extern __shared__ __align__(128) uint8_t smem[];
+  if (blockIdx.x >= a.hdr->nitems[grp]) return;  // a graph launches the full grid
   uint32_t* ticket = reinterpret_cast<uint32_t*>(smem + kPpTicket);
   PpCta c;
   pp_cta_init(smem, c);

@@ -1,0 +1,63 @@
+"""Work items of short sectors in a batch: sector lengths at the edges of the
+item rule (one frame, fewer frames than items, a ragged last item, frames that
+do not fill a CTA iteration) for each group, all groups side by side in one
+call, against the per-scan path: .raw bytes equal, spectra within the FP32
+tolerance of _cases.py; the same bit for bit with and without graphs."""
+import numpy as np
+import pytest
+
+import oracle
+from _cases import assert_sector_close, assert_spectra_close, make_scan, signal_raw, to_fxc
+
+pytestmark = pytest.mark.gpu
+
+DELAY = dict(net_d1_base=3.3e-7, total_rate1_base=2.1e-6, lo1_hz=8.4e9, lo2_hz=8.4e9)
+CORR = oracle.PROD_ACF | oracle.PROD_XCF
+PHASED = oracle.PROD_PHASED | oracle.PROD_RAW
+
+
+@pytest.mark.parametrize("scale", [0, 1, 2])
+def test_short_sector_items(engine, fxc_lib, scale):
+    import torch
+
+    # the least item of FFT n is 32768 / n frames: nf below it, one more than
+    # 24 (32) items of it, and a ragged multiple
+    def length(n, parts):
+        lo = 32768 // n
+        return (1, parts * lo + 1, 3 * parts * lo - 5)[scale]
+
+    items = []
+    for k, (n, prod) in enumerate([(n, p) for n in (1024, 2048, 4096, 8192, 16384)
+                                   for p in (CORR, PHASED)]):
+        nf = length(n, 24 if prod == CORR else 32)
+        nf = min(nf, 4_000_000 // n)
+        sc = make_scan(fft=n, fs=512e6, band=(8, 0, n // 2 - 16, 8), delay=DELAY, products=prod,
+                       shuffle="generic", seed=k)
+        r1, r2 = signal_raw(sc, nf, seed=100 * scale + k, rho=0.3, delay_samples=2.6)
+        d1, d2 = (torch.from_numpy(np.ascontiguousarray(r)).cuda() for r in (r1, r2))
+        items.append((sc, engine.open_scan(to_fxc(sc)), d1, d2, nf))
+
+    def run(batch):
+        acc = [torch.zeros(5 * s.cfg.h, dtype=torch.float64, device="cuda")
+               for _, s, *_ in items]
+        raw = [torch.zeros(nf * s.cfg.bpf(s.cfg.bits_out), dtype=torch.uint8, device="cuda")
+               if sc.products == PHASED else None for sc, s, _, _, nf in items]
+        batch.run_device_raw([i[1] for i in items], [i[2] for i in items],
+                             [i[3] for i in items], [i[4] for i in items], [3] * len(items),
+                             acc, raw)
+        torch.cuda.synchronize()
+        return [a.cpu().numpy() for a in acc], [None if r is None else r.cpu().numpy() for r in raw]
+
+    acc, raw = run(fxc_lib.Batch(engine))
+    acc_g, raw_g = run(fxc_lib.Batch(engine, use_graphs=True))
+    for (sc, s, d1, d2, nf), a, ag, r, rg in zip(items, acc, acc_g, raw, raw_g):
+        assert np.array_equal(a, ag)
+        one = s.sector_device(d1, d2, nf, first_frame=3)
+        h = sc.fft // 2 + 1
+        if sc.products == PHASED:
+            assert np.array_equal(r, rg) and np.array_equal(r, one["raw"])
+            assert_spectra_close(a[4 * h:], one["phased"], f"fft {sc.fft} nf {nf}")
+        else:
+            got = dict(acf11=a[:h], acf22=a[h:2 * h], xcf=a[2 * h:4 * h].view(np.complex128))
+            assert_sector_close(got, one, sc, f"fft {sc.fft} nf {nf}", nf=nf)
+        s.close()
