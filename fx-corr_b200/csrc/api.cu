@@ -9,6 +9,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <limits>
 #include <atomic>
 #include <mutex>
 #include <string>
@@ -89,6 +90,12 @@ struct SectorSlot {
   bool busy = false;
 };
 
+// The re-quantiser's thresholds (fxc_device.cuh, quantise).
+struct QuantTable {
+  int32_t kind = QUANT_SEARCH;
+  float hi = 0.0f, step = 0.0f, offset = 0.0f;
+};
+
 struct fxc_scan {
   fxc_engine* eng = nullptr;
   fxc_scan_cfg cfg{};
@@ -107,6 +114,7 @@ struct fxc_scan {
   float* d_qlevels = nullptr;     // levels1 as f32 for the phased re-quantiser
   uint32_t* d_enc_lut = nullptr;  // [4][256] byte LUTs of ant1's output shuffle
   int qmonotonic = 0;
+  QuantTable quant;
   double* d_partials = nullptr;
   uint64_t partials_elems = 0;
   uint64_t partials_cap = 0;     // elements allocated
@@ -152,6 +160,60 @@ void build_lut(const uint8_t sh[32], uint32_t* lut) {
     for (int v = 0; v < 256; ++v)
       if ((v >> bit) & 1) lut[byte * 256 + v] |= (1u << o);
   }
+}
+
+// Thresholds of the nearest-level rule (first index wins ties) for strictly
+// ascending levels: thr[i], i = 1..n-1, is the least f32 x whose rounded distance
+// to level i is below that to level i - 1.  Between two levels both rounded
+// distances are monotonic in x, so that is a step, found by bisection; and no
+// other level can be nearer or tie as long as the spacing does not vanish in the
+// rounding: levels no closer than 2^-20 of their range, |x| up to 2^20
+// spacings beyond them.  Other tables keep the search.
+QuantTable quant_thresholds(const float* lv, uint32_t n, bool ascending, float* thr) {
+  QuantTable q;
+  for (int i = 0; i < 257; ++i) thr[i] = std::numeric_limits<float>::infinity();
+  thr[0] = -thr[256];
+  if (!ascending || n < 2) return q;
+  double gap = 1e300;
+  for (uint32_t i = 1; i < n; ++i) gap = std::min(gap, (double)lv[i] - (double)lv[i - 1]);
+  const double top = std::max(std::fabs((double)lv[0]), std::fabs((double)lv[n - 1]));
+  if (!std::isfinite(top) || !(gap > 0x1p-100) || gap < top * 0x1p-20) return q;
+  // f32 values in order as integers
+  auto key = [](float x) {
+    int32_t b;
+    std::memcpy(&b, &x, 4);
+    return b < 0 ? (int64_t)INT32_MIN - b : (int64_t)b;
+  };
+  auto val = [](int64_t k) {
+    const int32_t b = k < 0 ? (int32_t)((int64_t)INT32_MIN - k) : (int32_t)k;
+    float x;
+    std::memcpy(&x, &b, 4);
+    return x;
+  };
+  for (uint32_t i = 1; i < n; ++i) {
+    int64_t lo = key(lv[i - 1]), hi = key(lv[i]);  // not past, past
+    while (hi - lo > 1) {
+      const int64_t m = lo + (hi - lo) / 2;
+      const float x = val(m);
+      const float below = std::fabs(x - lv[i - 1]), above = std::fabs(x - lv[i]);
+      if (above < below) hi = m;
+      else lo = m;
+    }
+    thr[i] = val(hi);
+  }
+  q.hi = (float)(gap * 0x1p+20);
+  if (n <= 4) {
+    q.kind = QUANT_COMPARE;
+    return q;
+  }
+  // a uniform table: the guess is right but next to a threshold
+  const double step = ((double)lv[n - 1] - (double)lv[0]) / (n - 1);
+  for (uint32_t i = 0; i < n; ++i)
+    if (std::fabs((double)lv[i] - ((double)lv[0] + i * step)) > 0.01 * step) return q;
+  q.kind = QUANT_STEP;
+  q.step = (float)(1.0 / step);
+  q.offset = (float)(0.5 - (double)lv[0] / step);
+  return q;
 }
 
 // Power of two nearest 1/RMS of a level table.  Both stations share one
@@ -366,6 +428,10 @@ PhasedParams phased_params(const fxc_scan* s, const uint8_t* r1, const uint8_t* 
   p.qlevels = s->d_qlevels;
   p.nqlevels = s->cfg.nlevels1;
   p.qmonotonic = s->qmonotonic;
+  p.qkind = s->quant.kind;
+  p.qhi = s->quant.hi;
+  p.qstep = s->quant.step;
+  p.qoffset = s->quant.offset;
   p.enc_lut = s->d_enc_lut;
   p.finfo = s->d_finfo;
   p.partials = s->d_partials;
@@ -763,7 +829,7 @@ fxc_status scan_bind(fxc_scan* s, const fxc_scan_cfg* cfg) {
 // then one async upload each on the scan's compute stream.
 fxc_status upload_tables(fxc_scan* s, const fxc_scan_cfg* cfg, uint64_t tlen) {
   fxc_status st;
-  constexpr uint64_t kLut = 0, kLv = 8192, kSh = kLv + 2048, kQl = kSh + 32, kEnc = kQl + 1024,
+  constexpr uint64_t kLut = 0, kLv = 8192, kSh = kLv + 2048, kQl = kSh + 32, kEnc = kQl + 4 * 514,
                      kTab = kEnc + 4096;
   if ((st = grow_host(&s->h_tab, &s->h_tab_cap, kTab + tlen * 8)) != FXC_OK) return st;
   uint32_t* lut = reinterpret_cast<uint32_t*>(s->h_tab + kLut);
@@ -780,6 +846,7 @@ fxc_status upload_tables(fxc_scan* s, const fxc_scan_cfg* cfg, uint64_t tlen) {
   // |x - lv as f32|) and the encode LUT of ant1's shuffle: packed bit pos
   // goes to bit shuffle1[pos] (utils.rs:395)
   std::memcpy(ql, lv, 256 * sizeof(float));
+  ql[513] = 0.0f;
   std::memset(enc, 0, 1024 * sizeof(uint32_t));
   for (int pos = 0; pos < 32; ++pos)
     for (int v = 0; v < 256; ++v)
@@ -789,11 +856,12 @@ fxc_status upload_tables(fxc_scan* s, const fxc_scan_cfg* cfg, uint64_t tlen) {
     if (!(lv[i] > lv[i - 1])) up = false;
     if (!(lv[i] < lv[i - 1])) down = false;
   }
+  s->quant = quant_thresholds(lv, cfg->nlevels1, up, ql + 256);
   if (tlen) std::memcpy(s->h_tab + kTab, cfg->delay.geom_table, tlen * 8);
   CK(cudaMemcpyAsync(s->d_lut, lut, 8192, cudaMemcpyHostToDevice, s->stream));
   CK(cudaMemcpyAsync(s->d_levels, lv, 2048, cudaMemcpyHostToDevice, s->stream));
   CK(cudaMemcpyAsync(s->d_shuffle_out, s->h_tab + kSh, 32, cudaMemcpyHostToDevice, s->stream));
-  CK(cudaMemcpyAsync(s->d_qlevels, ql, 1024, cudaMemcpyHostToDevice, s->stream));
+  CK(cudaMemcpyAsync(s->d_qlevels, ql, kQuantFloats * sizeof(float), cudaMemcpyHostToDevice, s->stream));
   CK(cudaMemcpyAsync(s->d_enc_lut, enc, 4096, cudaMemcpyHostToDevice, s->stream));
   if (tlen)
     CK(cudaMemcpyAsync(s->d_table, s->h_tab + kTab, tlen * 8, cudaMemcpyHostToDevice, s->stream));
@@ -905,7 +973,7 @@ fxc_status fxc_scan_open(fxc_engine* e, const fxc_scan_cfg* cfg, fxc_scan** out)
   CKS(cudaMalloc(&s->d_lut, 2 * 1024 * sizeof(uint32_t)));
   CKS(cudaMalloc(&s->d_levels, 2 * 256 * sizeof(float)));
   CKS(cudaMalloc(&s->d_shuffle_out, 32));
-  CKS(cudaMalloc(&s->d_qlevels, 256 * sizeof(float)));
+  CKS(cudaMalloc(&s->d_qlevels, kQuantFloats * sizeof(float)));
   CKS(cudaMalloc(&s->d_enc_lut, 1024 * sizeof(uint32_t)));
   CKS(cudaMalloc(&s->d_err, 16));
   CKS(cudaMemset(s->d_err, 0, 16));

@@ -182,14 +182,11 @@ __device__ __forceinline__ void twiddle(float2* v, float2 w) {
 // Complex buffers: one pad slot per 16 elements keeps the radix-16 Stockham
 // loads and stores free of bank conflicts for 8-byte accesses.
 __device__ __forceinline__ int cpad(int i) { return i + (i >> 4); }
-// Planar float buffers (decoded samples): one pad word per 32.
-__device__ __forceinline__ int fpad(int i) { return i + (i >> 5); }
 
 template <int N>
 struct Geom {
   static constexpr int T1 = N / 16;            // threads per frame pair
   static constexpr int CSTRIDE = N + N / 16;   // float2 per padded frame
-  static constexpr int FSTRIDE = N + N / 32;   // floats per padded station plane
   static constexpr int LOG2N = (N == 1024) ? 10 : (N == 2048) ? 11 : (N == 4096) ? 12
                              : (N == 8192) ? 13 : (N == 16384) ? 14 : 0;
   static constexpr int P16 = LOG2N / 4;            // radix-16 passes
@@ -230,16 +227,16 @@ struct Twiddles {
 // (OUT_PAD = false) stores an unpadded natural-order spectrum: its stores are
 // consecutive runs, and unpadded consecutive runs of any alignment (the
 // Z[N-k], Z[k+sb] reads of the consumers) are free of bank conflicts.
-template <int N, int R, int NS, bool OUT_PAD = true>
-__device__ __forceinline__ void stockham_pass(const float2* __restrict__ in, float2* __restrict__ out,
-                                              int t, float2 w) {
+// stockham_values leaves the thread's outputs in registers (output r of item wi
+// at v[wi R + out_pos<R>(r)]).
+template <int N, int R, int NS>
+__device__ __forceinline__ void stockham_values(const float2* __restrict__ in, int t, float2 w,
+                                                float2 (&v)[16]) {
   constexpr int T1 = N / 16;
   constexpr int WI = 16 / R;
   static_assert((N / R) % 16 == 0 && NS % 16 == 0, "padded strides");
   // cpad(j + r*M) = cpad(j) + r*(M + M/16) whenever M is a multiple of 16
   constexpr int LS = N / R + N / (16 * R);
-  constexpr int SS = NS + NS / 16;
-  float2 v[16];
 #pragma unroll
   for (int wi = 0; wi < WI; ++wi) {
     const int j = t + T1 * wi;
@@ -312,6 +309,16 @@ __device__ __forceinline__ void stockham_pass(const float2* __restrict__ in, flo
       }
     }
   }
+}
+
+template <int N, int R, int NS, bool OUT_PAD = true>
+__device__ __forceinline__ void stockham_pass(const float2* __restrict__ in, float2* __restrict__ out,
+                                              int t, float2 w) {
+  constexpr int T1 = N / 16;
+  constexpr int WI = 16 / R;
+  constexpr int SS = NS + NS / 16;
+  float2 v[16];
+  stockham_values<N, R, NS>(in, t, w, v);
 #pragma unroll
   for (int wi = 0; wi < WI; ++wi) {
     const int j = t + T1 * wi;
@@ -326,45 +333,6 @@ __device__ __forceinline__ void stockham_pass(const float2* __restrict__ in, flo
       for (int r = 0; r < R; ++r) dst[r * NS] = v[wi * R + out_pos<R>(r)];
     }
   }
-}
-
-// First pass: reads the two decoded station planes with their integer shifts
-// (zero fill, src/utils.rs:126-145) and packs z[n] = x1[n-s1] + i x2[n-s2].
-template <int N>
-__device__ __forceinline__ void first_pass(const float* __restrict__ x1, const float* __restrict__ x2,
-                                           int s1, int s2, float2* __restrict__ out, int t) {
-  constexpr int T1 = N / 16;
-  static_assert(T1 % 32 == 0, "plane stride");
-  // fpad(t + r*T1) = fpad(t) + r*(T1 + T1/32) since T1 is a multiple of 32
-  constexpr int PS = T1 + T1 / 32;
-  float2 v[16];
-  // the shift is uniform per frame: unshifted stations take the unchecked path
-  if (s1 == 0) {
-    const float* p = x1 + fpad(t);
-#pragma unroll
-    for (int r = 0; r < 16; ++r) v[r].x = p[r * PS];
-  } else {
-#pragma unroll
-    for (int r = 0; r < 16; ++r) {
-      const int m = t + r * T1 - s1;
-      v[r].x = ((unsigned)m < (unsigned)N) ? x1[fpad(m)] : 0.0f;
-    }
-  }
-  if (s2 == 0) {
-    const float* p = x2 + fpad(t);
-#pragma unroll
-    for (int r = 0; r < 16; ++r) v[r].y = p[r * PS];
-  } else {
-#pragma unroll
-    for (int r = 0; r < 16; ++r) {
-      const int m = t + r * T1 - s2;
-      v[r].y = ((unsigned)m < (unsigned)N) ? x2[fpad(m)] : 0.0f;
-    }
-  }
-  dft16(v);
-  float2* dst = out + 17 * t;  // cpad(16 t + r) = 17 t + r
-#pragma unroll
-  for (int r = 0; r < 16; ++r) dst[r] = v[out_pos<16>(r)];
 }
 
 // One station of a frame as staged packed words (already shuffled into the
@@ -482,6 +450,33 @@ __device__ __forceinline__ float2* fft_rest(float2* a, float2* b, int t, const T
     float2* x = in; in = out; out = x;
   }
   return in;
+}
+
+// fft_rest with the last pass's outputs left in registers: output r of item wi
+// is Z[t + N/16 wi + r N/R], R = fft_last_radix<N>, at v[wi R + out_pos<R>(r)].
+template <int N>
+constexpr int fft_last_radix = Geom<N>::RL > 1 ? Geom<N>::RL : 16;
+template <int N>
+__device__ __forceinline__ void fft_rest_values(float2* a, float2* b, int t, const Twiddles<N>& tw,
+                                                float2 (&v)[16]) {
+  constexpr int P16 = Geom<N>::P16;
+  constexpr int RL = Geom<N>::RL;
+  constexpr bool TRAIL = RL > 1;
+  float2* in = a;
+  float2* out = b;
+  if constexpr (P16 >= 3 || TRAIL) {
+    __syncthreads();
+    stockham_pass<N, 16, 16, true>(in, out, t, tw.w[1]);
+    float2* x = in; in = out; out = x;
+  }
+  if constexpr (P16 >= 3 && TRAIL) {
+    __syncthreads();
+    stockham_pass<N, 16, 256, true>(in, out, t, tw.w[2]);
+    float2* x = in; in = out; out = x;
+  }
+  __syncthreads();
+  if constexpr (TRAIL) stockham_values<N, RL, 1 << (4 * P16)>(in, t, tw.w[P16], v);
+  else stockham_values<N, 16, 1 << (4 * (P16 - 1))>(in, t, tw.w[P16 - 1], v);
 }
 
 // ------------------------------------------------------------ delay model
@@ -673,6 +668,38 @@ __device__ __forceinline__ uint32_t nearest_level(float x, const float* __restri
     }
   }
   return best;
+}
+
+// The same for level tables with decision thresholds (the host found them by
+// bisection with nearest_level's own f32 comparison: thr[i] is the least x that
+// takes level i or a higher one; thr[0] = -inf, thr[n] = +inf): up to four
+// levels by comparison, more by the step of a uniform table, whose guess is off
+// by one level at most, and the two thresholds around it.  The general search
+// takes about 8 instructions per level; this 6 in all, or 12.  Values beyond
+// `hi` (where the distances round to ties) and NaN take the general search.
+enum : int32_t { QUANT_SEARCH = 0, QUANT_COMPARE = 1, QUANT_STEP = 2 };
+struct Quantiser {
+  const float* ql;   // levels, then from 256 the thresholds
+  int32_t n, monotonic, kind;
+  float hi, step, offset;  // QUANT_STEP: level index ~ floor(x step + offset)
+};
+constexpr int kQuantFloats = 256 + 257;
+__device__ __forceinline__ uint32_t quantise(float x, const Quantiser& q, const float* thr) {
+  if (q.kind != QUANT_SEARCH && fabsf(x) <= q.hi) {
+    if (q.kind == QUANT_COMPARE)
+      return (uint32_t)(x >= thr[1]) + (uint32_t)(x >= thr[2]) + (uint32_t)(x >= thr[3]);
+    int g = __float2int_rd(fmaf(x, q.step, q.offset));
+    g = min(max(g, 0), q.n - 1);
+    g += (x >= thr[g + 1] ? 1 : 0) - (x < thr[g] ? 1 : 0);
+    return (uint32_t)g;
+  }
+  return nearest_level(x, q.ql, q.n, q.monotonic);
+}
+// At most four levels, the thresholds in registers (t = thr[1..3]).
+__device__ __forceinline__ uint32_t quantise4(float x, const Quantiser& q, float3 t) {
+  if (q.kind == QUANT_COMPARE && fabsf(x) <= q.hi)
+    return (uint32_t)(x >= t.x) + (uint32_t)(x >= t.y) + (uint32_t)(x >= t.z);
+  return nearest_level(x, q.ql, q.n, q.monotonic);
 }
 
 // ------------------------------------------------------ staging layout

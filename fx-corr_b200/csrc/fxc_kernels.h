@@ -52,9 +52,11 @@ struct PhasedParams {
   int32_t out_lsb;       // negate odd output samples (both stations LSB)
   int32_t want_raw;
   float w1, w2;
-  const float* qlevels;  // levels1 as f32 (device)
+  const float* qlevels;  // levels1 as f32, then from 256 their thresholds (device)
   uint32_t nqlevels;
   int32_t qmonotonic;    // +1 / -1 strictly ascending / descending levels, else 0
+  int32_t qkind;         // QUANT_*: how the thresholds may be used
+  float qhi, qstep, qoffset;
   const uint32_t* enc_lut;  // [4][256] byte LUTs of ant1's output shuffle (device)
   const FrameInfo* finfo;
   double* partials;      // [grid][H] f64

@@ -766,9 +766,10 @@ __global__ void phased_global_kernel(const LargeParams p, const PhasedParams pp,
 // ant1's levels, codes LSB-first, ant1's shuffle applied per word.
 __global__ void quant_global_kernel(const LargeParams p, const PhasedParams pp,
                                     const float2* __restrict__ X, uint64_t f0, uint64_t nb) {
-  __shared__ float ql[256];
+  __shared__ float ql[kQuantFloats];
   __shared__ uint32_t elut[1024];
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) ql[i] = i < (int)pp.nqlevels ? pp.qlevels[i] : 0.f;
+  for (int i = threadIdx.x; i < kQuantFloats; i += blockDim.x) ql[i] = pp.qlevels[i];
+  const Quantiser quant{ql, (int)pp.nqlevels, pp.qmonotonic, pp.qkind, pp.qhi, pp.qstep, pp.qoffset};
   for (int i = threadIdx.x; i < 1024; i += blockDim.x) elut[i] = pp.enc_lut[i];
   __syncthreads();
   const int C = p.c, M = kLargeM, N = p.n;
@@ -786,7 +787,7 @@ __global__ void quant_global_kernel(const LargeParams p, const PhasedParams pp,
       const int n = (int)(w * spw + i);
       float x = Xf[(n % C) * M + n / C].x * inv_n;
       if (pp.out_lsb && (n & 1)) x = -x;
-      word |= (nearest_level(x, ql, (int)pp.nqlevels, pp.qmonotonic) & qmask) << (i * pp.bits_out);
+      word |= (quantise(x, quant, ql + 256) & qmask) << (i * pp.bits_out);
     }
     const uint32_t sw = elut[word & 255u] | elut[256 + ((word >> 8) & 255u)] |
                         elut[512 + ((word >> 16) & 255u)] | elut[768 + (word >> 24)];

@@ -55,13 +55,13 @@ constexpr int kJ = kM / 2 / kT;  // bins per thread and row (8)
 // rows; XA then row B's spectrum, XB the secondary terms; then the inverse
 // rows), Y (row A's spectrum, then cb of both rows: row A's bins at [0, M/2],
 // row B's at M/2 + 1 + j) and one staging slot.
-constexpr uint32_t kQpFi = 4352, kQpBar = 4400, kQpFlag = 4408, kQpQl = 4416;
+constexpr uint32_t kQpFi = 4352, kQpBar = 4400, kQpFlag = 4408, kQpQl = 4416;  // four levels, five thresholds
 constexpr uint32_t kQpEnc = kTabLut;
 constexpr uint32_t kQpBuf = (uint32_t)Geom<kM>::CSTRIDE * (uint32_t)sizeof(float2);
 constexpr uint32_t kQpXA = kTabEnd, kQpXB = kQpXA + kQpBuf, kQpY = kQpXB + kQpBuf;
 constexpr uint32_t kQpStage = kQpY + kQpBuf;
 constexpr uint32_t kQpMaxSmem = 232448;  // 227 KB per CTA on sm_100
-static_assert(kQpFi + kFiBytes <= kQpBar && kQpQl + 16 * 4 <= kTabLut, "records fit the gap");
+static_assert(kQpFi + kFiBytes <= kQpBar && kQpQl + 9 * 4 <= kTabLut, "records fit the gap");
 
 __host__ __device__ constexpr uint32_t qp_smem_bytes(int c, int bits_1, int bits_2) {
   return kQpStage + ((128u + 4u * (uint32_t)c *
@@ -163,7 +163,8 @@ __global__ void __cluster_dims__(C / 2, 1, 1) __launch_bounds__(kT, 1)
     issue(it0, g->s1, g->s2);
   }
   build_decode_tables(s1, s2, false, false, smem, tid, kT);
-  for (int i = tid; i < 16; i += kT) ql[i] = i < (int)p.nqlevels ? p.qlevels[i] : 0.f;
+  for (int i = tid; i < 9; i += kT) ql[i] = p.qlevels[i < 4 ? i : 256 + i - 4];
+  const Quantiser quant{ql, (int)p.nqlevels, p.qmonotonic, p.qkind, p.qhi, p.qstep, p.qoffset};
   for (int i = tid; i < 1024; i += kT) elut[i] = p.enc_lut[i];
   const bool split1 = split_2bit(s1), split2 = split_2bit(s2);
   Twiddles<kM> tw;
@@ -422,6 +423,7 @@ __global__ void __cluster_dims__(C / 2, 1, 1) __launch_bounds__(kT, 1)
       // the cluster's CTAs OR their bits together (the words start at zero)
       uint32_t* out = reinterpret_cast<uint32_t*>(p.raw_out + it * p.bpf_out);
       const uint32_t per = spw / (uint32_t)C;  // samples of one row in a word
+      const float3 thr = make_float3(ql[5], ql[6], ql[7]);
       for (uint32_t wdx = (uint32_t)tid; wdx < wpf; wdx += kT) {
         uint32_t word = 0;
         for (uint32_t i = 0; i < per; ++i) {
@@ -432,7 +434,7 @@ __global__ void __cluster_dims__(C / 2, 1, 1) __launch_bounds__(kT, 1)
             const uint32_t n = (uint32_t)C * k + row;
             float x = (b ? XA : Y)[k].x * inv_n;
             if (p.out_lsb && (n & 1u)) x = -x;
-            word |= (nearest_level(x, ql, (int)p.nqlevels, p.qmonotonic) & qmask)
+            word |= (quantise4(x, quant, thr) & qmask)
                     << ((n - wdx * spw) * p.bits_out);
           }
         }

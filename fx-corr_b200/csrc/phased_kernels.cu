@@ -14,6 +14,16 @@
 //      1/N (src/utils.rs:60-66), odd samples negated when both inputs are LSB,
 //      nearest-level re-quantisation with ant1's levels and packing with ant1's
 //      shuffle (quantise_frame, src/utils.rs:378-410).
+//
+// Bound by instruction issue (59 % of the slots, 16 warps per SM): two FFTs, the
+// synthesis and the re-quantiser are 34.2k warp instructions per frame pair of
+// FFT 4096 with a search of the levels for every sample and the spectrum written
+// as two planes of the Hermitian extension.  With the spectrum kept by bin (one
+// 8-byte store; the inverse's first pass mirrors as it reads), thresholds
+// instead of the search, and 1- and 2-bit samples quantised in the registers of
+// the last pass (votes, no exchange): FFT 1024, 50001 frame pairs 620 -> 471 us,
+// 2048 1208 -> 908, 4096 (20000) 1004 -> 745, 8192 (12503) 1348 -> 1015 us; 8-bit
+// FFT 8192 2097 -> 1322 us; the .raw bytes are the same.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -21,6 +31,9 @@
 #include "fxc_kernels.h"
 
 namespace fxc {
+
+constexpr uint32_t kQuantBytes = (kQuantFloats * 4 + 15) / 16 * 16;
+constexpr uint32_t kTailBytes = kQuantBytes + 4096;  // quantiser and encode tables
 
 // Per-CTA state that outlives one sector: the twiddle bases and the number of
 // staging iterations consumed so far (it sets the mbarrier slot and phase, so
@@ -81,8 +94,8 @@ __device__ __noinline__ bool phased_span(const PhasedParams& p, uint64_t it0, ui
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L.off_bar);
   int* flag = reinterpret_cast<int*>(smem + L.off_flag);
   // quantiser tables live in the extra tail of the layout
-  float* ql = reinterpret_cast<float*>(smem + L.total);              // 256 levels
-  uint32_t* elut = reinterpret_cast<uint32_t*>(smem + L.total + 1024);  // [4][256] encode LUT
+  float* ql = reinterpret_cast<float*>(smem + L.total);  // levels and thresholds
+  uint32_t* elut = reinterpret_cast<uint32_t*>(smem + L.total + kQuantBytes);  // [4][256] encode LUT
 
   const int tid = threadIdx.x;
   const int g = tid / T1;
@@ -117,7 +130,7 @@ __device__ __noinline__ bool phased_span(const PhasedParams& p, uint64_t it0, ui
   for (int s = 0; s < 2; ++s)
     if (p.st[s].shkind == SH_GENERIC)
       for (int i = tid; i < 1024; i += T) lut[s * 1024 + i] = p.st[s].shlut[i];
-  for (int i = tid; i < 256; i += T) ql[i] = i < (int)p.nqlevels ? p.qlevels[i] : 0.f;
+  for (int i = tid; i < kQuantFloats; i += T) ql[i] = p.qlevels[i];
   for (int i = tid; i < 1024; i += T) elut[i] = p.enc_lut[i];
   __syncthreads();
 
@@ -189,14 +202,13 @@ __device__ __noinline__ bool phased_span(const PhasedParams& p, uint64_t it0, ui
     const bool fin_b = Z0 != za;
     __syncthreads();
 
-    // ---- per-bin synthesis over every valid frame of the iteration; the
-    // inverse-FFT input planes go to the buffer that does not hold Z
+    // ---- per-bin synthesis over every valid frame of the iteration; cb goes
+    // by bin to the buffer that does not hold Z
 #pragma unroll 1
     for (int f = 0; f < FPC; ++f) {
       if (it * FPC + f >= p.nf) break;
       const float2* Z = (fin_b ? bufB : bufA) + f * Geom<N>::CSTRIDE;
-      float* y1 = reinterpret_cast<float*>(fin_b ? bufA : bufB) + f * 2 * Geom<N>::FSTRIDE;
-      float* y2 = y1 + Geom<N>::FSTRIDE;
+      float2* cbs = (fin_b ? bufA : bufB) + f * Geom<N>::CSTRIDE;
       const FrameInfo& F = finfo[f];
       // spectrum of station s at its own bin k: unscaled, rotated by the
       // station's fractional delay, Nyquist imaginary part zeroed, times fr_lo
@@ -222,14 +234,8 @@ __device__ __noinline__ bool phased_span(const PhasedParams& p, uint64_t it0, ui
         return make_float2(a1.x * p.w1 + a2.x * p.w2, a1.y * p.w1 + a2.y * p.w2);
       };
       auto emit = [&](int k, float2 cb) {
-        // Hermitian extension of conj(cb) as planes for the forward FFT
         if (k == 0 || k == N / 2) cb.y = 0.f;
-        y1[fpad(k)] = cb.x;
-        y2[fpad(k)] = -cb.y;
-        if (k != 0 && k != N / 2) {
-          y1[fpad(N - k)] = cb.x;
-          y2[fpad(N - k)] = cb.y;
-        }
+        cbs[k] = cb;
       };
 #pragma unroll
       for (int i = 0; i < BPT; ++i) {
@@ -248,36 +254,116 @@ __device__ __noinline__ bool phased_span(const PhasedParams& p, uint64_t it0, ui
 
     if (p.want_raw) {
       __syncthreads();
-      // inverse real FFT of frame slot g: forward FFT of conj(C), real part / N
-      float* y1 = reinterpret_cast<float*>(fin_b ? bufA : bufB) + g * 2 * Geom<N>::FSTRIDE;
-      float* y2 = y1 + Geom<N>::FSTRIDE;
+      // inverse real FFT of frame slot g: forward FFT of the Hermitian extension
+      // of conj(cb), real part / N.  First pass: x[n] = conj(cb[n]) for n <= N/2,
+      // cb[N - n] above.
       float2* qa = (fin_b ? bufB : bufA) + g * Geom<N>::CSTRIDE;  // free: Z consumed
       float2* qb = (fin_b ? bufA : bufB) + g * Geom<N>::CSTRIDE;
-      first_pass<N>(y1, y2, 0, 0, qa, t);
-      float2* Y = fft_rest<N>(qa, qb, t, tw);
-      __syncthreads();
-      if (valid) {
-        const float inv_n = 1.0f / (float)N;
-        uint8_t* out = p.raw_out + frame_local * p.bpf_out;
-        // Consecutive lanes pack consecutive words, spw samples apart: each
-        // lane starts its word at a different sample (rot) so that the 16
-        // lanes of a half-warp read 16 different bank pairs of Y at every
-        // step instead of one.
-        const uint32_t lane = (uint32_t)t & 31u;
-        const uint32_t rot = spw >= 16 ? lane : lane / (16u / spw);
-        for (uint32_t w = (uint32_t)t; w < wpf; w += T1) {
-          uint32_t word = 0;
-          for (uint32_t i = 0; i < spw; ++i) {
-            const uint32_t ii = (i + rot) & (spw - 1u);
-            const uint32_t n = w * spw + ii;
-            float x = Y[n].x * inv_n;
-            if (p.out_lsb && (n & 1u)) x = -x;
-            word |= (nearest_level(x, ql, (int)p.nqlevels, p.qmonotonic) & qmask)
-                    << (ii * p.bits_out);
+      float2 v[16];
+#pragma unroll
+      for (int r = 0; r < 16; ++r) {
+        const int n = t + r * T1;
+        const float2 cb = qb[r < 8 || n == N / 2 ? n : N - n];
+        v[r] = make_float2(cb.x, r < 8 || n == N / 2 ? -cb.y : cb.y);
+      }
+      dft16(v);
+      {
+        float2* dst = qa + 17 * t;  // cpad(16 t + r) = 17 t + r
+#pragma unroll
+        for (int r = 0; r < 16; ++r) dst[r] = v[out_pos<16>(r)];
+      }
+      const float inv_n = 1.0f / (float)N;
+      uint32_t* out = reinterpret_cast<uint32_t*>(p.raw_out + frame_local * p.bpf_out);
+      const Quantiser quant{ql, (int)p.nqlevels, p.qmonotonic, p.qkind, p.qhi, p.qstep, p.qoffset};
+      auto encode = [&](uint32_t word) -> uint32_t {  // ant1's shuffle
+        return elut[word & 255u] | elut[256 + ((word >> 8) & 255u)] |
+               elut[512 + ((word >> 16) & 255u)] | elut[768 + (word >> 24)];
+      };
+      if (p.bits_out <= 2 && p.qkind == QUANT_COMPARE) {
+        // 1- and 2-bit output: a warp holds 32 consecutive samples in each of
+        // its 16 output registers; the comparisons with the thresholds are
+        // collected by votes, 32 codes at a time, and lane q of each half
+        // keeps row q.  No exchange of samples through shared memory, and the
+        // last pass has no imaginary parts to form.
+        constexpr int R = fft_last_radix<N>;
+        fft_rest_values<N>(qa, qb, t, tw, v);
+        if (valid) {
+          const uint32_t lane = (uint32_t)t & 31u;
+          const uint32_t flip = p.out_lsb ? lane << 31 : 0u;  // odd samples negated
+          float top = 0.f;
+#pragma unroll
+          for (int q = 0; q < 16; ++q) {
+            v[q].x = __uint_as_float(__float_as_uint(v[q].x * inv_n) ^ flip);
+            top = fmaxf(top, fabsf(v[q].x));
           }
-          const uint32_t sw = elut[word & 255u] | elut[256 + ((word >> 8) & 255u)] |
-                              elut[512 + ((word >> 16) & 255u)] | elut[768 + (word >> 24)];
-          reinterpret_cast<uint32_t*>(out)[w] = sw;
+          const float t1 = ql[257], t2 = ql[258], t3 = ql[259];
+          uint32_t lo = 0, hi = 0;
+          if (__all_sync(0xFFFFFFFFu, top <= p.qhi)) {
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+              const float x = v[q / R * R + out_pos<R>(q % R)].x;
+              const uint32_t b1 = __ballot_sync(0xFFFFFFFFu, x >= t1);
+              const uint32_t b2 = __ballot_sync(0xFFFFFFFFu, x >= t2);
+              const uint32_t b3 = __ballot_sync(0xFFFFFFFFu, x >= t3);
+              if ((lane & 15u) == (uint32_t)q) {
+                lo = b1 ^ b2 ^ b3;
+                hi = b2;
+              }
+            }
+          } else {
+#pragma unroll 1
+            for (int q = 0; q < 16; ++q) {
+              float x = 0.f;  // a runtime index would move v to local memory
+#pragma unroll
+              for (int k = 0; k < 16; ++k)
+                if (k == q) x = v[k / R * R + out_pos<R>(k % R)].x;
+              const uint32_t c = nearest_level(x, ql, (int)p.nqlevels, p.qmonotonic);
+              const uint32_t b0 = __ballot_sync(0xFFFFFFFFu, (c & 1u) != 0);
+              const uint32_t b1 = __ballot_sync(0xFFFFFFFFu, (c & 2u) != 0);
+              if ((lane & 15u) == (uint32_t)q) {
+                lo = b0;
+                hi = b1;
+              }
+            }
+          }
+          // row q: samples n0 + 0..31
+          const uint32_t q = lane & 15u;
+          const uint32_t n0 = ((uint32_t)t & ~31u) + T1 * (q / R) + (N / R) * (q % R);
+          if (p.bits_out == 1) {
+            if (lane < 16u) out[n0 / 32u] = encode(lo);
+          } else {
+            auto spread = [](uint32_t x) -> uint32_t {  // bit i to bit 2 i
+              x = (x | (x << 8)) & 0x00FF00FFu;
+              x = (x | (x << 4)) & 0x0F0F0F0Fu;
+              x = (x | (x << 2)) & 0x33333333u;
+              return (x | (x << 1)) & 0x55555555u;
+            };
+            const uint32_t sh = lane & 16u;
+            const uint32_t word = spread((lo >> sh) & 0xFFFFu) | (spread((hi >> sh) & 0xFFFFu) << 1);
+            out[n0 / 16u + (lane >> 4)] = encode(word);
+          }
+        }
+      } else {
+        float2* Y = fft_rest<N>(qa, qb, t, tw);
+        __syncthreads();
+        if (valid) {
+          // Consecutive lanes pack consecutive words, spw samples apart: each
+          // lane starts its word at a different sample (rot) so that the 16
+          // lanes of a half-warp read 16 different bank pairs of Y at every
+          // step instead of one.
+          const uint32_t lane = (uint32_t)t & 31u;
+          const uint32_t rot = spw >= 16 ? lane : lane / (16u / spw);
+          for (uint32_t w = (uint32_t)t; w < wpf; w += T1) {
+            uint32_t word = 0;
+            for (uint32_t i = 0; i < spw; ++i) {
+              const uint32_t ii = (i + rot) & (spw - 1u);
+              const uint32_t n = w * spw + ii;
+              float x = Y[n].x * inv_n;
+              if (p.out_lsb && (n & 1u)) x = -x;
+              word |= (quantise(x, quant, ql + 256) & qmask) << (ii * p.bits_out);
+            }
+            out[w] = encode(word);
+          }
         }
       }
     }
@@ -334,13 +420,13 @@ phased_batch_kernel(const BatchArgs a, int grp) {
 
 template <int N, int FPC>
 static cudaError_t launch_phased_one(const PhasedParams& p, int grid, cudaStream_t stream) {
-  const uint32_t smem = smem_layout<N, FPC>(p.stage_bytes).total + 1024 + 4096;
+  const uint32_t smem = smem_layout<N, FPC>(p.stage_bytes).total + kTailBytes;
   auto kern = phased_kernel<N, FPC>;
   // the limit is shared by every host thread: always the largest layout
   // (8-bit stations), never lowered under a concurrent launch
   cudaError_t e = cudaFuncSetAttribute(
       kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-      (int)(smem_layout<N, FPC>(2u * FPC * N).total + 1024 + 4096));
+      (int)(smem_layout<N, FPC>(2u * FPC * N).total + kTailBytes));
   if (e != cudaSuccess) return e;
   kern<<<grid, FPC * N / 16, smem, stream>>>(p);
   return cudaGetLastError();
@@ -359,7 +445,7 @@ cudaError_t launch_phased(uint32_t n, const PhasedParams& p, int grid, cudaStrea
 namespace {
 template <int N, int FPC>
 uint32_t phased_batch_smem() {
-  return smem_layout<N, FPC>(2u * FPC * N).total + 1024 + 4096;
+  return smem_layout<N, FPC>(2u * FPC * N).total + kTailBytes;
 }
 }  // namespace
 

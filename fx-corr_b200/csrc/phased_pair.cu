@@ -55,13 +55,13 @@ constexpr int kJ = kM / 2 / kT;  // bin pairs (rows 0 and 1) per thread
 // shuffles, the encode LUT and up to 256 output levels follow the buffers, and
 // the staging slot is a row buffer.
 constexpr uint32_t kPpFi = 4352, kPpBar = 4400, kPpFlag = 4408, kPpTicket = 4412;
-constexpr uint32_t kPpQl = 4416;  // 16 levels max
+constexpr uint32_t kPpQl = 4416;  // four levels, then five thresholds
 constexpr uint32_t kPpEnc = kTabLut;  // [4][256] u32
 constexpr uint32_t kPpBuf = (uint32_t)Geom<kM>::CSTRIDE * (uint32_t)sizeof(float2);
 constexpr uint32_t kPpB0 = kTabEnd, kPpB1 = kPpB0 + kPpBuf, kPpB2 = kPpB1 + kPpBuf;
 constexpr uint32_t kPpStage = kPpB2 + kPpBuf;
 constexpr uint32_t kPpMaxSmem = 232448;  // 227 KB per CTA on sm_100
-static_assert(kPpFi + kFiBytes <= kPpBar && kPpQl + 16 * 4 <= kTabLut, "records fit the gap");
+static_assert(kPpFi + kFiBytes <= kPpBar && kPpQl + 9 * 4 <= kTabLut, "records fit the gap");
 static_assert(kPpStage % 128 == 0, "alignment");
 
 __host__ __device__ constexpr uint32_t pp_smem_bytes(uint32_t bpf1, uint32_t bpf2) {
@@ -69,7 +69,7 @@ __host__ __device__ constexpr uint32_t pp_smem_bytes(uint32_t bpf1, uint32_t bpf
 }
 static_assert(pp_smem_bytes(kN2 / 4, kN2 / 4) <= kPpMaxSmem, "2-bit stations fit");
 constexpr uint32_t kPpWideEnc = kPpStage, kPpWideQl = kPpStage + 4096;
-constexpr uint32_t kPpWideSmem = kPpWideQl + 256 * 4;
+constexpr uint32_t kPpWideSmem = kPpWideQl + kQuantFloats * 4;
 static_assert(kPpWideSmem <= pp_smem_bytes(kN2 / 4, kN2 / 4), "one batch layout serves both");
 static_assert(128u + 2u * kN2 <= kPpBuf, "8-bit stations' words fit a row buffer");
 
@@ -169,8 +169,10 @@ __device__ __forceinline__ bool pp_span(const PhasedParams& p, uint64_t it0, uin
     issue(it0, stage);
   }
   build_decode_tables(s1, s2, pre1, pre2, smem, tid, kT);
-  const int nql = WIDE ? 256 : 16;
-  for (int i = tid; i < nql; i += kT) ql[i] = i < (int)p.nqlevels ? p.qlevels[i] : 0.f;
+  // levels, then thresholds (narrow: at most four levels)
+  constexpr int kLv = WIDE ? 256 : 4;
+  for (int i = tid; i < 2 * kLv + 1; i += kT) ql[i] = p.qlevels[i < kLv ? i : 256 + i - kLv];
+  const Quantiser quant{ql, (int)p.nqlevels, p.qmonotonic, p.qkind, p.qhi, p.qstep, p.qoffset};
   for (int i = tid; i < 1024; i += kT) elut[i] = p.enc_lut[i];
   const bool split1 = split_2bit(s1), split2 = split_2bit(s2);
   const Twiddles<kM>& tw = c.tw;
@@ -365,10 +367,13 @@ __device__ __forceinline__ bool pp_span(const PhasedParams& p, uint64_t it0, uin
       __syncthreads();
       // ---- re-quantise and pack: sample n is row n & 1, index n >> 1.  Each
       // lane starts its word at a different sample so that a warp's loads
-      // spread over the banks.
+      // spread over the banks.  Thresholds instead of a search of the levels:
+      // 3001 frame pairs of 4-bit stations 690 -> 566 us, of 2-bit ones 556 ->
+      // 516 us.
       uint8_t* out = p.raw_out + it * p.bpf_out;
       const uint32_t lane = (uint32_t)tid & 31u;
       const uint32_t rot = spw >= 16 ? lane : lane / (16u / spw);
+      const float3 thr = make_float3(ql[kLv + 1], ql[kLv + 2], ql[kLv + 3]);
       for (uint32_t wdx = (uint32_t)tid; wdx < wpf; wdx += kT) {
         uint32_t word = 0;
         for (uint32_t i = 0; i < spw; ++i) {
@@ -376,7 +381,8 @@ __device__ __forceinline__ bool pp_span(const PhasedParams& p, uint64_t it0, uin
           const uint32_t n = wdx * spw + ii;
           float x = ((n & 1u) ? (WIDE ? P : S) : Q)[n >> 1].x * inv_n;
           if (p.out_lsb && (n & 1u)) x = -x;
-          word |= (nearest_level(x, ql, (int)p.nqlevels, p.qmonotonic) & qmask) << (ii * p.bits_out);
+          const uint32_t code = WIDE ? quantise(x, quant, ql + kLv) : quantise4(x, quant, thr);
+          word |= (code & qmask) << (ii * p.bits_out);
         }
         reinterpret_cast<uint32_t*>(out)[wdx] =
             elut[word & 255u] | elut[256 + ((word >> 8) & 255u)] |
