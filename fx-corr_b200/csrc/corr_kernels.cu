@@ -1,28 +1,22 @@
-// corr_kernels.cu — the fused FX-correlation kernel for sm_100a.
+// corr_kernels.cu — what surrounds the correlation kernels, for sm_100a.
 //
 // frame_info_kernel evaluates the FP64 per-frame delay model
 // (src/main.rs:184-241) for every frame of a sector, one thread per frame, into
-// 48-byte FrameInfo records.
+// 48-byte FrameInfo records; batch_frame_info_kernel does so for every sector of
+// a batch.
 //
-// corr_kernel: one CTA processes a contiguous run of frame pairs of a sector.
-// Per frame pair (stations 1 and 2 share one complex FFT: z = x1 + i*x2):
-//   1. the frame's FrameInfo and the packed .raw words of both stations arrive
-//      in shared memory by cp.async.bulk (TMA bulk copy) tracked by an
-//      mbarrier, two stages deep;
-//   2. decode: 32-bit word shuffle, b-bit codes -> f32 levels, LSB->USB flip of
-//      odd samples (src/utils.rs:215-376);
-//   3. the first radix-16 pass reads the decoded planes with the integer shift
-//      and zero fill (src/utils.rs:126-145); the remaining Stockham passes run
-//      in padded shared memory;
-//   4. two-for-one split of Z into S1, S2 (the two real FFTs,
-//      src/utils.rs:47-59), band alignment, fringe x phase-ramp rotation and
-//      |S|^2 / S1 conj(S2) accumulation (src/main.rs:2491-2568) into per-thread
-//      f32 registers, flushed every 32 frames into per-CTA f64 partials;
-// reduce_partials_kernel then sums the per-CTA partials in a fixed order.
-// The frame loop is corr_span: the single-sector kernel runs it once per CTA
-// over the CTA's share of the sector, the batched kernel (corr_batch_kernel)
-// once per work item taken by ticket from a list spanning many scans, with
-// batch_frame_info_kernel and batch_reduce_kernel on either side.
+// corr_kernel is the stage entry points' kernel (FFT <= 8192): decode + integer
+// shift (MODE_DECODE), or the spectra of both stations (MODE_SPECTRA).  One CTA
+// processes a contiguous run of frame pairs: FrameInfo and packed words arrive
+// by cp.async.bulk tracked by an mbarrier, two stages deep; 32-bit word shuffle,
+// b-bit codes -> f32 levels, LSB->USB flip of odd samples (src/utils.rs:215-376),
+// integer shift with zero fill (src/utils.rs:126-145), one complex FFT for both
+// stations, two-for-one split (src/utils.rs:47-59).  The correlation itself is in
+// corr_small.cu (FFT 1024..4096), corr_fold.cu (8192, 16384) and the kernels of
+// larger FFTs.
+//
+// reduce_partials_kernel and its wide and batched forms sum the per-CTA partials
+// in a fixed order.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -54,20 +48,15 @@ __device__ __forceinline__ void corr_cta_drain(const SmemLayout& L, uint8_t* sme
   }
 }
 
-// Iterations [it0, it1) (FPC frame pairs each, frames below fend) of the
-// sector described by p; MODE_CORR accumulates into the f64 partials at part
-// ([4][H]).  seq counts the staging iterations this CTA consumed before (the
-// mbarrier slot and phase).  Returns false when a bounded wait gave up.
+// Iterations [it0, it1) (FPC frame pairs each) of the sector described by p into
+// p.out_a, p.out_b.
 template <int N, int FPC, int MODE>
-__device__ __forceinline__ bool corr_span(const CorrParams& p, uint64_t it0, uint64_t it1,
-                                          uint64_t fend, double* part, uint8_t* smem,
-                                          const SmemLayout& L, const Twiddles<N>& tw,
-                                          uint32_t& seq, uint32_t flush_every) {
+__device__ __forceinline__ void stage_span(const CorrParams& p, uint64_t it0, uint64_t it1,
+                                           uint8_t* smem, const SmemLayout& L,
+                                           const Twiddles<N>& tw) {
   constexpr int T1 = N / 16;
   constexpr int T = FPC * T1;
   constexpr int H = N / 2 + 1;
-  constexpr int BPT = (N / 2) / T;
-  static_assert(BPT * T == N / 2 && BPT >= 2, "bins per thread");
 
   float2* bufA = reinterpret_cast<float2*>(smem + L.off_a);
   float2* bufB = reinterpret_cast<float2*>(smem + L.off_b);
@@ -81,7 +70,6 @@ __device__ __forceinline__ bool corr_span(const CorrParams& p, uint64_t it0, uin
   const int tid = threadIdx.x;
   const int g = tid / T1;  // frame slot of this thread in an iteration
   const int t = tid % T1;  // thread index within its frame pair
-  const uint32_t seq0 = seq;
 
   const uint32_t bpf1 = p.st[0].bpf, bpf2 = p.st[1].bpf;
   const uint8_t* raw1 = p.st[0].raw;
@@ -90,9 +78,9 @@ __device__ __forceinline__ bool corr_span(const CorrParams& p, uint64_t it0, uin
   constexpr uint32_t kRaw1 = FPC * kFiBytes;  // offset of station 1 bytes in a slot
 
   auto issue = [&](uint64_t it) {
-    const int slot = (int)((seq0 + (uint32_t)(it - it0)) % kStages);
+    const int slot = (int)((uint32_t)(it - it0) % kStages);
     const uint64_t f0 = it * FPC;
-    const uint64_t nvalid = (fend - f0) < (uint64_t)FPC ? (fend - f0) : (uint64_t)FPC;
+    const uint64_t nvalid = (p.nf - f0) < (uint64_t)FPC ? (p.nf - f0) : (uint64_t)FPC;
     const uint32_t bf = (uint32_t)(nvalid * kFiBytes);
     const uint32_t b1 = (uint32_t)(nvalid * bpf1), b2 = (uint32_t)(nvalid * bpf2);
     uint8_t* dst = stage + slot * L.stage_stride;
@@ -101,9 +89,7 @@ __device__ __forceinline__ bool corr_span(const CorrParams& p, uint64_t it0, uin
     bulk_g2s(dst + kRaw1, raw1 + f0 * bpf1, b1, &bars[slot]);
     bulk_g2s(dst + kRaw1 + FPC * bpf1, raw2 + f0 * bpf2, b2, &bars[slot]);
   };
-  // The previous span, if any, is past its last decode and its last
-  // iteration's barriers: the staging ring and the tables are free.  The
-  // first iterations' copies go out first, the tables are built meanwhile.
+  // The first iterations' copies go out first, the tables are built meanwhile.
   __syncthreads();
   if (tid == 0) {
     fence_proxy_async();
@@ -115,49 +101,16 @@ __device__ __forceinline__ bool corr_span(const CorrParams& p, uint64_t it0, uin
       for (int i = tid; i < 1024; i += T) lut[s * 1024 + i] = p.st[s].shlut[i];
   __syncthreads();
 
-  float acc[BPT + 1][4];
-#pragma unroll
-  for (int i = 0; i <= BPT; ++i)
-#pragma unroll
-    for (int v = 0; v < 4; ++v) acc[i][v] = 0.f;
-  const int a1s = p.a1s, a1e = p.a1e, a2s = p.a2s;
-  const int ov = a1e - a1s;
-  const int sb = a2s - a1s;
-  const int a_gs = p.grid == 0 ? a1s : a2s;  // grid start of the overlap
-  const bool want_acf = (p.products & 1u) != 0;
-  const bool want_xcf = (p.products & 2u) != 0;
-  const bool ov_only = (p.products & 16u) != 0;
-  uint32_t* err = p.err;
-  bool first_flush = true;
-  uint32_t since_flush = 0;
-
-  auto flush = [&]() {
-#pragma unroll
-    for (int i = 0; i <= BPT; ++i) {
-      const int bin = (i < BPT) ? (tid + T * i) : N / 2;
-      if (i == BPT && tid != 0) continue;
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        double* q = part + (size_t)v * H + bin;
-        *q = (first_flush ? 0.0 : *q) + (double)acc[i][v];
-        acc[i][v] = 0.f;
-      }
-    }
-    first_flush = false;
-    since_flush = 0;
-  };
-
-  bool ok = true;
   for (uint64_t it = it0; it < it1; ++it) {
-    const uint32_t q_it = seq0 + (uint32_t)(it - it0);
+    const uint32_t q_it = (uint32_t)(it - it0);
     const int slot = (int)(q_it % kStages);
     const uint32_t parity = (q_it / kStages) & 1u;
     const uint64_t frame_local = it * FPC + g;
-    const bool valid = frame_local < fend;
+    const bool valid = frame_local < p.nf;
 
     if (!mbar_wait(&bars[slot], parity, kWaitPolls)) {
       atomicOr(flag, 1);
-      atomicOr(err, ERR_WAIT_TIMEOUT);
+      atomicOr(p.err, ERR_WAIT_TIMEOUT);
     }
     uint8_t* st = stage + slot * L.stage_stride;
     uint32_t* w1 = reinterpret_cast<uint32_t*>(st + kRaw1);
@@ -167,20 +120,13 @@ __device__ __forceinline__ bool corr_span(const CorrParams& p, uint64_t it0, uin
                     lut + 1024, tid, T);
     if (t == 0 && valid) finfo[g] = reinterpret_cast<const FrameInfo*>(st)[g];
     __syncthreads();
-    if (*flag) {
-      ok = false;
-      break;
-    }
+    if (*flag) break;
     const int s1 = valid ? finfo[g].s1 : 0;
     const int s2 = valid ? finfo[g].s2 : 0;
     const PackedStation pa{w1 + g * (bpf1 / 4), lv, (uint32_t)p.st[0].bits,
                            (1u << p.st[0].bits) - 1u, p.st[0].lsb ? 1 : 0, s1};
-    // MODE_CORR: station 2 enters odd frames negated, undone in the
-    // accumulation, so that the shared FFT's cross-station rounding leak
-    // alternates in sign and cancels over frames instead of biasing the XCF
     const PackedStation pb{w2 + g * (bpf2 / 4), lv + 256, (uint32_t)p.st[1].bits,
-                           (1u << p.st[1].bits) - 1u, p.st[1].lsb ? 1 : 0, s2,
-                           MODE == MODE_CORR ? (uint32_t)(frame_local & 1u) : 0u};
+                           (1u << p.st[1].bits) - 1u, p.st[1].lsb ? 1 : 0, s2};
 
     if constexpr (MODE == MODE_DECODE) {
       if (valid) {
@@ -211,8 +157,6 @@ __device__ __forceinline__ bool corr_span(const CorrParams& p, uint64_t it0, uin
       fence_proxy_async();
       issue(it + kStages);
     }
-    // the final buffer sits at the same offset for every frame slot
-    const bool fin_b = Z0 != za;
     __syncthreads();
 
     if constexpr (MODE == MODE_SPECTRA) {
@@ -229,82 +173,12 @@ __device__ __forceinline__ bool corr_span(const CorrParams& p, uint64_t it0, uin
       __syncthreads();
       continue;
     }
-
-    // ---- MODE_CORR: accumulate every valid frame of the iteration
-#pragma unroll 1
-    for (int f = 0; f < FPC; ++f) {
-      if (it * FPC + f >= fend) break;
-      const float2* Z = (fin_b ? bufB : bufA) + f * Geom<N>::CSTRIDE;
-      const FrameInfo& F = finfo[f];
-      // Ramp rotation of owned bin tid + T*i: SFU sin/cos (|angle| <= ~pi,
-      // absolute error < 4e-7) at i = 0 and i = BPT/2, short recurrences between.
-      float sn, cs;
-      __sincosf(fmaf((float)(tid - a_gs), F.dphi, F.phi0), &sn, &cs);
-      float2 rot = cmul(F.fr_mix, make_float2(cs, sn));
-      __sincosf(fmaf((float)(tid + T * (BPT / 2) - a_gs), F.dphi, F.phi0), &sn, &cs);
-      const float2 rot_half = cmul(F.fr_mix, make_float2(cs, sn));
-      __sincosf((float)T * F.dphi, &sn, &cs);
-      const float2 rstep = make_float2(cs, sn);
-      const float sg = ((it * FPC + f) & 1u) ? -1.0f : 1.0f;  // station 2 sign of this frame
-      auto bin_acc = [&](int bin, float2 r, float* a) {
-        const float2 u = Z[bin], w = Z[(N - bin) & (N - 1)];
-        if (p.grid == 0) {
-          const bool inov = bin >= a1s && bin < a1e;
-          const float2 p1 = make_float2(u.x + w.x, u.y - w.y);  // 2*S1[bin]
-          if (want_acf && (!ov_only || inov)) a[0] += cnorm2(p1);
-          if (inov) {
-            const int i2 = bin + sb;
-            const float2 c = Z[i2], d = Z[(N - i2) & (N - 1)];
-            const float2 q2 = make_float2(sg * (c.y + d.y), sg * (d.x - c.x));  // 2*S2[i2]
-            if (want_acf) a[1] += cnorm2(q2);
-            if (want_xcf) {
-              const float2 x = cmul(cmulc(p1, q2), r);
-              a[2] += x.x;
-              a[3] += x.y;
-            }
-          }
-        } else {
-          const bool inov = bin >= a2s && bin < a2s + ov;
-          const float2 p2 = make_float2(sg * (u.y + w.y), sg * (w.x - u.x));  // 2*S2[bin]
-          if (want_acf && (!ov_only || inov)) a[1] += cnorm2(p2);
-          if (inov) {
-            const int i1 = bin - sb;
-            const float2 c = Z[i1], d = Z[(N - i1) & (N - 1)];
-            const float2 q1 = make_float2(c.x + d.x, c.y - d.y);  // 2*S1[i1]
-            if (want_acf) a[0] += cnorm2(q1);
-            if (want_xcf) {
-              const float2 x = cmul(cmulc(q1, p2), r);
-              a[2] += x.x;
-              a[3] += x.y;
-            }
-          }
-        }
-      };
-#pragma unroll
-      for (int i = 0; i < BPT; ++i) {
-        if (i == BPT / 2) rot = rot_half;
-        bin_acc(tid + T * i, rot, acc[i]);
-        rot = cmul(rot, rstep);
-      }
-      if (tid == 0) {
-        __sincosf(fmaf((float)(N / 2 - a_gs), F.dphi, F.phi0), &sn, &cs);
-        bin_acc(N / 2, cmul(F.fr_mix, make_float2(cs, sn)), acc[BPT]);
-      }
-    }
-    if (++since_flush >= flush_every) flush();
-    __syncthreads();
   }
-  if constexpr (MODE == MODE_CORR) {
-    if (ok && (since_flush > 0 || first_flush)) flush();
-  }
-  seq = seq0 + (uint32_t)(it1 - it0);
-  return ok;
 }
 
 template <int N, int FPC, int MODE>
 __global__ void __launch_bounds__(FPC * N / 16, (N >= 8192 ? 1 : 2))
 corr_kernel(const CorrParams p) {
-  constexpr int H = N / 2 + 1;
   extern __shared__ __align__(128) uint8_t smem[];
   const SmemLayout L = smem_layout<N, FPC>(p.stage_bytes);
   Twiddles<N> tw;
@@ -313,39 +187,7 @@ corr_kernel(const CorrParams p) {
   const uint64_t iters = (p.nf + FPC - 1) / FPC;
   const uint64_t it0 = (blockIdx.x * iters) / gridDim.x;
   const uint64_t it1 = ((blockIdx.x + 1) * iters) / gridDim.x;
-  uint32_t seq = 0;
-  corr_span<N, FPC, MODE>(p, it0, it1, p.nf, p.partials + (size_t)blockIdx.x * 4 * H, smem, L, tw,
-                          seq, p.flush_every);
-  corr_cta_drain(L, smem);
-}
-
-// Batched: a persistent grid takes the items of batch group `grp` by ticket;
-// every item is a frame range of one scan's sector (frames aligned to FPC)
-// with its own partials.  The layout is sized for the largest stage (8-bit
-// stations), so one launch serves every bit depth.
-template <int N, int FPC, int MINB>
-__global__ void __launch_bounds__(FPC * N / 16, MINB) corr_batch_kernel(const BatchArgs a, int grp) {
-  extern __shared__ __align__(128) uint8_t smem[];
-  const SmemLayout L = smem_layout<N, FPC>(2u * FPC * N);
-  if (blockIdx.x >= a.hdr->nitems[grp]) return;  // a graph launches the full grid
-  uint32_t* ticket = reinterpret_cast<uint32_t*>(smem + L.off_flag + 4);
-  Twiddles<N> tw;
-  corr_cta_init<N, FPC>(L, smem, tw);
-  const uint32_t n_items = a.hdr->nitems[grp];
-  const BatchItem* items = a.hdr->items + a.hdr->item0[grp];
-  const BatchScan* scans = a.hdr->scans;
-  uint32_t seq = 0;
-  for (;;) {
-    if (threadIdx.x == 0) *ticket = atomicAdd(&a.hdr->ticket[grp], 1u);
-    __syncthreads();
-    const uint32_t k = *ticket;  // corr_span opens with a barrier before the next write
-    if (k >= n_items) break;
-    const BatchItem w = items[k];
-    // f32 accumulators flushed every 32 frames, whatever the variant
-    if (!corr_span<N, FPC, MODE_CORR>(scans[w.scan].p, w.f0 / FPC, (w.f1 + FPC - 1) / FPC, w.f1,
-                                      a.partials + w.part, smem, L, tw, seq, 32u / FPC))
-      break;
-  }
+  stage_span<N, FPC, MODE>(p, it0, it1, smem, L, tw);
   corr_cta_drain(L, smem);
 }
 
@@ -551,20 +393,19 @@ static cudaError_t launch_one(const CorrParams& p, int grid, cudaStream_t stream
 
 template <int MODE>
 static cudaError_t launch_mode(uint32_t n, const CorrParams& p, int grid, cudaStream_t s) {
-  switch (n) {
-    case 1024: return launch_one<1024, 4, MODE>(p, grid, s);
-    case 2048: return launch_one<2048, 2, MODE>(p, grid, s);
-    case 4096: return launch_one<4096, 1, MODE>(p, grid, s);
-    case 8192:
-      // the FFT-8192 correlation has a kernel of its own (corr_fold.cu)
-      if constexpr (MODE == MODE_CORR) return launch_corr_fold(p, grid, s);
-      else return launch_one<8192, 1, MODE>(p, grid, s);
-    case 16384:
-      // FFT 16384 as two 8192-point rows (corr_fold.cu); other modes and odd
-      // band shifts take the four-step path (large_kernels.cu)
-      if constexpr (MODE == MODE_CORR) return launch_corr_fold2(p, grid, s);
-      else return cudaErrorInvalidValue;
-    default: return cudaErrorInvalidValue;
+  if constexpr (MODE == MODE_CORR) {
+    // FFT 16384 as two 8192-point rows; odd band shifts take other kernels
+    if (n == 8192) return launch_corr_fold(p, grid, s);
+    if (n == 16384) return launch_corr_fold2(p, grid, s);
+    return launch_corr_small(n, p, grid, s);
+  } else {
+    switch (n) {
+      case 1024: return launch_one<1024, 4, MODE>(p, grid, s);
+      case 2048: return launch_one<2048, 2, MODE>(p, grid, s);
+      case 4096: return launch_one<4096, 1, MODE>(p, grid, s);
+      case 8192: return launch_one<8192, 1, MODE>(p, grid, s);
+      default: return cudaErrorInvalidValue;  // the four-step path
+    }
   }
 }
 
@@ -582,59 +423,6 @@ cudaError_t launch_corr(uint32_t n, int mode, const CorrParams& p, int grid, cud
 
 // ------------------------------------------------------- batched launchers
 
-namespace {
-
-// Variants of the batched kernels: FFT length, frames per CTA iteration and
-// resident CTAs per SM (shared memory with 8-bit staging: FPC*N = 1024 ->
-// 32 KB, 2048 -> 54 KB, 4096 -> 95 KB, 8192 -> 183 KB).
-template <int N, int FPC>
-constexpr int batch_minb() {
-  return FPC * N <= 1024 ? 6 : (FPC * N <= 2048 ? 4 : (FPC * N <= 4096 ? 2 : 1));
-}
-
-template <int N, int FPC>
-uint32_t batch_smem() {
-  return smem_layout<N, FPC>(2u * FPC * N).total;
-}
-
-template <int N, int FPC>
-cudaError_t batch_prepare_one() {
-  return cudaFuncSetAttribute(corr_batch_kernel<N, FPC, batch_minb<N, FPC>()>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)batch_smem<N, FPC>());
-}
-
-template <int N, int FPC>
-int batch_ctas_one() {
-  int nb = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, corr_batch_kernel<N, FPC, batch_minb<N, FPC>()>,
-                                                    FPC * N / 16, batch_smem<N, FPC>()) != cudaSuccess)
-    return 0;
-  return nb;
-}
-
-template <int N, int FPC>
-cudaError_t batch_launch_one(const BatchArgs& a, int grp, int grid, cudaStream_t s) {
-  corr_batch_kernel<N, FPC, batch_minb<N, FPC>()><<<grid, FPC * N / 16, batch_smem<N, FPC>(), s>>>(a, grp);
-  return cudaGetLastError();
-}
-
-// Calls f.template operator()<N, FPC>() for the variant (g, fpc); returns
-// cudaErrorInvalidValue for a variant that does not exist.
-#define FXC_BATCH_VARIANTS(g, fpc, CALL)              \
-  switch ((g) * 16 + (fpc)) {                         \
-    case BG_1024 * 16 + 1: return CALL(1024, 1);      \
-    case BG_1024 * 16 + 2: return CALL(1024, 2);      \
-    case BG_1024 * 16 + 4: return CALL(1024, 4);      \
-    case BG_2048 * 16 + 1: return CALL(2048, 1);      \
-    case BG_2048 * 16 + 2: return CALL(2048, 2);      \
-    case BG_2048 * 16 + 4: return CALL(2048, 4);      \
-    case BG_4096 * 16 + 1: return CALL(4096, 1);      \
-    case BG_4096 * 16 + 2: return CALL(4096, 2);      \
-    default: break;                                   \
-  }
-
-}  // namespace
-
 uint32_t fold_batch_smem_bytes(int rows);
 cudaError_t prepare_fold_batch(int rows);
 cudaError_t launch_fold_batch(int rows, const BatchArgs& a, int grp, int grid, cudaStream_t s);
@@ -642,27 +430,18 @@ int fold_batch_ctas_per_sm(int rows);
 
 cudaError_t batch_prepare(int g, int fpc) {
   if (g == BG_8192 || g == BG_16384) return prepare_fold_batch(g == BG_8192 ? 1 : 2);
-#define FXC_PREP(N, F) batch_prepare_one<N, F>()
-  FXC_BATCH_VARIANTS(g, fpc, FXC_PREP)
-#undef FXC_PREP
-  return cudaErrorInvalidValue;
+  return small_batch_prepare(g, fpc);
 }
 
 int batch_group_ctas_per_sm(int g, int fpc) {
   if (g == BG_8192 || g == BG_16384) return fold_batch_ctas_per_sm(g == BG_8192 ? 1 : 2);
-#define FXC_CTAS(N, F) batch_ctas_one<N, F>()
-  FXC_BATCH_VARIANTS(g, fpc, FXC_CTAS)
-#undef FXC_CTAS
-  return 0;
+  return small_batch_ctas_per_sm(g, fpc);
 }
 
 cudaError_t launch_batch_group(int g, int fpc, const BatchArgs& a, int grid, cudaStream_t s) {
   if (grid <= 0) return cudaErrorInvalidValue;
   if (g == BG_8192 || g == BG_16384) return launch_fold_batch(g == BG_8192 ? 1 : 2, a, g, grid, s);
-#define FXC_LAUNCH(N, F) batch_launch_one<N, F>(a, g, grid, s)
-  FXC_BATCH_VARIANTS(g, fpc, FXC_LAUNCH)
-#undef FXC_LAUNCH
-  return cudaErrorInvalidValue;
+  return launch_small_batch(g, fpc, a, grid, s);
 }
 
 cudaError_t launch_batch_frame_info(const BatchArgs& a, int grid, cudaStream_t s) {

@@ -26,12 +26,13 @@ constexpr uint32_t kTabPos = 4096, kTabLut = 4608, kTabEnd = kTabLut + 8192;
 // preA / preB: the station's words are rewritten in place by its byte LUTs
 // before decoding (4- and 8-bit stations with a non-identity shuffle), so its
 // rotate amounts are those of the natural bit order.
-__device__ __forceinline__ void build_decode_tables(const StationParams& sa, const StationParams& sb,
-                                                    bool preA, bool preB, uint8_t* smem, int tid,
-                                                    int nthreads) {
+// `lut`: where the byte LUTs go.
+__device__ __forceinline__ void build_decode_tables_at(const StationParams& sa,
+                                                       const StationParams& sb, bool preA,
+                                                       bool preB, uint8_t* smem, uint32_t* lut,
+                                                       int tid, int nthreads) {
   float* lv = reinterpret_cast<float*>(smem);
   uint32_t* pos = reinterpret_cast<uint32_t*>(smem + kTabPos);
-  uint32_t* lut = reinterpret_cast<uint32_t*>(smem + kTabLut);
   for (int i = tid; i < 1024; i += nthreads) {
     // per station: 2^b levels, then their negations (the two sign groups of a
     // warp's table loads fall in different banks)
@@ -59,6 +60,13 @@ __device__ __forceinline__ void build_decode_tables(const StationParams& sa, con
     if ((k ? preB : preA) && q.shkind == SH_GENERIC)
       for (int i = tid; i < 1024; i += nthreads) lut[k * 1024 + i] = q.shlut[i];
   }
+}
+
+__device__ __forceinline__ void build_decode_tables(const StationParams& sa, const StationParams& sb,
+                                                    bool preA, bool preB, uint8_t* smem, int tid,
+                                                    int nthreads) {
+  build_decode_tables_at(sa, sb, preA, preB, smem, reinterpret_cast<uint32_t*>(smem + kTabLut), tid,
+                         nthreads);
 }
 
 // A 2-bit shuffle keeps every sample's two bits adjacent and in order, or it

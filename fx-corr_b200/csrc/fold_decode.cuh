@@ -109,5 +109,70 @@ __device__ __forceinline__ void fold_station(int bits, bool split, const uint32_
   }
 }
 
+// The same for a frame of one row of N points (N/16 threads; FFT 1024..4096):
+// samples x[t + r N/16 - shift], r < 16.  The zero fill is checked for a half of
+// them only where the frame's shift reaches into it.
+template <int N, int BITS, bool IMAG, bool SPLIT>
+__device__ __forceinline__ void row_inputs(const uint32_t* __restrict__ words, const uint8_t* lvbase,
+                                           int shift, uint32_t rots, uint32_t tbase,
+                                           float2 (&v)[16], int t) {
+  constexpr int T1 = N / 16;
+  constexpr int SPW = 32 / BITS;
+  constexpr int LOG2_SPW = BITS == 1 ? 5 : (BITS == 2 ? 4 : (BITS == 4 ? 3 : 2));
+  constexpr int WSTEP = T1 / SPW;
+  constexpr uint32_t OMASK = ((1u << BITS) - 1u) << 2;
+  static_assert(T1 % SPW == 0, "frame stride is a whole number of words");
+  const int m0 = t - shift;
+  const int w0 = m0 >> LOG2_SPW;  // floor division
+  const uint32_t r0 = rots & 31u, r1 = (rots >> 8) & 31u;
+  auto level = [&](uint32_t w) -> float {
+    uint32_t off;
+    if constexpr (SPLIT) {
+      off = (__funnelshift_r(w, w, r0) & 4u) | tbase;
+      off |= __funnelshift_r(w, w, r1) & 8u;
+    } else {
+      off = (__funnelshift_r(w, w, r0) & OMASK) | tbase;
+    }
+    return *reinterpret_cast<const float*>(lvbase + off);
+  };
+  const uint32_t* w = words + w0;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    // samples of the half, over all threads of the frame: 8 h T1 - shift up to
+    // 8 (h + 1) T1 - 1 - shift
+    const bool inside = h == 0 ? (shift <= 0 && shift > -8 * T1) : (shift >= 0 && shift < 8 * T1);
+    if (inside) {
+#pragma unroll
+      for (int r = 8 * h; r < 8 * h + 8; ++r) {
+        const float x = level(w[r * WSTEP]);
+        if (IMAG) v[r].y = x; else v[r].x = x;
+      }
+    } else {
+#pragma unroll
+      for (int r = 8 * h; r < 8 * h + 8; ++r) {
+        const bool in = (unsigned)(m0 + r * T1) < (unsigned)N;
+        float x = level(words[in ? w0 + r * WSTEP : 0]);
+        x = in ? x : 0.0f;
+        if (IMAG) v[r].y = x; else v[r].x = x;
+      }
+    }
+  }
+}
+
+template <int N, bool IMAG>
+__device__ __forceinline__ void row_station(int bits, bool split, const uint32_t* words,
+                                            const uint8_t* lvbase, int shift, uint32_t rots,
+                                            uint32_t tbase, float2 (&v)[16], int t) {
+  switch (bits) {
+    case 1: row_inputs<N, 1, IMAG, false>(words, lvbase, shift, rots, tbase, v, t); break;
+    case 2:
+      if (split) row_inputs<N, 2, IMAG, true>(words, lvbase, shift, rots, tbase, v, t);
+      else row_inputs<N, 2, IMAG, false>(words, lvbase, shift, rots, tbase, v, t);
+      break;
+    case 4: row_inputs<N, 4, IMAG, false>(words, lvbase, shift, rots, tbase, v, t); break;
+    default: row_inputs<N, 8, IMAG, false>(words, lvbase, shift, rots, tbase, v, t); break;
+  }
+}
+
 }  // namespace fold
 }  // namespace fxc

@@ -67,6 +67,13 @@ struct PhasedParams {
 int corr_frames_per_cta_iter(uint32_t n);
 int corr_ctas_per_sm(uint32_t n);
 cudaError_t launch_corr(uint32_t n, int mode, const CorrParams& p, int grid, cudaStream_t s);
+// FFT 1024..4096 correlation (MODE_CORR; corr_small.cu), corr_frames_per_cta_iter
+// frame pairs per CTA iteration; its batched form by variant (batch_prepare etc.)
+cudaError_t launch_corr_small(uint32_t n, const CorrParams& p, int grid, cudaStream_t s);
+cudaError_t small_batch_prepare(int g, int fpc);
+int small_batch_ctas_per_sm(int g, int fpc);
+struct BatchArgs;
+cudaError_t launch_small_batch(int g, int fpc, const BatchArgs& a, int grid, cudaStream_t s);
 // FFT-8192 correlation (MODE_CORR), one frame pair per CTA iteration (corr_fold.cu)
 cudaError_t launch_corr_fold(const CorrParams& p, int grid, cudaStream_t s);
 // FFT-8192 decode + integer shift through the correlation kernel's own decode

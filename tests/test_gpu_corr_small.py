@@ -1,0 +1,82 @@
+"""The FFT 1024..4096 correlation kernel against the FP64 oracle where its decode
+and accumulation change form: integer shifts at the edges of the half of a frame
+that is decoded unchecked, every bit depth and shuffle class, both grids, band
+shifts of either sign, none, and overlaps that end inside a warp's bins, frame
+counts that do not fill a CTA iteration, each product subset.  Tolerance of
+_cases.py."""
+import numpy as np
+import pytest
+
+import oracle
+from _cases import assert_sector_close, make_scan, signal_raw, to_fxc
+
+pytestmark = pytest.mark.gpu
+
+CORR = oracle.PROD_ACF | oracle.PROD_XCF
+
+
+def dev(a):
+    import torch
+
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def check(engine, scan, nf, seed, what):
+    r1, r2 = signal_raw(scan, nf, seed=seed, rho=0.3, delay_samples=2.6)
+    s = engine.open_scan(to_fxc(scan))
+    got = s.sector_device(dev(r1), dev(r2), nf, first_frame=3)
+    s.close()
+    ref = oracle.fp64_sector_corr(scan, r1, r2, nf, first_frame=3)
+    full = oracle.fp64_sector_corr(
+        __import__("dataclasses").replace(scan, products=CORR), r1, r2, nf, first_frame=3)
+    assert_sector_close(got, ref, scan, what, nf=nf, ref_acf=full)
+    if not scan.products & oracle.PROD_ACF:
+        assert not np.any(got["acf11"]) and not np.any(got["acf22"])
+    if not scan.products & oracle.PROD_XCF:
+        assert not np.any(got["xcf"])
+
+
+def delays(fs, s1, s2):
+    return dict(net_d1_base=s1 / fs + 0.2 / fs, net_d2_base=s2 / fs - 0.1 / fs,
+                lo1_hz=8.4e9, lo2_hz=8.4e9)
+
+
+@pytest.mark.parametrize("fft", [1024, 2048, 4096])
+@pytest.mark.parametrize("edge", [0, 1, 511, 512, 513, 1023, 1025])
+def test_shift_edges(engine, fft, edge):
+    # in 1024ths of a frame: 512 is half a frame, 8 N/16 samples
+    s = edge * (fft // 1024) + (edge % 2) * (fft // 1024 - 1)
+    fs = 512e6
+    for s1, s2 in ((s, -s), (-s, s)):
+        scan = make_scan(fft=fft, fs=fs, delay=delays(fs, s1, s2), shuffle="generic", lsb1=True)
+        check(engine, scan, 9, fft + edge, f"shifts {s1} {s2}")
+
+
+@pytest.mark.parametrize("fft", [1024, 2048, 4096])
+@pytest.mark.parametrize("bits1,bits2,shuffle", [
+    (1, 1, "generic"), (1, 2, "identity"), (2, 2, "pairswap"), (2, 2, "sample2"),
+    (2, 2, "generic"), (4, 2, "generic"), (4, 4, "identity"), (8, 8, "generic"),
+    (8, 1, "pairswap")])
+def test_depths_and_shuffles(engine, fft, bits1, bits2, shuffle):
+    fs = 512e6
+    for lsb in ((False, False), (True, False), (True, True)):
+        scan = make_scan(fft=fft, fs=fs, bits1=bits1, bits2=bits2, shuffle=shuffle,
+                         lsb1=lsb[0], lsb2=lsb[1], delay=delays(fs, 37, -5),
+                         band=(3, 0, fft // 2 - 7, 3))
+        check(engine, scan, 7, fft + 10 * bits1 + bits2, f"{bits1}/{bits2} {shuffle} {lsb}")
+
+
+@pytest.mark.parametrize("fft", [1024, 2048, 4096])
+@pytest.mark.parametrize("grid", [0, 1])
+@pytest.mark.parametrize("products", [CORR, oracle.PROD_XCF, oracle.PROD_ACF,
+                                      oracle.PROD_ACF | oracle.PROD_ACF_OVERLAP_ONLY])
+def test_bands_and_products(engine, fft, grid, products):
+    h = fft // 2
+    fs = 512e6
+    # no shift over every bin; either sign; an odd shift; an overlap of one bin; one
+    # that ends inside a warp
+    for band in ((0, 0, h + 1, 0), (5, 0, h - 5, 5), (-7, 7, h, 0), (h // 2, 0, h // 2 + 1, h // 2),
+                 (0, 17, 18, 17), (-3, 100, 133, 97)):
+        scan = make_scan(fft=fft, fs=fs, grid=grid, band=band, products=products,
+                         delay=delays(fs, 11, 4))
+        check(engine, scan, 10, fft + grid, f"grid {grid} band {band} products {products}")
