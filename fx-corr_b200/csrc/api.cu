@@ -1059,11 +1059,10 @@ fxc_status fxc_sector_run_device(fxc_scan* s, const uint8_t* d_raw1, const uint8
 fxc_status fxc_scan_check(fxc_scan* s) {
   if (!s) return fail(FXC_EINVAL, "scan is NULL");
   DeviceGuard g(s->eng->device);
-  CK(cudaStreamSynchronize(s->stream));
-  CK(cudaDeviceSynchronize());
+  CK(cudaDeviceSynchronize());  // the scan's streams and the caller's
   uint32_t err = 0;
   CK(cudaMemcpy(&err, s->d_err, 4, cudaMemcpyDeviceToHost));
-  CK(cudaMemset(s->d_err, 0, 4));
+  if (err) CK(cudaMemset(s->d_err, 0, 4));
   return internal_device_error(err);
 }
 
