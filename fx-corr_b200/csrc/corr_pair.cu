@@ -242,7 +242,6 @@ __global__ void __cluster_dims__(C / 2, 1, 1) __launch_bounds__(kT, 1)
   const bool want_acf = (p.products & 1u) != 0;
   const bool want_xcf = (p.products & 2u) != 0;
   const bool ov_only = (p.products & 16u) != 0;
-  const float xconj = g0 ? 1.0f : -1.0f;  // XCF = S1 conj(S2): conj(P conj(S)) for grid 1
   const int lsbP = sp.lsb ? 1 : 0, lsbS = ss.lsb ? 1 : 0;
   const int colP = g0 ? 0 : 1, colS = g0 ? 1 : 0;  // output columns of the two ACFs
   const bool half = r == 0 && tid == 0;            // bin N/2 (row 0, index M/2)
@@ -255,23 +254,28 @@ __global__ void __cluster_dims__(C / 2, 1, 1) __launch_bounds__(kT, 1)
   // registers.  v: primary ACF, secondary ACF (at the primary bin), XCF re, im.
   float acc_h[4] = {0.f, 0.f, 0.f, 0.f};
 
+  // Every sum runs for every bin: out of the overlap the secondary spectrum is
+  // zero, and the products that were not asked for are left out here.  (Predicates
+  // per bin and product, and the odd frames' sign on every secondary value: FFT
+  // 16384 odd shift, 8001 frame pairs 736 -> 711 us 1-bit, 786 -> 754 us 2-bit; 32768
+  // (6000) 1209 -> 1176; 65536 (3001) 1413 -> 1375 us.)
   auto add_part = [&](int bin, int v, float x) {
     const int col = v == 0 ? colP : (v == 1 ? colS : v);
+    const bool in = (unsigned)(bin - ovs) < (unsigned)ov;
+    if (v == 0 ? !(want_acf && (!ov_only || in)) : (v == 1 ? !want_acf : !want_xcf)) x = 0.f;
+    if (v == 3 && !g0) x = -x;  // grid 1: the conjugate was summed
     double* d = part + (size_t)col * H + bin;
     *d = (first_flush ? 0.0 : *d) + (double)x;
   };
   auto bin_acc = [&](int bin, const float2* qp, float2 pv, float2 rt, float* a) {
-    const bool inov = (unsigned)(bin - ovs) < (unsigned)ov;
-    if (want_acf && (!ov_only || inov)) a[0] = fmaf(pv.x, pv.x, fmaf(pv.y, pv.y, a[0]));
-    if (inov) {
-      const float2 qv = *qp;
-      if (want_acf) a[1] = fmaf(qv.x, qv.x, fmaf(qv.y, qv.y, a[1]));
-      if (want_xcf) {
-        float2 x = cmulc(pv, qv);
-        x.y *= xconj;
-        a[2] = fmaf(x.x, rt.x, fmaf(-x.y, rt.y, a[2]));
-        a[3] = fmaf(x.x, rt.y, fmaf(x.y, rt.x, a[3]));
-      }
+    float2 qv = make_float2(0.f, 0.f);
+    if ((unsigned)(bin - ovs) < (unsigned)ov) qv = *qp;
+    a[0] = fmaf(pv.x, pv.x, fmaf(pv.y, pv.y, a[0]));
+    a[1] = fmaf(qv.x, qv.x, fmaf(qv.y, qv.y, a[1]));
+    if (want_xcf) {
+      const float2 x = cmulc(pv, qv);
+      a[2] = fmaf(x.x, rt.x, fmaf(-x.y, rt.y, a[2]));
+      a[3] = fmaf(x.x, rt.y, fmaf(x.y, rt.x, a[3]));
     }
   };
   // the secondary spectra: row A's at XB[0 .. M/2], row B's at XB[M/2 + 1 ..]
@@ -302,7 +306,7 @@ __global__ void __cluster_dims__(C / 2, 1, 1) __launch_bounds__(kT, 1)
       const bool inP = aP >= 0 && aP + CW <= kM, inS = aS >= 0 && aS + CW <= kM;
       const int cP = mP & ((32 / bitsP) - 1), cS = mS & ((32 / bitsS) - 1);
       const uint32_t tbP = (uint32_t)((mP & lsbP) << (bitsP + 2));
-      // the secondary station enters odd frames negated (undone by sgn below)
+      // the secondary station enters odd frames negated (undone in the ramp)
       const uint32_t tbS = 2048u + (uint32_t)((((uint32_t)mS & (uint32_t)lsbS) ^ (uint32_t)(it & 1u))
                                               << (bitsS + 2));
       auto rows_out = [&](float2 (&v)[16], auto ub) {
@@ -379,12 +383,16 @@ __global__ void __cluster_dims__(C / 2, 1, 1) __launch_bounds__(kT, 1)
     // shift is a multiple of C), then the accumulation into TMEM.  Rounding
     // in the shared complex FFT leaks a fixed fraction (~1e-6) of each
     // station's spectrum into the other's; the secondary's odd-frame negation
-    // (undone by sgn) makes it alternate in sign and cancel over frames.
-    const float sgn = (it & 1u) ? -1.0f : 1.0f;
+    // (undone in the ramp) makes it alternate in sign and cancel over frames.
+    // XCF = S1 conj(S2): P conj(S) times the ramp for grid 0; for grid 1 its
+    // conjugate is summed, P conj(S) times the ramp's conjugate.
+    const float sgn = (it & 1u) ? -1.0f : 1.0f, cj = g0 ? 1.0f : -1.0f;
     const FrameInfo& F = finfo[fb];
+    const float dphi = cj * F.dphi, phi0 = cj * F.phi0;
+    const float2 mix = make_float2(sgn * F.fr_mix.x, sgn * cj * F.fr_mix.y);
     const bool flush_now = ++since_flush >= flush_every;
     float sn, cs;
-    __sincosf((float)(C * kT) * F.dphi, &sn, &cs);
+    __sincosf((float)(C * kT) * dphi, &sn, &cs);
     const float2 rstep = make_float2(cs, sn);
     if constexpr (C == 2) {
       // Slot of primary bin kp's secondary spectrum: with both rows in the CTA,
@@ -428,14 +436,14 @@ __global__ void __cluster_dims__(C / 2, 1, 1) __launch_bounds__(kT, 1)
           prim[i] = make_float2(u.x + w.x, u.y - w.y);
           const int kp = C * j + row - qoff;
           if ((unsigned)(kp - ovs) < (unsigned)ov)
-            *q_slot(kp) = make_float2(sgn * (u.y + w.y), sgn * (w.x - u.x));
+            *q_slot(kp) = make_float2(u.y + w.y, w.x - u.x);
         }
         if (RB == 0 && half) {  // Z[N/2] = Y[0] - Y[M/2] pairs with itself
           const float2 u = csub(Y[0], Y[kM / 2]);
           prim_h = make_float2(2.f * u.x, 0.f);
           const int kp = N / 2 - qoff;
           if ((unsigned)(kp - ovs) < (unsigned)ov)
-            *q_slot(kp) = make_float2(sgn * 2.f * u.y, 0.f);
+            *q_slot(kp) = make_float2(2.f * u.y, 0.f);
         }
       };
       // accumulation of a row's bins into TMEM (its secondary spectra in place)
@@ -444,12 +452,12 @@ __global__ void __cluster_dims__(C / 2, 1, 1) __launch_bounds__(kT, 1)
         const int row = RB ? rowB : rowA;
         const float2* Q = RB ? QB : QA;
         // fringe x ramp rotation of the thread's bins of this row
-        __sincosf(fmaf((float)(C * tid + row - ovs), F.dphi, F.phi0), &sn, &cs);
-        float2 rot = cmul(F.fr_mix, make_float2(cs, sn));
+        __sincosf(fmaf((float)(C * tid + row - ovs), dphi, phi0), &sn, &cs);
+        float2 rot = cmul(mix, make_float2(cs, sn));
         float2 rhalf = make_float2(0.f, 0.f);
         if (RB == 0 && half) {
-          __sincosf(fmaf((float)(N / 2 - ovs), F.dphi, F.phi0), &sn, &cs);
-          rhalf = cmul(F.fr_mix, make_float2(cs, sn));
+          __sincosf(fmaf((float)(N / 2 - ovs), dphi, phi0), &sn, &cs);
+          rhalf = cmul(mix, make_float2(cs, sn));
         }
         float t[32];
         tmem_ld32(taddr + (uint32_t)(32 * RB), t);
@@ -533,22 +541,22 @@ __global__ void __cluster_dims__(C / 2, 1, 1) __launch_bounds__(kT, 1)
           prim[i] = make_float2(u.x + w.x, u.y - w.y);
           const int kp = C * j + row - qoff;
           if ((unsigned)(kp - ovs) < (unsigned)ov)
-            Q[j + dq] = make_float2(sgn * (u.y + w.y), sgn * (w.x - u.x));
+            Q[j + dq] = make_float2(u.y + w.y, w.x - u.x);
         }
         float2 prim_h = make_float2(0.f, 0.f);
         if (RB == 0 && half) {  // Z[N/2] = Y[0] - Y[M/2] pairs with itself
           const float2 u = csub(Y[0], Y[kM / 2]);
           prim_h = make_float2(2.f * u.x, 0.f);
           const int kp = N / 2 - qoff;
-          if ((unsigned)(kp - ovs) < (unsigned)ov) Q[kM / 2 + dq] = make_float2(sgn * 2.f * u.y, 0.f);
+          if ((unsigned)(kp - ovs) < (unsigned)ov) Q[kM / 2 + dq] = make_float2(2.f * u.y, 0.f);
         }
         // fringe x ramp rotation of the thread's bins of this row
-        __sincosf(fmaf((float)(C * tid + row - ovs), F.dphi, F.phi0), &sn, &cs);
-        float2 rot = cmul(F.fr_mix, make_float2(cs, sn));
+        __sincosf(fmaf((float)(C * tid + row - ovs), dphi, phi0), &sn, &cs);
+        float2 rot = cmul(mix, make_float2(cs, sn));
         float2 rhalf = make_float2(0.f, 0.f);
         if (RB == 0 && half) {
-          __sincosf(fmaf((float)(N / 2 - ovs), F.dphi, F.phi0), &sn, &cs);
-          rhalf = cmul(F.fr_mix, make_float2(cs, sn));
+          __sincosf(fmaf((float)(N / 2 - ovs), dphi, phi0), &sn, &cs);
+          rhalf = cmul(mix, make_float2(cs, sn));
         }
         __syncthreads();  // this row's secondary spectra are in place
         float t[32];
