@@ -478,11 +478,9 @@ fxc_status run_large(fxc_scan* s, const uint8_t* r1, const uint8_t* r2, uint64_t
                      0.25 * u1 * u2, d_acc, st));
     s->all_launches += 1;
     s->kernel_launches += 1;
-  } else if (!corr_done) {
-    CK(cudaMemsetAsync(d_acc, 0, sizeof(double) * 5 * h, st));
   }
   if (phased) {
-    CK(launch_reduce_phased(part_ph, groups, (int)h, d_acc, st));
+    CK(launch_reduce_phased(part_ph, groups, (int)h, !corr && !corr_done, d_acc, st));
     s->all_launches += 1;
   }
   return FXC_OK;
@@ -520,20 +518,18 @@ fxc_status run_sector_device(fxc_scan* s, const uint8_t* r1, const uint8_t* r2, 
     if (phased) {
       const PhasedParams pp = phased_params(s, r1, r2, nf, first, d_raw_out);
       if (phased_pair_supported(s->n, pp)) {
-        if (!corr) CK(cudaMemsetAsync(d_acc, 0, sizeof(double) * 5 * h, st));
         const int g = phased_pair_grid(s->eng->sm_count, nf);
         CK(launch_phased_pair(pp, g, st));
-        CK(launch_reduce_phased(s->d_partials, g, (int)h, d_acc, st));
+        CK(launch_reduce_phased(s->d_partials, g, (int)h, !corr, d_acc, st));
         s->all_launches += 2;
         return run_large(s, r1, r2, nf, first, d_acc, d_raw_out, corr && !corr_done, false, true,
                          st);
       }
       if (phased_cpair_supported(s->n, pp)) {
-        if (!corr) CK(cudaMemsetAsync(d_acc, 0, sizeof(double) * 5 * h, st));
         if (pp.want_raw) CK(cudaMemsetAsync(d_raw_out, 0, (size_t)nf * s->bpfo, st));
         const int g = phased_cpair_count(s->n, nf);
         CK(launch_phased_cpair(s->n, pp, g, st));
-        CK(launch_reduce_phased(s->d_partials, g, (int)h, d_acc, st));
+        CK(launch_reduce_phased(s->d_partials, g, (int)h, !corr, d_acc, st));
         s->all_launches += 2;
         return run_large(s, r1, r2, nf, first, d_acc, d_raw_out, corr && !corr_done, false, true,
                          st);
@@ -542,16 +538,14 @@ fxc_status run_sector_device(fxc_scan* s, const uint8_t* r1, const uint8_t* r2, 
     return run_large(s, r1, r2, nf, first, d_acc, d_raw_out, corr && !corr_done, phased, corr_done,
                      st);
   }
-  if (!corr) {
-    CK(cudaMemsetAsync(d_acc, 0, sizeof(double) * 5 * h, st));
-  } else {
+  if (corr) {
     fst = run_corr_stage(s, r1, r2, nf, first, grid, d_acc, st);
     if (fst != FXC_OK) return fst;
   }
   if (phased) {
     PhasedParams pp = phased_params(s, r1, r2, nf, first, d_raw_out);
     CK(launch_phased(s->n, pp, grid, st));
-    CK(launch_reduce_phased(s->d_partials, grid, (int)h, d_acc, st));
+    CK(launch_reduce_phased(s->d_partials, grid, (int)h, !corr, d_acc, st));
     s->all_launches += 2;
   }
   return FXC_OK;

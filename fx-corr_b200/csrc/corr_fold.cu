@@ -467,7 +467,9 @@ __global__ void __launch_bounds__(kT, 1) corr_fold_kernel(const CorrParams p, in
   extern __shared__ __align__(128) uint8_t smem[];
   const FoldLayout L = fold_layout(p.stage_bytes);
   FoldCta<ROWS> c;
+  grid_dependents();
   fold_cta_init<ROWS>(smem, c);
+  grid_wait();  // the frame records (row 1: and row 0's kernel)
   const uint64_t iters = p.nf;
   const uint64_t it0 = (blockIdx.x * iters) / gridDim.x;
   const uint64_t it1 = ((blockIdx.x + 1) * iters) / gridDim.x;
@@ -577,8 +579,7 @@ cudaError_t launch_corr_fold(const CorrParams& p, int grid, cudaStream_t stream)
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)fold_smem_bytes(2u * kN));
   if (e != cudaSuccess) return e;
-  corr_fold_kernel<1><<<grid, kT, smem, stream>>>(p, 0);
-  return cudaGetLastError();
+  return launch_dependent(corr_fold_kernel<1>, dim3(grid), kT, smem, stream, p, 0);
 }
 
 bool corr_fold2_supported(const CorrParams& p) {
@@ -593,8 +594,8 @@ cudaError_t launch_corr_fold2(const CorrParams& p, int grid, cudaStream_t stream
                                        (int)fold_smem_bytes(4u * kN));
   if (e != cudaSuccess) return e;
   for (int row = 0; row < 2; ++row) {
-    corr_fold_kernel<2><<<grid, kT, smem, stream>>>(p, row);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    e = launch_dependent(corr_fold_kernel<2>, dim3(grid), kT, smem, stream, p, row);
+    if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
 }

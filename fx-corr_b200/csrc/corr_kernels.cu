@@ -242,6 +242,7 @@ reduce_partials_wide_kernel(const double* __restrict__ part, int nblk, int h, do
                             double m22, double m12, double* __restrict__ out) {
   __shared__ double sm[32][kRedBins];
   const int k = blockIdx.x * kRedBins + (threadIdx.x & 31), v = blockIdx.y;
+  grid_wait();
   const double t = reduce_column<32>(part + (size_t)v * h, nblk, (size_t)4 * h, k, k < h, sm);
   if (threadIdx.x < kRedBins && k < h) reduce_store(v, k, h, t, m11, m22, m12, out);
 }
@@ -255,6 +256,7 @@ reduce_partials_kernel(const double* __restrict__ part, int nblk, int h, double 
   const int k = blockIdx.x * kRedBins + lane;
   const int b0 = (nblk * grp) / 8, b1 = (nblk * (grp + 1)) / 8;
   double s[4] = {0, 0, 0, 0};
+  grid_wait();
   if (k < h) {
     for (int b = b0; b < b1; ++b) {
       const double* q = part + (size_t)b * 4 * h + k;
@@ -278,11 +280,18 @@ reduce_partials_kernel(const double* __restrict__ part, int nblk, int h, double 
 // Fixed-order sum of the per-CTA phased partials into acc[4H, 5H).
 template <int WARPS>
 __global__ void __launch_bounds__(kRedBins * WARPS)
-reduce_phased_kernel(const double* __restrict__ part, int nblk, int h, double* __restrict__ out) {
+reduce_phased_kernel(const double* __restrict__ part, int nblk, int h, int zero,
+                     double* __restrict__ out) {
   __shared__ double sm[WARPS][kRedBins];
   const int k = blockIdx.x * kRedBins + (threadIdx.x & 31);
+  grid_wait();
   const double t = reduce_column<WARPS>(part, nblk, (size_t)h, k, k < h, sm);
-  if (threadIdx.x < kRedBins && k < h) out[4 * (size_t)h + k] = t;
+  if (threadIdx.x >= kRedBins || k >= h) return;
+  out[4 * (size_t)h + k] = t;
+  if (zero) {
+    out[k] = out[(size_t)h + k] = 0.0;
+    out[2 * (size_t)h + 2 * k] = out[2 * (size_t)h + 2 * k + 1] = 0.0;
+  }
 }
 
 __global__ void delay_entries_kernel(const DelayParams p, uint64_t first, uint64_t nf,
@@ -307,6 +316,7 @@ __global__ void delay_entries_kernel(const DelayParams p, uint64_t first, uint64
 
 __global__ void frame_info_kernel(const DelayParams p, uint64_t first, uint64_t nf, int n,
                                   double df_hz, int a1s, int a2s, FrameInfo* out) {
+  grid_dependents();
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nf) return;
   FrameInfo fi;
@@ -458,20 +468,19 @@ cudaError_t launch_reduce(const double* part, int nblk, int h, double m11, doubl
                           double* out, cudaStream_t s) {
   const int grid = (h + kRedBins - 1) / kRedBins;
   if (nblk >= kRedWideSlots)
-    reduce_partials_wide_kernel<<<dim3(grid, 4), kRedBins * 32, 0, s>>>(part, nblk, h, m11, m22,
-                                                                        m12, out);
-  else
-    reduce_partials_kernel<<<grid, kRedBins * 8, 0, s>>>(part, nblk, h, m11, m22, m12, out);
-  return cudaGetLastError();
+    return launch_dependent(reduce_partials_wide_kernel, dim3(grid, 4), kRedBins * 32, 0, s, part,
+                            nblk, h, m11, m22, m12, out);
+  return launch_dependent(reduce_partials_kernel, dim3(grid), kRedBins * 8, 0, s, part, nblk, h, m11,
+                          m22, m12, out);
 }
 
-cudaError_t launch_reduce_phased(const double* part, int nblk, int h, double* out, cudaStream_t s) {
-  const int grid = (h + kRedBins - 1) / kRedBins;
+cudaError_t launch_reduce_phased(const double* part, int nblk, int h, bool zero, double* out,
+                                 cudaStream_t s) {
+  const dim3 grid((h + kRedBins - 1) / kRedBins);
+  const int z = zero ? 1 : 0;
   if (nblk >= kRedWideSlots)
-    reduce_phased_kernel<32><<<grid, kRedBins * 32, 0, s>>>(part, nblk, h, out);
-  else
-    reduce_phased_kernel<8><<<grid, kRedBins * 8, 0, s>>>(part, nblk, h, out);
-  return cudaGetLastError();
+    return launch_dependent(reduce_phased_kernel<32>, grid, kRedBins * 32, 0, s, part, nblk, h, z, out);
+  return launch_dependent(reduce_phased_kernel<8>, grid, kRedBins * 8, 0, s, part, nblk, h, z, out);
 }
 
 cudaError_t launch_delay_entries(const DelayParams& p, uint64_t first, uint64_t nf,

@@ -185,6 +185,8 @@ __global__ void __cluster_dims__(C / 2, 1, 1) __launch_bounds__(kT, 1)
     tmem_st32(taddr, z);
     tmem_st32(taddr + 32u, z);
   }
+  grid_dependents();
+  grid_wait();  // the frame records
   if (tid < 32 && it0 < it1) {
     int a, b;
     shifts(it0, &a, &b);
@@ -680,17 +682,15 @@ cudaError_t launch_corr_pair(uint32_t n, const CorrParams& p, int clusters, cuda
   cudaError_t e;
   if (n == 16384) {
     if ((e = pair_prepare<2>()) != cudaSuccess) return e;
-    corr_pair_kernel<2><<<clusters, kT, pr_smem_bytes(2, bp, bs), s>>>(p);
+    return launch_dependent(corr_pair_kernel<2>, dim3(clusters), kT, pr_smem_bytes(2, bp, bs), s, p);
   } else if (n == 32768) {
     if ((e = pair_prepare<4>()) != cudaSuccess) return e;
-    corr_pair_kernel<4><<<2 * clusters, kT, pr_smem_bytes(4, bp, bs), s>>>(p);
+    return launch_dependent(corr_pair_kernel<4>, dim3(2 * clusters), kT, pr_smem_bytes(4, bp, bs), s, p);
   } else if (n == 65536) {
     if ((e = pair_prepare<8>()) != cudaSuccess) return e;
-    corr_pair_kernel<8><<<4 * clusters, kT, pr_smem_bytes(8, bp, bs), s>>>(p);
-  } else {
-    return cudaErrorInvalidValue;
+    return launch_dependent(corr_pair_kernel<8>, dim3(4 * clusters), kT, pr_smem_bytes(8, bp, bs), s, p);
   }
-  return cudaGetLastError();
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace fxc

@@ -65,7 +65,6 @@ template <int N>
 struct SmallCta {
   Twiddles<N> tw;
   uint32_t seq;  // staging iterations so far (mbarrier slot and phase, start buffer)
-  bool ready;    // twiddles computed (by the first span, while its copies are in flight)
 };
 
 template <int N, int FPC>
@@ -77,8 +76,8 @@ __device__ __forceinline__ void small_cta_init(uint8_t* smem, SmallCta<N>& c) {
     *reinterpret_cast<int*>(smem + L::FLAG) = 0;
     fence_proxy_async();
   }
+  c.tw.init(threadIdx.x % (N / 16));
   c.seq = 0;
-  c.ready = false;
 }
 
 // Never leave a bulk copy in flight into a finished CTA's shared memory.
@@ -144,8 +143,6 @@ __device__ __forceinline__ bool small_span(const CorrParams& p, uint64_t it0, ui
     fence_proxy_async();
     for (uint64_t it = it0; it < it1 && it < it0 + kStages; ++it) issue(it);
   }
-  if (!c.ready) c.tw.init(t);
-  c.ready = true;
   build_decode_tables_at(sp, ss, preP, preS, smem, lut, tid, T);
   const bool splitP = split_2bit(sp), splitS = split_2bit(ss);
   __syncthreads();
@@ -344,7 +341,9 @@ corr_small_kernel(const __grid_constant__ CorrParams p) {
   constexpr int H = N / 2 + 1;
   extern __shared__ __align__(128) uint8_t smem[];
   SmallCta<N> c;
+  grid_dependents();
   small_cta_init<N, FPC>(smem, c);
+  grid_wait();  // the frame records
   const uint64_t iters = (p.nf + FPC - 1) / FPC;
   const uint64_t it0 = (blockIdx.x * iters) / gridDim.x;
   const uint64_t it1 = ((blockIdx.x + 1) * iters) / gridDim.x;
@@ -391,9 +390,8 @@ cudaError_t launch_one(const CorrParams& p, int grid, cudaStream_t s) {
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)SmallLayout<N, FPC>::total(2u * FPC * N));
   if (e != cudaSuccess) return e;
-  corr_small_kernel<N, FPC>
-      <<<grid, FPC * N / 16, SmallLayout<N, FPC>::total(p.stage_bytes), s>>>(p);
-  return cudaGetLastError();
+  return launch_dependent(corr_small_kernel<N, FPC>, dim3(grid), FPC * N / 16,
+                          SmallLayout<N, FPC>::total(p.stage_bytes), s, p);
 }
 
 // Variants of the batched kernels: FFT length, frames per CTA iteration and

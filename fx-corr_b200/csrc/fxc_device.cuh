@@ -601,6 +601,18 @@ __device__ __forceinline__ void preshuffle_slot(uint32_t* w1, uint32_t n1, int k
     for (uint32_t i = tid; i < n2; i += nthreads) w2[i] = shuffle_word(w2[i], kind2, lut2);
 }
 
+// Programmatic dependent launch: the kernels of a sector (frame records, FFT
+// kernel, reduction) are launched with launch_dependent (fxc_kernels.h).  A
+// kernel lets its successor's CTAs start beside it with grid_dependents(); the
+// successor sets up what does not depend on it and then waits, in grid_wait(),
+// until it has completed and its writes are visible.
+__device__ __forceinline__ void grid_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void grid_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Bounded mbarrier helpers (cp.async.bulk staging).
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   const uint32_t a = (uint32_t)__cvta_generic_to_shared(bar);

@@ -381,7 +381,9 @@ phased_kernel(const __grid_constant__ PhasedParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
   const SmemLayout L = smem_layout<N, FPC>(p.stage_bytes);
   PhasedCta<N> c;
+  grid_dependents();
   phased_cta_init<N, FPC>(smem, L, c);
+  grid_wait();  // the frame records
   const uint64_t iters = (p.nf + FPC - 1) / FPC;
   const uint64_t it0 = (blockIdx.x * iters) / gridDim.x;
   const uint64_t it1 = ((blockIdx.x + 1) * iters) / gridDim.x;
@@ -428,8 +430,7 @@ static cudaError_t launch_phased_one(const PhasedParams& p, int grid, cudaStream
       kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
       (int)(smem_layout<N, FPC>(2u * FPC * N).total + kTailBytes));
   if (e != cudaSuccess) return e;
-  kern<<<grid, FPC * N / 16, smem, stream>>>(p);
-  return cudaGetLastError();
+  return launch_dependent(kern, dim3(grid), FPC * N / 16, smem, stream, p);
 }
 
 cudaError_t launch_phased(uint32_t n, const PhasedParams& p, int grid, cudaStream_t s) {

@@ -405,7 +405,9 @@ template <bool WIDE>
 __global__ void __launch_bounds__(kT, 1) phased_pair_kernel(const __grid_constant__ PhasedParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
   PpCta c;
+  grid_dependents();
   pp_cta_init(smem, c);
+  grid_wait();  // the frame records
   const uint64_t it0 = ((uint64_t)blockIdx.x * p.nf) / gridDim.x;
   const uint64_t it1 = ((uint64_t)(blockIdx.x + 1) * p.nf) / gridDim.x;
   pp_span<WIDE>(p, it0, it1, p.partials + (size_t)blockIdx.x * kH2, smem, c);
@@ -457,8 +459,8 @@ cudaError_t launch_phased_pair(const PhasedParams& p, int grid, cudaStream_t s) 
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kPpMaxSmem);
   if (e != cudaSuccess) return e;
-  kern<<<grid, kT, wide ? kPpWideSmem : pp_smem_bytes(p.st[0].bpf, p.st[1].bpf), s>>>(p);
-  return cudaGetLastError();
+  return launch_dependent(kern, dim3(grid), kT,
+                          wide ? kPpWideSmem : pp_smem_bytes(p.st[0].bpf, p.st[1].bpf), s, p);
 }
 
 // The batch group's kernel, its shared memory sized for the narrow layout with
