@@ -23,17 +23,44 @@
 // instead of the search, and 1- and 2-bit samples quantised in the registers of
 // the last pass (votes, no exchange): FFT 1024, 50001 frame pairs 620 -> 471 us,
 // 2048 1208 -> 908, 4096 (20000) 1004 -> 745, 8192 (12503) 1348 -> 1015 us; 8-bit
-// FFT 8192 2097 -> 1322 us; the .raw bytes are the same.
+// FFT 8192 2097 -> 1322 us; the .raw bytes are the same.  Decoding from the raw words
+// as the correlation kernels do (one barrier and a rewrite of every shuffled word
+// less): 462 -> 431 us, 4096 733 -> 681, 8192 1011 -> 972, 4-bit FFT 1024 584 -> 547 us.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "decode_tables.cuh"
+#include "fold_decode.cuh"
 #include "fxc_device.cuh"
 #include "fxc_kernels.h"
 
 namespace fxc {
 
 constexpr uint32_t kQuantBytes = (kQuantFloats * 4 + 15) / 16 * 16;
-constexpr uint32_t kTailBytes = kQuantBytes + 4096;  // quantiser and encode tables
+
+// Shared memory: decode tables (levels and rotate amounts, decode_tables.cuh),
+// frame records, mbarriers, flag and ticket, byte LUTs of 4- and 8-bit generic
+// shuffles, quantiser and encode tables, the two buffers, the staging slots
+// [FPC FrameInfo][FPC frames of station 1][FPC frames of station 2].
+template <int N, int FPC>
+struct PhasedLayout {
+  static constexpr uint32_t FI = kTabPos + 256;
+  static constexpr uint32_t BAR = FI + FPC * kFiBytes;
+  static constexpr uint32_t FLAG = BAR + kStages * 8;
+  static constexpr uint32_t TICKET = FLAG + 4;
+  static constexpr uint32_t LUT = (FLAG + 8 + 15) / 16 * 16;
+  static constexpr uint32_t QL = LUT + 8192;
+  static constexpr uint32_t ENC = QL + kQuantBytes;
+  static constexpr uint32_t A = (ENC + 4096 + 127) / 128 * 128;
+  static constexpr uint32_t B = A + FPC * Geom<N>::CSTRIDE * 8;
+  static constexpr uint32_t STAGE = (B + FPC * Geom<N>::CSTRIDE * 8 + 127) / 128 * 128;
+  __host__ __device__ static constexpr uint32_t stride(uint32_t raw) {
+    return (FPC * kFiBytes + raw + 127u) & ~127u;
+  }
+  __host__ __device__ static constexpr uint32_t total(uint32_t raw) {
+    return STAGE + kStages * stride(raw);
+  }
+};
 
 // Per-CTA state that outlives one sector: the twiddle bases and the number of
 // staging iterations consumed so far (it sets the mbarrier slot and phase, so
@@ -45,27 +72,25 @@ struct PhasedCta {
 };
 
 template <int N, int FPC>
-__device__ __forceinline__ void phased_cta_init(uint8_t* smem, const SmemLayout& L,
-                                                PhasedCta<N>& c) {
-  constexpr int T1 = N / 16;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L.off_bar);
-  int* flag = reinterpret_cast<int*>(smem + L.off_flag);
+__device__ __forceinline__ void phased_cta_init(uint8_t* smem, PhasedCta<N>& c) {
+  using L = PhasedLayout<N, FPC>;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR);
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) mbar_init(&bars[s], 1);
-    *flag = 0;
+    *reinterpret_cast<int*>(smem + L::FLAG) = 0;
     fence_proxy_async();
   }
-  c.tw.init(threadIdx.x % T1);
+  c.tw.init(threadIdx.x % (N / 16));
   c.seq = 0;
 }
 
 // Never leave a bulk copy in flight into a finished CTA's shared memory.
-__device__ __forceinline__ void phased_cta_drain(uint8_t* smem, const SmemLayout& L) {
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L.off_bar);
-  const int* flag = reinterpret_cast<const int*>(smem + L.off_flag);
-  if (threadIdx.x == 0 && *flag) {
+template <int N, int FPC>
+__device__ __forceinline__ void phased_cta_drain(uint8_t* smem) {
+  using L = PhasedLayout<N, FPC>;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR);
+  if (threadIdx.x == 0 && *reinterpret_cast<const int*>(smem + L::FLAG))
     for (int s = 0; s < kStages; ++s) mbar_wait(&bars[s], 0, kWaitPolls);
-  }
 }
 
 // CTA iterations [it0, it1) (FPC frame pairs each) of the sector p: phased
@@ -78,24 +103,25 @@ __device__ __forceinline__ void phased_cta_drain(uint8_t* smem, const SmemLayout
 // moves samples that sit on a quantiser decision boundary.
 template <int N, int FPC>
 __device__ __noinline__ bool phased_span(const PhasedParams& p, uint64_t it0, uint64_t it1,
-                                            double* part, uint8_t* smem, const SmemLayout& L,
+                                            double* part, uint8_t* smem, uint32_t raw_bytes,
                                             PhasedCta<N>& c) {
+  using L = PhasedLayout<N, FPC>;
   constexpr int T1 = N / 16;
   constexpr int T = FPC * T1;
   constexpr int BPT = (N / 2) / T;
   static_assert(BPT * T == N / 2 && BPT >= 2, "bins per thread");
 
-  float2* bufA = reinterpret_cast<float2*>(smem + L.off_a);
-  float2* bufB = reinterpret_cast<float2*>(smem + L.off_b);
-  uint8_t* stage = smem + L.off_stage;
-  uint32_t* lut = reinterpret_cast<uint32_t*>(smem + L.off_lut);  // decode LUTs, then encode LUT
-  float* lv = reinterpret_cast<float*>(smem + L.off_lv);          // [0,512) decode levels
-  FrameInfo* finfo = reinterpret_cast<FrameInfo*>(smem + L.off_fi);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L.off_bar);
-  int* flag = reinterpret_cast<int*>(smem + L.off_flag);
-  // quantiser tables live in the extra tail of the layout
-  float* ql = reinterpret_cast<float*>(smem + L.total);  // levels and thresholds
-  uint32_t* elut = reinterpret_cast<uint32_t*>(smem + L.total + kQuantBytes);  // [4][256] encode LUT
+  float2* bufA = reinterpret_cast<float2*>(smem + L::A);
+  float2* bufB = reinterpret_cast<float2*>(smem + L::B);
+  uint8_t* stage = smem + L::STAGE;
+  const uint32_t stride = L::stride(raw_bytes);
+  uint32_t* lut = reinterpret_cast<uint32_t*>(smem + L::LUT);
+  const uint32_t* pos = reinterpret_cast<const uint32_t*>(smem + kTabPos);
+  FrameInfo* finfo = reinterpret_cast<FrameInfo*>(smem + L::FI);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR);
+  int* flag = reinterpret_cast<int*>(smem + L::FLAG);
+  float* ql = reinterpret_cast<float*>(smem + L::QL);  // levels and thresholds
+  uint32_t* elut = reinterpret_cast<uint32_t*>(smem + L::ENC);  // [4][256] encode LUT
 
   const int tid = threadIdx.x;
   const int g = tid / T1;
@@ -112,7 +138,7 @@ __device__ __noinline__ bool phased_span(const PhasedParams& p, uint64_t it0, ui
     const uint64_t nvalid = (p.nf - f0) < (uint64_t)FPC ? (p.nf - f0) : (uint64_t)FPC;
     const uint32_t bf = (uint32_t)(nvalid * kFiBytes);
     const uint32_t b1 = (uint32_t)(nvalid * bpf1), b2 = (uint32_t)(nvalid * bpf2);
-    uint8_t* dst = stage + slot * L.stage_stride;
+    uint8_t* dst = stage + slot * stride;
     mbar_expect_tx(&bars[slot], bf + b1 + b2);
     bulk_g2s(dst, p.finfo + f0, bf, &bars[slot]);
     bulk_g2s(dst + kRaw1, p.st[0].raw + f0 * bpf1, b1, &bars[slot]);
@@ -126,10 +152,12 @@ __device__ __noinline__ bool phased_span(const PhasedParams& p, uint64_t it0, ui
     fence_proxy_async();
     for (uint64_t it = it0; it < it1 && it < it0 + kStages; ++it) issue(it);
   }
-  for (int i = tid; i < 512; i += T) lv[i] = p.st[i >> 8].levels[i & 255] * p.st[i >> 8].scale;
-  for (int s = 0; s < 2; ++s)
-    if (p.st[s].shkind == SH_GENERIC)
-      for (int i = tid; i < 1024; i += T) lut[s * 1024 + i] = p.st[s].shlut[i];
+  // 4- and 8-bit stations with a non-identity shuffle are rewritten in place
+  // (byte LUTs); 1- and 2-bit stations are decoded from the raw words
+  const bool pre1 = p.st[0].bits > 2 && p.st[0].shkind != SH_IDENTITY;
+  const bool pre2 = p.st[1].bits > 2 && p.st[1].shkind != SH_IDENTITY;
+  build_decode_tables_at(p.st[0], p.st[1], pre1, pre2, smem, lut, tid, T);
+  const bool split1 = split_2bit(p.st[0]), split2 = split_2bit(p.st[1]);
   for (int i = tid; i < kQuantFloats; i += T) ql[i] = p.qlevels[i];
   for (int i = tid; i < 1024; i += T) elut[i] = p.enc_lut[i];
   __syncthreads();
@@ -173,34 +201,48 @@ __device__ __noinline__ bool phased_span(const PhasedParams& p, uint64_t it0, ui
       atomicOr(flag, 1);
       atomicOr(p.err, ERR_WAIT_TIMEOUT);
     }
-    uint8_t* st = stage + slot * L.stage_stride;
+    uint8_t* st = stage + slot * stride;
     uint32_t* w1 = reinterpret_cast<uint32_t*>(st + kRaw1);
     uint32_t* w2 = reinterpret_cast<uint32_t*>(st + kRaw1 + FPC * bpf1);
-    preshuffle_slot(w1, FPC * bpf1 / 4, p.st[0].shkind, lut, w2, FPC * bpf2 / 4, p.st[1].shkind,
-                    lut + 1024, tid, T);
-    if (t == 0 && valid) finfo[g] = reinterpret_cast<const FrameInfo*>(st)[g];
-    __syncthreads();
-    if (*flag) {
-      ok = false;
-      break;
+    if (pre1 || pre2) {  // CTA-uniform
+      preshuffle_slot(w1, FPC * bpf1 / 4, pre1 ? p.st[0].shkind : SH_IDENTITY, lut, w2,
+                      FPC * bpf2 / 4, pre2 ? p.st[1].shkind : SH_IDENTITY, lut + 1024, tid, T);
+      __syncthreads();
     }
-    const int s1 = valid ? finfo[g].s1 : 0;
-    const int s2 = valid ? finfo[g].s2 : 0;
-    const PackedStation pa{w1 + g * (bpf1 / 4), lv, (uint32_t)p.st[0].bits,
-                           (1u << p.st[0].bits) - 1u, p.st[0].lsb ? 1 : 0, s1};
-    const PackedStation pb{w2 + g * (bpf2 / 4), lv + 256, (uint32_t)p.st[1].bits,
-                           (1u << p.st[1].bits) - 1u, p.st[1].lsb ? 1 : 0, s2};
-
     float2* za = bufA + g * Geom<N>::CSTRIDE;
     float2* zb = bufB + g * Geom<N>::CSTRIDE;
-    first_pass_packed<N>(pa, pb, za, t);
+    if (valid) {  // warp-uniform
+      const FrameInfo* fs = reinterpret_cast<const FrameInfo*>(st) + g;
+      const int b1 = p.st[0].bits, b2 = p.st[1].bits;
+      const int s1 = fs->s1, s2 = fs->s2;
+      const int m1 = t - s1, m2 = t - s2;
+      const uint32_t tb1 = (uint32_t)((m1 & (p.st[0].lsb ? 1 : 0)) << (b1 + 2));
+      const uint32_t tb2 = 2048u + (uint32_t)((m2 & (p.st[1].lsb ? 1 : 0)) << (b2 + 2));
+      float2 v[16];
+      fold::row_station<N, false>(b1, split1, w1 + g * (bpf1 / 4), smem, s1,
+                                  pos[m1 & ((32 / b1) - 1)], tb1, v, t);
+      fold::row_station<N, true>(b2, split2, w2 + g * (bpf2 / 4), smem, s2,
+                                 pos[32 + (m2 & ((32 / b2) - 1))], tb2, v, t);
+      if (t == 0) finfo[g] = *fs;
+      dft16(v);
+      float2* dst = za + 17 * t;  // cpad(16 t + r) = 17 t + r
+#pragma unroll
+      for (int r = 0; r < 16; ++r) dst[r] = v[out_pos<16>(r)];
+    }
     float2* Z0 = fft_rest<N>(za, zb, t, tw);
-    if (tid == 0 && it + kStages < it1) {
+    // fft_rest opened with a barrier after the first pass: the staging slot is
+    // consumed, refill it.  Not after a wait gave up (flagged before it).
+    if (tid == 0 && it + kStages < it1 && !*flag) {
       fence_proxy_async();
       issue(it + kStages);
     }
     const bool fin_b = Z0 != za;
+    const bool stop = *flag != 0;  // not written between the first barrier and the next frame
     __syncthreads();
+    if (stop) {
+      ok = false;
+      break;
+    }
 
     // ---- per-bin synthesis over every valid frame of the iteration; cb goes
     // by bin to the buffer that does not hold Z
@@ -379,16 +421,15 @@ __global__ void __launch_bounds__(FPC * N / 16, (N >= 8192 ? 1 : 2))
 phased_kernel(const __grid_constant__ PhasedParams p) {
   constexpr int H = N / 2 + 1;
   extern __shared__ __align__(128) uint8_t smem[];
-  const SmemLayout L = smem_layout<N, FPC>(p.stage_bytes);
   PhasedCta<N> c;
   grid_dependents();
-  phased_cta_init<N, FPC>(smem, L, c);
+  phased_cta_init<N, FPC>(smem, c);
   grid_wait();  // the frame records
   const uint64_t iters = (p.nf + FPC - 1) / FPC;
   const uint64_t it0 = (blockIdx.x * iters) / gridDim.x;
   const uint64_t it1 = ((blockIdx.x + 1) * iters) / gridDim.x;
-  phased_span<N, FPC>(p, it0, it1, p.partials + (size_t)blockIdx.x * H, smem, L, c);
-  phased_cta_drain(smem, L);
+  phased_span<N, FPC>(p, it0, it1, p.partials + (size_t)blockIdx.x * H, smem, p.stage_bytes, c);
+  phased_cta_drain<N, FPC>(smem);
 }
 
 // Batched: a persistent grid takes the items of batch group `grp` by ticket;
@@ -400,11 +441,10 @@ template <int N, int FPC>
 __global__ void __launch_bounds__(FPC * N / 16, (N >= 8192 ? 1 : 2))
 phased_batch_kernel(const BatchArgs a, int grp) {
   extern __shared__ __align__(128) uint8_t smem[];
-  const SmemLayout L = smem_layout<N, FPC>(2u * FPC * N);
   if (blockIdx.x >= a.hdr->nitems[grp]) return;  // a graph launches the full grid
-  uint32_t* ticket = reinterpret_cast<uint32_t*>(smem + L.off_flag + 4);
+  uint32_t* ticket = reinterpret_cast<uint32_t*>(smem + PhasedLayout<N, FPC>::TICKET);
   PhasedCta<N> c;
-  phased_cta_init<N, FPC>(smem, L, c);
+  phased_cta_init<N, FPC>(smem, c);
   const uint32_t n_items = a.hdr->nitems[grp];
   const BatchItem* items = a.hdr->items + a.hdr->item0[grp];
   const BatchScan* scans = a.hdr->scans;
@@ -415,20 +455,21 @@ phased_batch_kernel(const BatchArgs a, int grp) {
     if (k >= n_items) break;
     const BatchItem w = items[k];
     const uint64_t it0 = w.f0 / FPC, it1 = (w.f1 + FPC - 1) / FPC;
-    if (!phased_span<N, FPC>(scans[w.scan].pp, it0, it1, a.partials + w.part, smem, L, c)) break;
+    if (!phased_span<N, FPC>(scans[w.scan].pp, it0, it1, a.partials + w.part, smem, 2u * FPC * N, c))
+      break;
   }
-  phased_cta_drain(smem, L);
+  phased_cta_drain<N, FPC>(smem);
 }
 
 template <int N, int FPC>
 static cudaError_t launch_phased_one(const PhasedParams& p, int grid, cudaStream_t stream) {
-  const uint32_t smem = smem_layout<N, FPC>(p.stage_bytes).total + kTailBytes;
+  const uint32_t smem = PhasedLayout<N, FPC>::total(p.stage_bytes);
   auto kern = phased_kernel<N, FPC>;
   // the limit is shared by every host thread: always the largest layout
   // (8-bit stations), never lowered under a concurrent launch
   cudaError_t e = cudaFuncSetAttribute(
       kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-      (int)(smem_layout<N, FPC>(2u * FPC * N).total + kTailBytes));
+      (int)(PhasedLayout<N, FPC>::total(2u * FPC * N)));
   if (e != cudaSuccess) return e;
   return launch_dependent(kern, dim3(grid), FPC * N / 16, smem, stream, p);
 }
@@ -446,7 +487,7 @@ cudaError_t launch_phased(uint32_t n, const PhasedParams& p, int grid, cudaStrea
 namespace {
 template <int N, int FPC>
 uint32_t phased_batch_smem() {
-  return smem_layout<N, FPC>(2u * FPC * N).total + kTailBytes;
+  return PhasedLayout<N, FPC>::total(2u * FPC * N);
 }
 }  // namespace
 
