@@ -268,6 +268,7 @@ void station_params(const fxc_scan* s, const uint8_t* r1, const uint8_t* r2, Sta
     st[k].shkind = s->shkind[k];
     st[k].scale = s->scale[k];
     std::memcpy(st[k].perm, k ? s->cfg.shuffle2 : s->cfg.shuffle1, 32);
+    st[k].whole = whole_samples(st[k].perm, st[k].bits) ? 1 : 0;
   }
 }
 

@@ -10,8 +10,8 @@
 //   2. a thread's 16 first-pass inputs of a station sit at one bit position of
 //      16 words (fold_decode.cuh): word load, rotate, masked merge into a byte
 //      offset of the level table; the LSB flip selects a negated copy.  Shuffles
-//      of 1- and 2-bit stations are part of the rotate, those of wider ones are
-//      applied in place by byte LUTs first;
+//      of 1- and 2-bit stations and of whole samples are part of the rotate, those
+//      that tear wider samples apart are applied in place by byte LUTs first;
 //   3. radix-16 Stockham passes and the trailing radix-4 or -8 pass in padded
 //      shared memory.  The three passes end in the buffer they began in, so the
 //      next iteration begins in the other one and no barrier closes an iteration:
@@ -26,9 +26,9 @@
 // FP32).  Against the general form it replaces (words rewritten by LUT for every
 // shuffle, a check and a sign per sample, grid selects and product predicates per
 // bin, five barriers), sector calls of 31250 frame pairs, 2-bit, no band shift:
-// FFT 1024 173 -> 143 us, 2048 291 -> 256, 4096 566 -> 502; 8-bit auto-spectra of FFT
-// 2048 (20011) 204 -> 182; 4-bit against 2-bit cross-spectra of FFT 4096 (12207),
-// LSB, shifted band 256 -> 237 us.
+// FFT 1024 173 -> 141 us, 2048 291 -> 256, 4096 566 -> 502; 8-bit auto-spectra of FFT
+// 2048 (20011), pairs of bits swapped, 204 -> 167; 4-bit against 2-bit cross-spectra
+// of FFT 4096 (12207), LSB, shifted band 256 -> 237 us.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -120,8 +120,8 @@ __device__ __forceinline__ bool small_span(const CorrParams& p, uint64_t it0, ui
   const bool g0 = p.grid == 0;
   const StationParams& sp = p.st[g0 ? 0 : 1];
   const StationParams& ss = p.st[g0 ? 1 : 0];
-  const bool preP = sp.bits > 2 && sp.shkind != SH_IDENTITY;
-  const bool preS = ss.bits > 2 && ss.shkind != SH_IDENTITY;
+  const bool preP = rewritten(sp);
+  const bool preS = rewritten(ss);
 
   // slot: [FPC FrameInfo][FPC primary frames][FPC secondary frames]
   auto issue = [&](uint64_t it) {
@@ -143,8 +143,8 @@ __device__ __forceinline__ bool small_span(const CorrParams& p, uint64_t it0, ui
     fence_proxy_async();
     for (uint64_t it = it0; it < it1 && it < it0 + kStages; ++it) issue(it);
   }
-  build_decode_tables_at(sp, ss, preP, preS, smem, lut, tid, T);
-  const bool splitP = split_2bit(sp), splitS = split_2bit(ss);
+  build_decode_tables_at<true>(sp, ss, preP, preS, smem, lut, tid, T);
+  const bool splitP = split_2bit<true>(sp), splitS = split_2bit<true>(ss);
   __syncthreads();
 
   // Sums of bins tid + T i (and N/2 by thread 0): primary ACF, secondary ACF at

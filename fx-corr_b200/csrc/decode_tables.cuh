@@ -22,11 +22,28 @@ namespace fxc {
 
 constexpr uint32_t kTabPos = 4096, kTabLut = 4608, kTabEnd = kTabLut + 8192;
 
+// WHOLE, here and below: the kernel decodes every shuffle of whole samples from the
+// raw words as they are.  The kernels of FFT <= 8192 that hold a frame's words in
+// registers do (WHOLE = true): for them the rewriting costs an exchange through
+// shared memory and a barrier per frame (FFT 2048 8-bit ACF with pair-swapped
+// bits: 181 us with it, 167 without; phased FFT 8192, the same stations:
+// 1257 -> 1204 us, 2-bit 974 -> 950; the test costs the identity at FFT 1024 1 us of
+// 140).  The other kernels (WHOLE = false) rewrite the words of every shuffle but
+// the identity: there the flag cost the generic shuffles 2.5 % (FFT 8192, 20,000
+// frames: 667 -> 684 us; phased FFT 16384 4-bit: 558 -> 578), more than it gave the
+// whole-sample ones.
+
+// Words rewritten in place by the station's byte LUTs before decoding: 4- and
+// 8-bit stations whose shuffle tears samples apart.
+__device__ __forceinline__ bool rewritten(const StationParams& q) { return q.bits > 2 && !q.whole; }
+
 // Builds the tables of stations a and b (needs a barrier before use).
-// preA / preB: the station's words are rewritten in place by its byte LUTs
-// before decoding (4- and 8-bit stations with a non-identity shuffle), so its
-// rotate amounts are those of the natural bit order.
+// preA / preB: the station's words are rewritten before decoding, so its rotate
+// amounts and levels are those of the natural bit order.  With WHOLE, a shuffle of
+// whole samples has the field's place in the rotate amounts and its bit order in
+// the level table.
 // `lut`: where the byte LUTs go.
+template <bool WHOLE>
 __device__ __forceinline__ void build_decode_tables_at(const StationParams& sa,
                                                        const StationParams& sb, bool preA,
                                                        bool preB, uint8_t* smem, uint32_t* lut,
@@ -38,7 +55,16 @@ __device__ __forceinline__ void build_decode_tables_at(const StationParams& sa,
     // warp's table loads fall in different banks)
     const StationParams& q = (i < 512) ? sa : sb;
     const int n = 1 << q.bits, c2 = i & 511;
-    const float x = c2 < 2 * n ? q.levels[c2 & (n - 1)] * q.scale : 0.0f;
+    float x = 0.0f;
+    if (c2 < 2 * n) {
+      uint32_t code = (uint32_t)(c2 & (n - 1));
+      if (WHOLE && q.whole && q.shkind != SH_IDENTITY && !(i < 512 ? preA : preB)) {
+        const uint32_t field = code;
+        code = 0;
+        for (int j = 0; j < q.bits; ++j) code |= ((field >> (q.perm[j] & (q.bits - 1))) & 1u) << j;
+      }
+      x = q.levels[code] * q.scale;
+    }
     lv[i] = c2 >= n ? -x : x;
   }
   for (int i = tid; i < 64; i += nthreads) {
@@ -49,7 +75,7 @@ __device__ __forceinline__ void build_decode_tables_at(const StationParams& sa,
     const bool natural = (k ? preB : preA) || q.shkind == SH_IDENTITY;
     uint32_t r = 0;
     if (cc * b < 32) {
-      const int p0 = natural ? cc * b : q.perm[cc * b];
+      const int p0 = natural ? cc * b : (WHOLE && q.whole ? q.perm[cc * b] & ~(b - 1) : q.perm[cc * b]);
       const int p1 = b >= 2 ? (natural ? cc * b + 1 : q.perm[cc * b + 1]) : 0;
       r = (uint32_t)((p0 - 2) & 31) | ((uint32_t)((p1 - 3) & 31) << 8);
     }
@@ -65,13 +91,16 @@ __device__ __forceinline__ void build_decode_tables_at(const StationParams& sa,
 __device__ __forceinline__ void build_decode_tables(const StationParams& sa, const StationParams& sb,
                                                     bool preA, bool preB, uint8_t* smem, int tid,
                                                     int nthreads) {
-  build_decode_tables_at(sa, sb, preA, preB, smem, reinterpret_cast<uint32_t*>(smem + kTabLut), tid,
-                         nthreads);
+  build_decode_tables_at<false>(sa, sb, preA, preB, smem,
+                                reinterpret_cast<uint32_t*>(smem + kTabLut), tid, nthreads);
 }
 
 // A 2-bit shuffle keeps every sample's two bits adjacent and in order, or it
-// splits them (two rotates per sample).
+// splits them (two rotates per sample).  With WHOLE, only one that tears samples
+// apart splits them.
+template <bool WHOLE = false>
 __device__ __forceinline__ bool split_2bit(const StationParams& q) {
+  if (WHOLE) return q.bits == 2 && !q.whole;
   if (q.bits != 2 || q.shkind == SH_IDENTITY) return false;
   for (int cc = 0; cc < 16; ++cc)
     if (q.perm[2 * cc + 1] != q.perm[2 * cc] + 1 || (q.perm[2 * cc] & 1)) return true;

@@ -45,7 +45,20 @@ struct StationParams {
   float scale;             // power of two equalising the two stations' RMS level
                            // inside the shared complex FFT (exact to undo)
   uint8_t perm[32];        // the 32-bit shuffle: decoder bit o is word bit perm[o]
+  int32_t whole;           // the shuffle moves whole samples (whole_samples)
 };
+
+// Whether a shuffle keeps every sample's bits together in an aligned field of the
+// word and orders them the same way in each: fields may change places, and a bit
+// order other than the natural one is a permutation of the level table.  Such
+// words need no rewriting (4- and 8-bit stations) and one rotate per sample.
+__host__ __device__ inline bool whole_samples(const uint8_t* perm, int bits) {
+  for (int o = 0; o < 32; ++o) {
+    const int j = o & (bits - 1);  // bits is 1, 2, 4 or 8
+    if (perm[o] != (perm[o - j] & ~(bits - 1)) + (perm[j] & (bits - 1))) return false;
+  }
+  return true;
+}
 
 enum { SH_IDENTITY = 0, SH_PAIRSWAP = 1, SH_GENERIC = 2 };
 

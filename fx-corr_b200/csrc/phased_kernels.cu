@@ -152,12 +152,12 @@ __device__ __noinline__ bool phased_span(const PhasedParams& p, uint64_t it0, ui
     fence_proxy_async();
     for (uint64_t it = it0; it < it1 && it < it0 + kStages; ++it) issue(it);
   }
-  // 4- and 8-bit stations with a non-identity shuffle are rewritten in place
-  // (byte LUTs); 1- and 2-bit stations are decoded from the raw words
-  const bool pre1 = p.st[0].bits > 2 && p.st[0].shkind != SH_IDENTITY;
-  const bool pre2 = p.st[1].bits > 2 && p.st[1].shkind != SH_IDENTITY;
-  build_decode_tables_at(p.st[0], p.st[1], pre1, pre2, smem, lut, tid, T);
-  const bool split1 = split_2bit(p.st[0]), split2 = split_2bit(p.st[1]);
+  // 4- and 8-bit stations whose shuffle tears samples apart are rewritten in place
+  // (byte LUTs), all others decoded from the raw words
+  const bool pre1 = rewritten(p.st[0]);
+  const bool pre2 = rewritten(p.st[1]);
+  build_decode_tables_at<true>(p.st[0], p.st[1], pre1, pre2, smem, lut, tid, T);
+  const bool split1 = split_2bit<true>(p.st[0]), split2 = split_2bit<true>(p.st[1]);
   for (int i = tid; i < kQuantFloats; i += T) ql[i] = p.qlevels[i];
   for (int i = tid; i < 1024; i += T) elut[i] = p.enc_lut[i];
   __syncthreads();
