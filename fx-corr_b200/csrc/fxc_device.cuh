@@ -727,6 +727,49 @@ __device__ __forceinline__ uint32_t quantise4(float x, const Quantiser& q, float
   return nearest_level(x, q.ql, q.n, q.monotonic);
 }
 
+// The search out of line: callers that quantise several samples keep it out of
+// their loop's code and registers.
+static __device__ __noinline__ uint32_t nearest_cold(float x, const float* ql, int n,
+                                                     int monotonic) {
+  return nearest_level(x, ql, n, monotonic);
+}
+// K samples at a time, one test of the thresholds' range for all.  STEP: tables of
+// more than four levels too (`thr` their thresholds; t = thr[1..3]).
+template <bool STEP, int K>
+__device__ __forceinline__ void quantise_many(const float (&x)[K], const Quantiser& q,
+                                              const float* thr, float3 t, uint32_t (&c)[K]) {
+  bool in = true;
+#pragma unroll
+  for (int k = 0; k < K; ++k) in = in && fabsf(x[k]) <= q.hi;
+  if (in && q.kind == QUANT_COMPARE) {
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      c[k] = (uint32_t)(x[k] >= t.x) + (uint32_t)(x[k] >= t.y) + (uint32_t)(x[k] >= t.z);
+  } else if (STEP && in && q.kind == QUANT_STEP) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      int g = __float2int_rd(fmaf(x[k], q.step, q.offset));
+      g = min(max(g, 0), q.n - 1);
+      g += (x[k] >= thr[g + 1] ? 1 : 0) - (x[k] < thr[g] ? 1 : 0);
+      c[k] = (uint32_t)g;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < K; ++k) c[k] = nearest_cold(x[k], q.ql, q.n, q.monotonic);
+  }
+}
+// A word's share of K / 4 words of four byte codes each (code k in byte k & 3 of
+// cw[k / 4], each below 2^bits), code k at bit `bits` k; 8 bits: K = 4.
+__device__ __forceinline__ uint32_t pack_codes(const uint32_t* cw, uint32_t words, uint32_t bits) {
+  const uint32_t m2 = ((1u << (2 * bits)) - 1u) * 0x10001u;
+  uint32_t word = 0;
+  for (uint32_t i = 0; i < words; ++i) {
+    const uint32_t y = (cw[i] | cw[i] >> (8 - bits)) & m2;
+    word |= ((y & 0xFFFFu) | (y >> 16) << (2 * bits)) << (4 * bits * i);
+  }
+  return word;
+}
+
 // ------------------------------------------------------ staging layout
 
 constexpr int kStages = 2;

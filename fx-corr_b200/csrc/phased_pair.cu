@@ -8,8 +8,8 @@
 //      y_q[m] = W_N^(m q) (z[m] + (-1)^q z[m + M]), z = x1 + i x2, is decoded
 //      straight from the staged words by the FFT-16384 fold kernel's decode
 //      (fold_decode.cuh) into its first radix-16 pass; the row FFTs run in
-//      shared memory, the trailing radix-2 pass in place, so bin 2 j + q of
-//      the frame is Z_q[j];
+//      shared memory, the trailing radix-2 pass left to their readers; bin
+//      2 j + q of the frame is Z_q[j];
 //   2. per bin: both stations' spectra from the shared FFT (two-for-one),
 //      each rotated by its fractional delay with the Nyquist imaginary part
 //      zeroed and multiplied by its fringe phasor, band-aligned onto the
@@ -21,7 +21,8 @@
 //      (src/utils.rs:60-66) through the same two-row decomposition (x[m] and
 //      x[m + M] gathered from cb), odd samples negated when both inputs are
 //      LSB, nearest-level re-quantisation with ant1's levels and packing with
-//      ant1's shuffle (src/utils.rs:378-410) of whole words from both rows.
+//      ant1's shuffle (src/utils.rs:378-410) of whole words from both rows'
+//      codes.
 // Three padded row buffers.  With 1- and 2-bit stations a staging slot of its
 // own follows them and the next frame's words are copied while the frame is
 // computed; 4- and 8-bit stations (twice or four times the words) stage into
@@ -69,9 +70,10 @@ __host__ __device__ constexpr uint32_t pp_smem_bytes(uint32_t bpf1, uint32_t bpf
 }
 static_assert(pp_smem_bytes(kN2 / 4, kN2 / 4) <= kPpMaxSmem, "2-bit stations fit");
 constexpr uint32_t kPpWideEnc = kPpStage, kPpWideQl = kPpStage + 4096;
+constexpr uint32_t kPpCodes = 128 + 2 * kN2;  // WIDE: codes behind the staged words
 constexpr uint32_t kPpWideSmem = kPpWideQl + kQuantFloats * 4;
 static_assert(kPpWideSmem <= pp_smem_bytes(kN2 / 4, kN2 / 4), "one batch layout serves both");
-static_assert(128u + 2u * kN2 <= kPpBuf, "8-bit stations' words fit a row buffer");
+static_assert(kPpCodes + kN2 <= kPpBuf, "8-bit stations' words and the codes fit a row buffer");
 
 // Narrow stations take the separate staging slot (and the encode LUT and
 // output levels at their narrow places); any wider station or output selects
@@ -82,7 +84,6 @@ __host__ __device__ inline bool pp_wide(uint32_t bits1, uint32_t bits2, uint32_t
 
 using rows::first_pass_regs;
 using rows::row1_twiddle;
-using rows::row_radix2;
 using rows::fold_lower;
 using rows::fold_mirror;
 using rows::fold_twiddles;
@@ -343,47 +344,71 @@ __device__ __forceinline__ bool pp_span(const PhasedParams& p, uint64_t it0, uin
         if (q == 1) row1_twiddle(v, dtw0, dtw1);
         if (q == 0) {
           first_pass_regs(v, Q, tid);
-          fft_rest<kM, true>(Q, S, tid, tw);  // X[2 k] (pre radix-2) in Q
-          __syncthreads();
-          row_radix2(Q, tid, tw);
+          fft_rest<kM, true>(Q, S, tid, tw);  // X[2 k] (before the radix-2 pass) in Q
         } else if (!WIDE) {
+          __syncthreads();  // row 0's last pass has read S
           first_pass_regs(v, S, tid);
           fft_rest<kM, true>(S, P, tid, tw);  // X[2 k + 1] in S (cb consumed)
-          __syncthreads();
-          row_radix2(S, tid, tw);
         } else {
           __syncthreads();  // every thread has read its cb values
           first_pass_regs(v, P, tid);
           fft_rest<kM, true>(P, S, tid, tw);  // X[2 k + 1] in P
-          __syncthreads();
-          // S is free until the next frame's decode: its words go there
-          if (tid == 0 && it + 1 < it1) {
-            fence_proxy_async();
-            issue(it + 1, stage);
-          }
-          row_radix2(P, tid, tw);
         }
       }
       __syncthreads();
-      // ---- re-quantise and pack: sample n is row n & 1, index n >> 1.  Each
-      // lane starts its word at a different sample so that a warp's loads
-      // spread over the banks.  Thresholds instead of a search of the levels:
-      // 3001 frame pairs of 4-bit stations 690 -> 566 us, of 2-bit ones 556 ->
-      // 516 us.
-      uint8_t* out = p.raw_out + it * p.bpf_out;
-      const uint32_t lane = (uint32_t)tid & 31u;
-      const uint32_t rot = spw >= 16 ? lane : lane / (16u / spw);
+      // S is free until the next frame's decode: its words go there
+      if (WIDE && tid == 0 && it + 1 < it1) {
+        fence_proxy_async();
+        issue(it + 1, stage);
+      }
+      // ---- the rows' trailing radix-2 pass (real parts only) and the
+      // re-quantiser: samples n = 2 j + q and n + M, j = t + T i, of both rows,
+      // their codes by sample into a free buffer (WIDE: behind the staged words),
+      // packed into words after a barrier.  Against the pass in place and a
+      // quantiser that gathered every word's samples from both rows (shared memory
+      // written and read once more, an address and an inlined search per sample):
+      // 3001 frame pairs of 4-bit stations 558 -> 475 us, of 8-bit ones 641 -> 553,
+      // of 2-bit ones 507 -> 442.  The loop is not unrolled further (8 times: 534,
+      // the code no longer fits the instruction cache); the twiddles are formed
+      // before it.
+      uint8_t* codes = WIDE ? stage + kPpCodes : reinterpret_cast<uint8_t*>(P);
       const float3 thr = make_float3(ql[kLv + 1], ql[kLv + 2], ql[kLv + 3]);
-      for (uint32_t wdx = (uint32_t)tid; wdx < wpf; wdx += kT) {
-        uint32_t word = 0;
-        for (uint32_t i = 0; i < spw; ++i) {
-          const uint32_t ii = (i + rot) & (spw - 1u);
-          const uint32_t n = wdx * spw + ii;
-          float x = ((n & 1u) ? (WIDE ? P : S) : Q)[n >> 1].x * inv_n;
-          if (p.out_lsb && (n & 1u)) x = -x;
-          const uint32_t code = WIDE ? quantise(x, quant, ql + kLv) : quantise4(x, quant, thr);
-          word |= (code & qmask) << (ii * p.bits_out);
+      const float inv_odd = p.out_lsb ? -inv_n : inv_n;
+      float2 wq[kJ];
+#pragma unroll
+      for (int i = 0; i < kJ; ++i) {
+        float2 unused;
+        fold_twiddles(tw, wb1, i, wq[i], unused);
+      }
+#pragma unroll 2
+      for (int i = 0; i < kJ; ++i) {
+        const int j = tid + kT * i;
+        float2 wj = wq[0];
+#pragma unroll
+        for (int k = 1; k < kJ; ++k)
+          if (i == k) wj = wq[k];
+        float x[4];  // samples 2 j, 2 j + 1, 2 j + M, 2 j + 1 + M
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const float2* Y = q == 0 ? Q : (WIDE ? P : S);
+          const float a = Y[j].x, wb = cmul(wj, Y[j + kM / 2]).x;
+          const float in = q == 0 ? inv_n : inv_odd;
+          x[q] = (a + wb) * in;
+          x[2 + q] = (a - wb) * in;
         }
+        uint32_t c[4];
+        quantise_many<WIDE>(x, quant, ql + kLv, thr, c);
+        const uint32_t lo = (c[0] & qmask) | (c[1] & qmask) << 8;
+        const uint32_t hi = (c[2] & qmask) | (c[3] & qmask) << 8;
+        reinterpret_cast<uint16_t*>(codes)[j] = (uint16_t)lo;
+        reinterpret_cast<uint16_t*>(codes)[j + kM / 2] = (uint16_t)hi;
+      }
+      __syncthreads();
+      // ---- pack
+      uint8_t* out = p.raw_out + it * p.bpf_out;
+      for (uint32_t wdx = (uint32_t)tid; wdx < wpf; wdx += kT) {
+        const uint32_t word = pack_codes(reinterpret_cast<const uint32_t*>(codes + wdx * spw),
+                                         spw / 4, p.bits_out);
         reinterpret_cast<uint32_t*>(out)[wdx] =
             elut[word & 255u] | elut[256 + ((word >> 8) & 255u)] |
             elut[512 + ((word >> 16) & 255u)] | elut[768 + (word >> 24)];
