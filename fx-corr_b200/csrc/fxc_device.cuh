@@ -469,6 +469,10 @@ __device__ __forceinline__ float2* fft_rest(float2* a, float2* b, int t, const T
 // is Z[t + N/16 wi + r N/R], R = fft_last_radix<N>, at v[wi R + out_pos<R>(r)].
 template <int N>
 constexpr int fft_last_radix = Geom<N>::RL > 1 ? Geom<N>::RL : 16;
+// With an even number of passes after the first, the last of them reads b, otherwise
+// a; the other buffer is free from that pass's barrier on.
+template <int N>
+constexpr bool fft_last_reads_b = ((Geom<N>::P16 - 1 + (Geom<N>::RL > 1 ? 1 : 0)) % 2) == 0;
 template <int N>
 __device__ __forceinline__ void fft_rest_values(float2* a, float2* b, int t, const Twiddles<N>& tw,
                                                 float2 (&v)[16]) {
@@ -733,15 +737,16 @@ static __device__ __noinline__ uint32_t nearest_cold(float x, const float* ql, i
                                                      int monotonic) {
   return nearest_level(x, ql, n, monotonic);
 }
-// K samples at a time, one test of the thresholds' range for all.  STEP: tables of
-// more than four levels too (`thr` their thresholds; t = thr[1..3]).
-template <bool STEP, int K>
+// K samples at a time, one test of the thresholds' range for all.  COMPARE, STEP: the
+// kinds of table that the caller can meet, any other takes the search (`thr`: the
+// thresholds; t = thr[1..3]).
+template <bool COMPARE, bool STEP, int K>
 __device__ __forceinline__ void quantise_many(const float (&x)[K], const Quantiser& q,
                                               const float* thr, float3 t, uint32_t (&c)[K]) {
   bool in = true;
 #pragma unroll
   for (int k = 0; k < K; ++k) in = in && fabsf(x[k]) <= q.hi;
-  if (in && q.kind == QUANT_COMPARE) {
+  if (COMPARE && in && q.kind == QUANT_COMPARE) {
 #pragma unroll
     for (int k = 0; k < K; ++k)
       c[k] = (uint32_t)(x[k] >= t.x) + (uint32_t)(x[k] >= t.y) + (uint32_t)(x[k] >= t.z);

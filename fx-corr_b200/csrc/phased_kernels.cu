@@ -321,14 +321,14 @@ __device__ __noinline__ bool phased_span(const PhasedParams& p, uint64_t it0, ui
         return elut[word & 255u] | elut[256 + ((word >> 8) & 255u)] |
                elut[512 + ((word >> 16) & 255u)] | elut[768 + (word >> 24)];
       };
+      constexpr int R = fft_last_radix<N>;
+      fft_rest_values<N>(qa, qb, t, tw, v);
       if (p.bits_out <= 2 && p.qkind == QUANT_COMPARE) {
         // 1- and 2-bit output: a warp holds 32 consecutive samples in each of
         // its 16 output registers; the comparisons with the thresholds are
         // collected by votes, 32 codes at a time, and lane q of each half
         // keeps row q.  No exchange of samples through shared memory, and the
         // last pass has no imaginary parts to form.
-        constexpr int R = fft_last_radix<N>;
-        fft_rest_values<N>(qa, qb, t, tw, v);
         if (valid) {
           const uint32_t lane = (uint32_t)t & 31u;
           const uint32_t flip = p.out_lsb ? lane << 31 : 0u;  // odd samples negated
@@ -386,24 +386,31 @@ __device__ __noinline__ bool phased_span(const PhasedParams& p, uint64_t it0, ui
           }
         }
       } else {
-        float2* Y = fft_rest<N>(qa, qb, t, tw);
+        // wider output (or a table without thresholds): the codes of the last
+        // pass's samples, one byte each, go into the buffer that pass does not read
+        // and are packed after a barrier.  Against samples written there and
+        // gathered by word, an inlined search each: 4-bit stations at FFT 8192
+        // (12503 frame pairs) 1222 -> 1048 us, at FFT 1024 (50001) 546 -> 481 us.
+        uint8_t* codes = reinterpret_cast<uint8_t*>(fft_last_reads_b<N> ? qa : qb);
+        const float3 thr = make_float3(ql[257], ql[258], ql[259]);
+        const float in = p.out_lsb && (t & 1) ? -inv_n : inv_n;  // odd samples negated
+#pragma unroll
+        for (int q0 = 0; q0 < 16; q0 += 4) {
+          float x[4];
+          uint32_t c[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            x[k] = v[(q0 + k) / R * R + out_pos<R>((q0 + k) % R)].x * in;
+          quantise_many<false, true>(x, quant, ql + 256, thr, c);
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            codes[t + T1 * ((q0 + k) / R) + (N / R) * ((q0 + k) % R)] = (uint8_t)(c[k] & qmask);
+        }
         __syncthreads();
         if (valid) {
-          // Consecutive lanes pack consecutive words, spw samples apart: each
-          // lane starts its word at a different sample (rot) so that the 16
-          // lanes of a half-warp read 16 different bank pairs of Y at every
-          // step instead of one.
-          const uint32_t lane = (uint32_t)t & 31u;
-          const uint32_t rot = spw >= 16 ? lane : lane / (16u / spw);
           for (uint32_t w = (uint32_t)t; w < wpf; w += T1) {
-            uint32_t word = 0;
-            for (uint32_t i = 0; i < spw; ++i) {
-              const uint32_t ii = (i + rot) & (spw - 1u);
-              const uint32_t n = w * spw + ii;
-              float x = Y[n].x * inv_n;
-              if (p.out_lsb && (n & 1u)) x = -x;
-              word |= (quantise(x, quant, ql + 256) & qmask) << (ii * p.bits_out);
-            }
+            const uint32_t word = pack_codes(reinterpret_cast<const uint32_t*>(codes + w * spw),
+                                             spw / 4, p.bits_out);
             out[w] = encode(word);
           }
         }

@@ -397,7 +397,7 @@ __device__ __forceinline__ bool pp_span(const PhasedParams& p, uint64_t it0, uin
           x[2 + q] = (a - wb) * in;
         }
         uint32_t c[4];
-        quantise_many<WIDE>(x, quant, ql + kLv, thr, c);
+        quantise_many<true, WIDE>(x, quant, ql + kLv, thr, c);
         const uint32_t lo = (c[0] & qmask) | (c[1] & qmask) << 8;
         const uint32_t hi = (c[2] & qmask) | (c[3] & qmask) << 8;
         reinterpret_cast<uint16_t*>(codes)[j] = (uint16_t)lo;
