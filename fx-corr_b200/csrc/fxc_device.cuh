@@ -724,13 +724,6 @@ __device__ __forceinline__ uint32_t quantise(float x, const Quantiser& q, const 
   }
   return nearest_level(x, q.ql, q.n, q.monotonic);
 }
-// At most four levels, the thresholds in registers (t = thr[1..3]).
-__device__ __forceinline__ uint32_t quantise4(float x, const Quantiser& q, float3 t) {
-  if (q.kind == QUANT_COMPARE && fabsf(x) <= q.hi)
-    return (uint32_t)(x >= t.x) + (uint32_t)(x >= t.y) + (uint32_t)(x >= t.z);
-  return nearest_level(x, q.ql, q.n, q.monotonic);
-}
-
 // The search out of line: callers that quantise several samples keep it out of
 // their loop's code and registers.
 static __device__ __noinline__ uint32_t nearest_cold(float x, const float* ql, int n,

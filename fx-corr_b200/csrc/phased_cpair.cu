@@ -20,9 +20,10 @@
 //      row m mod C and of its mirror, i.e. of this CTA when m mod C is one of
 //      its rows, so each CTA forms the radix-C step of those columns from its
 //      own spectra and stores each output row into the row's owner; two
-//      inverse row FFTs per CTA give the samples n = C k + q of its rows, each
-//      re-quantised with ant1's levels (odd samples negated when both inputs
-//      are LSB) into its bits of the packed output words, which the CTAs of
+//      inverse row FFTs per CTA give the samples n = C k + q of its rows,
+//      re-quantised in the trailing radix-2 pass with ant1's levels (odd samples
+//      negated when both inputs are LSB), their codes going into the CTA's bits of
+//      the packed output words, which the CTAs of
 //      the cluster OR together in global memory (zeroed first) after ant1's
 //      output shuffle, a bit permutation (src/utils.rs:378-410).
 // Four cluster barriers per frame: after the forward rows are stored (B1),
@@ -407,8 +408,7 @@ __global__ void __cluster_dims__(C / 2, 1, 1) __launch_bounds__(kT, 1)
         first_pass_regs(v, Y, tid);
       }
       fft_rest<kM, true>(Y, XA, tid, tw);
-      __syncthreads();
-      row_radix2(Y, tid, tw);
+      __syncthreads();  // XA is read
       {
         float2 v[16];
 #pragma unroll
@@ -417,26 +417,51 @@ __global__ void __cluster_dims__(C / 2, 1, 1) __launch_bounds__(kT, 1)
       }
       fft_rest<kM, true>(XA, XB, tid, tw);
       __syncthreads();
-      row_radix2(XA, tid, tw);
+      // the rows' trailing radix-2 pass (real parts only) and the re-quantiser:
+      // indices j and j + M/2 of both rows, their codes by index and row into XB.
+      // Against the pass in place and a gather of every word's samples: FFT 32768
+      // (1500 frame pairs, 2-bit) 745 -> 713 us, 1-bit 735 -> 688, 65536 (750)
+      // 987 -> 941 us.
+      uint8_t* codes = reinterpret_cast<uint8_t*>(XB);
+      const float3 thr = make_float3(ql[5], ql[6], ql[7]);
+      const float inA = p.out_lsb && (rowA & 1) ? -inv_n : inv_n;  // odd samples negated
+      const float inB = p.out_lsb && (rowB & 1) ? -inv_n : inv_n;
+      float2 wq[kJ];
+#pragma unroll
+      for (int i = 0; i < kJ; ++i) wq[i] = rows::radix2_twiddle(tw, i);
+#pragma unroll 2
+      for (int i = 0; i < kJ; ++i) {
+        const int j = tid + kT * i;
+        float2 wj = wq[0];
+#pragma unroll
+        for (int k = 1; k < kJ; ++k)
+          if (i == k) wj = wq[k];
+        float x[4];
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          const float2* R = b ? XA : Y;
+          const float a = R[j].x, wb = cmul(wj, R[j + kM / 2]).x;
+          x[b] = (a + wb) * (b ? inB : inA);
+          x[2 + b] = (a - wb) * (b ? inB : inA);
+        }
+        uint32_t c[4];
+        quantise_many<true, false>(x, quant, nullptr, thr, c);
+        uint16_t* cj = reinterpret_cast<uint16_t*>(codes) + j;
+        cj[0] = (uint16_t)((c[0] & qmask) | (c[1] & qmask) << 8);
+        cj[kM / 2] = (uint16_t)((c[2] & qmask) | (c[3] & qmask) << 8);
+      }
       __syncthreads();
-      // re-quantise this CTA's samples into their bits of each output word;
-      // the cluster's CTAs OR their bits together (the words start at zero)
+      // pack this CTA's bits of each output word; the cluster's CTAs OR their bits
+      // together (the words start at zero)
       uint32_t* out = reinterpret_cast<uint32_t*>(p.raw_out + it * p.bpf_out);
       const uint32_t per = spw / (uint32_t)C;  // samples of one row in a word
-      const float3 thr = make_float3(ql[5], ql[6], ql[7]);
+      const uint32_t bA = (uint32_t)rowA * p.bits_out, bB = (uint32_t)rowB * p.bits_out;
       for (uint32_t wdx = (uint32_t)tid; wdx < wpf; wdx += kT) {
+        const uint16_t* cw = reinterpret_cast<const uint16_t*>(codes) + wdx * per;
         uint32_t word = 0;
         for (uint32_t i = 0; i < per; ++i) {
-          const uint32_t k = wdx * per + i;  // index in the rows
-#pragma unroll
-          for (int b = 0; b < 2; ++b) {
-            const uint32_t row = (uint32_t)(b ? rowB : rowA);
-            const uint32_t n = (uint32_t)C * k + row;
-            float x = (b ? XA : Y)[k].x * inv_n;
-            if (p.out_lsb && (n & 1u)) x = -x;
-            word |= (quantise4(x, quant, thr) & qmask)
-                    << ((n - wdx * spw) * p.bits_out);
-          }
+          const uint32_t y = cw[i], at = (uint32_t)C * i * p.bits_out;
+          word |= (y & 255u) << (at + bA) | (y >> 8) << (at + bB);
         }
         const uint32_t sw = elut[word & 255u] | elut[256 + ((word >> 8) & 255u)] |
                             elut[512 + ((word >> 16) & 255u)] | elut[768 + (word >> 24)];

@@ -13,23 +13,26 @@ constexpr int kM = 8192;       // row length
 constexpr int kT = kM / 16;    // threads per CTA
 constexpr int kJ = kM / 2 / kT;  // radix-2 butterflies per thread
 
+// W_M^j = W_M^t W_16^i, j = t + T i (i a constant once unrolled).
+__device__ __forceinline__ float2 radix2_twiddle(const Twiddles<kM>& tw, int i) {
+  switch (i) {
+    case 0: return tw.w[Geom<kM>::P16];
+    case 1: return mul_w16<1>(tw.w[Geom<kM>::P16]);
+    case 2: return mul_w16<2>(tw.w[Geom<kM>::P16]);
+    case 3: return mul_w16<3>(tw.w[Geom<kM>::P16]);
+    case 4: return mul_w16<4>(tw.w[Geom<kM>::P16]);
+    case 5: return mul_w16<5>(tw.w[Geom<kM>::P16]);
+    case 6: return mul_w16<6>(tw.w[Geom<kM>::P16]);
+    default: return mul_w16<7>(tw.w[Geom<kM>::P16]);
+  }
+}
 // The trailing radix-2 pass of a row in place: Z[j], Z[j + M/2] from the last
 // radix-16 pass's output, j = t + T i.
 __device__ __forceinline__ void row_radix2(float2* Z, int tid, const Twiddles<kM>& tw) {
 #pragma unroll
   for (int i = 0; i < kJ; ++i) {
     const int j = tid + kT * i;
-    float2 wj;  // W_M^j = W_M^t W_16^i
-    switch (i) {  // compile-time after unrolling
-      case 0: wj = tw.w[Geom<kM>::P16]; break;
-      case 1: wj = mul_w16<1>(tw.w[Geom<kM>::P16]); break;
-      case 2: wj = mul_w16<2>(tw.w[Geom<kM>::P16]); break;
-      case 3: wj = mul_w16<3>(tw.w[Geom<kM>::P16]); break;
-      case 4: wj = mul_w16<4>(tw.w[Geom<kM>::P16]); break;
-      case 5: wj = mul_w16<5>(tw.w[Geom<kM>::P16]); break;
-      case 6: wj = mul_w16<6>(tw.w[Geom<kM>::P16]); break;
-      default: wj = mul_w16<7>(tw.w[Geom<kM>::P16]); break;
-    }
+    const float2 wj = radix2_twiddle(tw, i);
     const float2 a = Z[j], wb = cmul(wj, Z[j + kM / 2]);
     Z[j] = cadd(a, wb);
     Z[j + kM / 2] = csub(a, wb);

@@ -1,10 +1,10 @@
 """The re-quantiser takes the samples in the inverse transform's last pass, keeps their
-codes by sample and packs them (FFT 16384, and 4- and 8-bit output or tables without
-thresholds up to FFT 8192): every output width, both staging layouts, odd samples
-negated or not, several frames per CTA, a last iteration with frames to spare, against
-the FP64 oracle.
-A code may differ only where the sample lies within f32 rounding of a decision point
-(1e-4 of the series' RMS, the bound of the phased parity tests)."""
+codes by sample and packs them (FFT 16384; 4- and 8-bit output or tables without
+thresholds up to FFT 8192; FFT 32768 and 65536 in a cluster): every output width, both
+staging layouts, odd samples negated or not, several frames per CTA, a last iteration
+with frames to spare, against the FP64 oracle.  A code may differ only where the sample
+lies within f32 rounding of a decision point (1e-4 of the series' RMS, the bound of the
+phased parity tests)."""
 import numpy as np
 import pytest
 
@@ -50,3 +50,13 @@ def test_codes_of_one_row(engine, fft, nf, bits, down):
                      band=(8, 0, fft // 2 - 8, 8), delay=DELAY,
                      products=oracle.PROD_PHASED | oracle.PROD_RAW)
     check(engine, scan, nf, seed=fft + bits)
+
+
+@pytest.mark.parametrize("fft,nf", [(32768, 1), (32768, 81), (65536, 43)])
+@pytest.mark.parametrize("bits1,bits2", [(1, 2), (2, 2)])
+@pytest.mark.parametrize("grid", [0, 1])
+def test_codes_of_a_clusters_rows(engine, fft, nf, bits1, bits2, grid):
+    scan = make_scan(fft=fft, fs=512e6, bits1=bits1, bits2=bits2, lsb1=nf > 1, lsb2=nf > 1,
+                     grid=grid, shuffle="generic", band=(-64, 64, fft // 2, 0), delay=DELAY,
+                     products=oracle.PROD_PHASED | oracle.PROD_RAW)
+    check(engine, scan, nf, seed=fft + bits1 + grid)
