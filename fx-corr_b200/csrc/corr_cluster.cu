@@ -197,7 +197,6 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kT, 1)
   const bool want_acf = (p.products & 1u) != 0;
   const bool want_xcf = (p.products & 2u) != 0;
   const bool ov_only = (p.products & 16u) != 0;
-  const float xconj = g0 ? 1.0f : -1.0f;  // XCF = S1 conj(S2): conj(P conj(S)) for grid 1
   const int lsbP = sp.lsb ? 1 : 0, lsbS = ss.lsb ? 1 : 0;
   const int colP = g0 ? 0 : 1, colS = g0 ? 1 : 0;  // output columns of the two ACFs
   const bool half = q == 0 && tid == 0;            // bin N/2
@@ -213,16 +212,25 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kT, 1)
 #pragma unroll
     for (int v = 0; v < 4; ++v) acc[i][v] = 0.f;
 
+  // Every sum runs for every bin: out of the overlap the secondary spectrum is
+  // zero, and the products that were not asked for are left out here.  (Predicates
+  // per bin and product and the odd frames' sign on every secondary value: FFT 65536,
+  // 3001 frame pairs, 4-bit 2181 -> 2140 us; 32768 829 -> 809; 16384 with an odd band
+  // shift, 8001 frame pairs, 966 -> 951 us.)
   auto flush = [&]() {
 #pragma unroll
     for (int i = 0; i <= kJ; ++i) {
       if (i == kJ && !half) continue;
       const int bin = i == kJ ? N / 2 : C * (tid + kT * i) + q;
+      const bool in = (unsigned)(bin - ovs) < (unsigned)ov;
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
         const int col = v == 0 ? colP : (v == 1 ? colS : v);
         double* d = part + (size_t)col * H + bin;
-        *d = (first_flush ? 0.0 : *d) + (double)acc[i][v];
+        float x = acc[i][v];
+        if (v == 0 ? !(want_acf && (!ov_only || in)) : (v == 1 ? !want_acf : !want_xcf)) x = 0.f;
+        if (v == 3 && !g0) x = -x;  // grid 1: the conjugate was summed
+        *d = (first_flush ? 0.0 : *d) + (double)x;
         acc[i][v] = 0.f;
       }
     }
@@ -268,7 +276,7 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kT, 1)
       const bool inP = aP >= 0 && aP + kM / C <= kM, inS = aS >= 0 && aS + kM / C <= kM;
       const int cP = mP & ((32 / bitsP) - 1), cS = mS & ((32 / bitsS) - 1);
       const uint32_t tbP = (uint32_t)((mP & lsbP) << (bitsP + 2));
-      // the secondary station enters odd frames negated (undone by sgn below)
+      // the secondary station enters odd frames negated (undone in the ramp)
       const uint32_t tbS = 2048u + (uint32_t)((((uint32_t)mS & (uint32_t)lsbS) ^ (uint32_t)(it & 1u))
                                               << (bitsS + 2));
       cl_station<C, kM / C, 0, U, 8, false>(bitsP, splitP, wP, smem, mP, lwP, pos[cP], tbP, inP, v);
@@ -342,22 +350,26 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kT, 1)
     // fringe x ramp rotation of the thread's bins (while the barrier completes)
     const FrameInfo& F = finfo[fb];
     float sn, cs;
-    __sincosf(fmaf((float)(C * tid + q - ovs), F.dphi, F.phi0), &sn, &cs);
-    float2 rot = cmul(F.fr_mix, make_float2(cs, sn));
-    __sincosf((float)(C * kT) * F.dphi, &sn, &cs);
+    // XCF = S1 conj(S2): P conj(S) times the ramp for grid 0; for grid 1 its
+    // conjugate is summed, P conj(S) times the ramp's conjugate.
+    const float sgn = (it & 1u) ? -1.0f : 1.0f, cj = g0 ? 1.0f : -1.0f;
+    const float dphi = cj * F.dphi, phi0 = cj * F.phi0;
+    const float2 mix = make_float2(sgn * F.fr_mix.x, sgn * cj * F.fr_mix.y);
+    __sincosf(fmaf((float)(C * tid + q - ovs), dphi, phi0), &sn, &cs);
+    float2 rot = cmul(mix, make_float2(cs, sn));
+    __sincosf((float)(C * kT) * dphi, &sn, &cs);
     const float2 rstep = make_float2(cs, sn);
     float2 rhalf = make_float2(0.f, 0.f);
     if (half) {
-      __sincosf(fmaf((float)(N / 2 - ovs), F.dphi, F.phi0), &sn, &cs);
-      rhalf = cmul(F.fr_mix, make_float2(cs, sn));
+      __sincosf(fmaf((float)(N / 2 - ovs), dphi, phi0), &sn, &cs);
+      rhalf = cmul(mix, make_float2(cs, sn));
     }
-    const float sgn = (it & 1u) ? -1.0f : 1.0f;
     cl_wait();
 
     // ---- 4. two-for-one split; secondary spectra to the primary bins' CTA
     // Rounding in the shared complex FFT leaks a fixed fraction (~1e-6) of
     // each station's spectrum into the other's; the secondary's odd-frame
-    // negation (undone by sgn) makes that leak alternate in sign and cancel.
+    // negation (undone in the ramp) makes that leak alternate in sign and cancel.
     float2 prim[kJ];
     float2 prim_h = make_float2(0.f, 0.f);
     {
@@ -373,7 +385,7 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kT, 1)
         prim[i] = make_float2(u.x + w.x, u.y - w.y);
         const int kp = C * j + q - qoff;
         if ((unsigned)(kp - ovs) < (unsigned)ov) {
-          const float2 sv = make_float2(sgn * (u.y + w.y), sgn * (w.x - u.x));
+          const float2 sv = make_float2(u.y + w.y, w.x - u.x);
           if (qlocal) Yb[j + dq] = sv;
           else cl_st(qaddr + (uint32_t)(j + dq) * (uint32_t)sizeof(float2), sv);
         }
@@ -382,7 +394,7 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kT, 1)
         prim_h = make_float2(2.f * zhalf.x, 0.f);
         const int kp = N / 2 - qoff;
         if ((unsigned)(kp - ovs) < (unsigned)ov) {
-          const float2 sv = make_float2(sgn * 2.f * zhalf.y, 0.f);
+          const float2 sv = make_float2(2.f * zhalf.y, 0.f);
           if (qlocal) Yb[kM / 2 + dq] = sv;
           else cl_st(qaddr + (uint32_t)(kM / 2 + dq) * (uint32_t)sizeof(float2), sv);
         }
@@ -393,17 +405,14 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kT, 1)
 
     // ---- 5. accumulation (constant indices into acc[][])
     auto bin_acc = [&](int bin, int j, float2 pv, float2 r, float* a) {
-      const bool inov = (unsigned)(bin - ovs) < (unsigned)ov;
-      if (want_acf && (!ov_only || inov)) a[0] = fmaf(pv.x, pv.x, fmaf(pv.y, pv.y, a[0]));
-      if (inov) {
-        const float2 qv = Yb[j];
-        if (want_acf) a[1] = fmaf(qv.x, qv.x, fmaf(qv.y, qv.y, a[1]));
-        if (want_xcf) {
-          float2 x = cmulc(pv, qv);
-          x.y *= xconj;
-          a[2] = fmaf(x.x, r.x, fmaf(-x.y, r.y, a[2]));
-          a[3] = fmaf(x.x, r.y, fmaf(x.y, r.x, a[3]));
-        }
+      float2 qv = make_float2(0.f, 0.f);
+      if ((unsigned)(bin - ovs) < (unsigned)ov) qv = Yb[j];
+      a[0] = fmaf(pv.x, pv.x, fmaf(pv.y, pv.y, a[0]));
+      a[1] = fmaf(qv.x, qv.x, fmaf(qv.y, qv.y, a[1]));
+      if (want_xcf) {
+        const float2 x = cmulc(pv, qv);
+        a[2] = fmaf(x.x, r.x, fmaf(-x.y, r.y, a[2]));
+        a[3] = fmaf(x.x, r.y, fmaf(x.y, r.x, a[3]));
       }
     };
 #pragma unroll
