@@ -282,8 +282,9 @@ FXC_API fxc_status fxc_server_destroy(fxc_server* sv);
  * No reference counterpart (the reference runs one scan per process).  A
  * batch runs one sector of each of many distinct scans in a few launches:
  * the frame records of every sector in one launch, every sector of one FFT
- * length in one persistent kernel (1-8 bit stations mixed; work items of a
- * few hundred frames handed out to the CTAs by an atomic ticket), and one
+ * length in one persistent kernel (1-8 bit stations mixed; work items of up to
+ * a few hundred frames, at least two dozen of a long sector, handed out to the
+ * CTAs by an atomic ticket; the lengths' kernels side by side), and one
  * fixed-order reduction for all.  With use_graphs the launches of each set of
  * FFT lengths are captured once in a CUDA graph and replayed.  The frames per
  * CTA iteration and frames per work item of each FFT length come from an
