@@ -327,8 +327,8 @@ __device__ __noinline__ bool phased_span(const PhasedParams& p, uint64_t it0, ui
         // 1- and 2-bit output: a warp holds 32 consecutive samples in each of
         // its 16 output registers; the comparisons with the thresholds are
         // collected by votes, 32 codes at a time, and lane q of each half
-        // keeps row q.  No exchange of samples through shared memory, and the
-        // last pass has no imaginary parts to form.
+        // keeps row q.  (Codes by way of shared memory, as below: 2-bit FFT 8192
+        // 972 us against 959, FFT 1024 444 against 433, 1-bit 432 against 413.)
         if (valid) {
           const uint32_t lane = (uint32_t)t & 31u;
           const uint32_t flip = p.out_lsb ? lane << 31 : 0u;  // odd samples negated
