@@ -713,17 +713,6 @@ struct Quantiser {
   float hi, step, offset;  // QUANT_STEP: level index ~ floor(x step + offset)
 };
 constexpr int kQuantFloats = 256 + 257;
-__device__ __forceinline__ uint32_t quantise(float x, const Quantiser& q, const float* thr) {
-  if (q.kind != QUANT_SEARCH && fabsf(x) <= q.hi) {
-    if (q.kind == QUANT_COMPARE)
-      return (uint32_t)(x >= thr[1]) + (uint32_t)(x >= thr[2]) + (uint32_t)(x >= thr[3]);
-    int g = __float2int_rd(fmaf(x, q.step, q.offset));
-    g = min(max(g, 0), q.n - 1);
-    g += (x >= thr[g + 1] ? 1 : 0) - (x < thr[g] ? 1 : 0);
-    return (uint32_t)g;
-  }
-  return nearest_level(x, q.ql, q.n, q.monotonic);
-}
 // The search out of line: callers that quantise several samples keep it out of
 // their loop's code and registers.
 static __device__ __noinline__ uint32_t nearest_cold(float x, const float* ql, int n,

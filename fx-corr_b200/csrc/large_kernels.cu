@@ -764,34 +764,55 @@ __global__ void phased_global_kernel(const LargeParams p, const PhasedParams pp,
 // src/utils.rs:378-410): x[n] = Re(X[n]) / N in the row layout of the
 // FFT output, odd samples negated when both inputs are LSB, nearest of
 // ant1's levels, codes LSB-first, ant1's shuffle applied per word.
-__global__ void quant_global_kernel(const LargeParams p, const PhasedParams pp,
-                                    const float2* __restrict__ X, uint64_t f0, uint64_t nb) {
+// A thread takes one index k of all C rows, the samples C k .. C k + C - 1, so that
+// a warp reads whole lines of each row; the lanes of a word OR their bits.  Bound by
+// reading the complex rows (67 MB a batch).  Against a thread per word that gathers
+// its samples one by one (33 us a batch): 4-bit stations of FFT 32768, 1500 frame
+// pairs, 1368 -> 1304 us in all, 65536 (750) 1441 -> 1338, 8-bit 1515 -> 1389.
+template <int C>
+__global__ void quant_global_kernel(const PhasedParams pp, const float2* __restrict__ X, uint64_t f0,
+                                    uint64_t nb) {
   __shared__ float ql[kQuantFloats];
   __shared__ uint32_t elut[1024];
   for (int i = threadIdx.x; i < kQuantFloats; i += blockDim.x) ql[i] = pp.qlevels[i];
   const Quantiser quant{ql, (int)pp.nqlevels, pp.qmonotonic, pp.qkind, pp.qhi, pp.qstep, pp.qoffset};
   for (int i = threadIdx.x; i < 1024; i += blockDim.x) elut[i] = pp.enc_lut[i];
   __syncthreads();
-  const int C = p.c, M = kLargeM, N = p.n;
-  const uint32_t spw = 32u / pp.bits_out, wpf = (uint32_t)N / spw;
-  const uint32_t qmask = (1u << pp.bits_out) - 1u;
-  const float inv_n = 1.0f / (float)N;
-  const uint64_t total = nb * (uint64_t)wpf;
-  for (uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
+  constexpr int M = kLargeM;
+  const float3 thr = make_float3(ql[257], ql[258], ql[259]);
+  const uint32_t bits = pp.bits_out, qmask = (1u << bits) - 1u;
+  const float inv_n = 1.0f / (float)(C * M);
+  const float inv_odd = pp.out_lsb ? -inv_n : inv_n;  // odd samples: odd rows
+  const uint32_t per = C * bits;                       // a thread's bits
+  const uint32_t lanes = per < 32u ? 32u / per : 1u;   // threads of a word
+  const uint32_t at = (threadIdx.x & (lanes - 1u)) * per;
+  auto encode = [&](uint32_t word) -> uint32_t {
+    return elut[word & 255u] | elut[256 + ((word >> 8) & 255u)] | elut[512 + ((word >> 16) & 255u)] |
+           elut[768 + (word >> 24)];
+  };
+  // nb M and the grid's stride are multiples of 32: whole warps iterate
+  for (uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < nb * (uint64_t)M;
        idx += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t fl = idx / wpf;
-    const uint32_t w = (uint32_t)(idx - fl * wpf);
-    const float2* Xf = X + fl * (uint64_t)N;
-    uint32_t word = 0;
-    for (uint32_t i = 0; i < spw; ++i) {
-      const int n = (int)(w * spw + i);
-      float x = Xf[(n % C) * M + n / C].x * inv_n;
-      if (pp.out_lsb && (n & 1)) x = -x;
-      word |= (quantise(x, quant, ql + 256) & qmask) << (i * pp.bits_out);
+    const uint64_t fl = idx / M;
+    const uint32_t k = (uint32_t)(idx % M);
+    const float2* Xf = X + fl * (uint64_t)(C * M) + k;
+    float x[C];
+    uint32_t c[C];
+#pragma unroll
+    for (int r = 0; r < C; ++r) x[r] = Xf[r * M].x * ((r & 1) ? inv_odd : inv_n);
+    quantise_many<true, true>(x, quant, ql + 256, thr, c);
+    uint64_t v = 0;
+#pragma unroll
+    for (int r = 0; r < C; ++r) v |= (uint64_t)(c[r] & qmask) << (r * bits);
+    uint32_t* out = reinterpret_cast<uint32_t*>(pp.raw_out + (f0 + fl) * pp.bpf_out);
+    if (per <= 32u) {
+      uint32_t word = (uint32_t)v << at;
+      for (uint32_t o = 1; o < lanes; o <<= 1) word |= __shfl_xor_sync(0xFFFFFFFFu, word, (int)o);
+      if (at == 0) out[k / lanes] = encode(word);
+    } else {  // C = 8, 8 bits
+      out[2 * k] = encode((uint32_t)v);
+      out[2 * k + 1] = encode((uint32_t)(v >> 32));
     }
-    const uint32_t sw = elut[word & 255u] | elut[256 + ((word >> 8) & 255u)] |
-                        elut[512 + ((word >> 16) & 255u)] | elut[768 + (word >> 24)];
-    reinterpret_cast<uint32_t*>(pp.raw_out + (f0 + fl) * pp.bpf_out)[w] = sw;
   }
 }
 
@@ -958,8 +979,13 @@ cudaError_t launch_large_phased(const LargeParams& p, const PhasedParams& pp, fl
   e = p.c <= 4 ? launch_rows_fft_complex(p, nb, buf0, buf1, sms, s)
                : large_fft_core(p, nb, buf0, buf1, sms, s);
   if (e != cudaSuccess) return e;
-  const uint64_t words = nb * (uint64_t)(p.n / (32 / pp.bits_out));
-  quant_global_kernel<<<grid_for(words, 256, sms), 256, 0, s>>>(p, pp, buf1, f0, nb);
+  const int ctas = grid_for(nb * (uint64_t)kLargeM, 256, sms);
+  switch (p.c) {
+    case 2: quant_global_kernel<2><<<ctas, 256, 0, s>>>(pp, buf1, f0, nb); break;
+    case 4: quant_global_kernel<4><<<ctas, 256, 0, s>>>(pp, buf1, f0, nb); break;
+    case 8: quant_global_kernel<8><<<ctas, 256, 0, s>>>(pp, buf1, f0, nb); break;
+    default: return cudaErrorInvalidValue;
+  }
   return cudaGetLastError();
 }
 

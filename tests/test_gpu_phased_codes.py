@@ -1,10 +1,10 @@
 """The re-quantiser takes the samples in the inverse transform's last pass, keeps their
 codes by sample and packs them (FFT 16384; 4- and 8-bit output or tables without
-thresholds up to FFT 8192; FFT 32768 and 65536 in a cluster): every output width, both
-staging layouts, odd samples negated or not, several frames per CTA, a last iteration
-with frames to spare, against the FP64 oracle.  A code may differ only where the sample
-lies within f32 rounding of a decision point (1e-4 of the series' RMS, the bound of the
-phased parity tests)."""
+thresholds up to FFT 8192; FFT 32768 and 65536 in a cluster), or a thread takes one index
+of all rows (the four-step path): every output width, both staging layouts, odd samples
+negated or not, several frames per CTA, a last iteration with frames to spare, against
+the FP64 oracle.  A code may differ only where the sample lies within f32 rounding of a
+decision point (1e-4 of the series' RMS, the bound of the phased parity tests)."""
 import numpy as np
 import pytest
 
@@ -60,3 +60,13 @@ def test_codes_of_a_clusters_rows(engine, fft, nf, bits1, bits2, grid):
                      grid=grid, shuffle="generic", band=(-64, 64, fft // 2, 0), delay=DELAY,
                      products=oracle.PROD_PHASED | oracle.PROD_RAW)
     check(engine, scan, nf, seed=fft + bits1 + grid)
+
+
+@pytest.mark.parametrize("fft,shift", [(32768, 3), (65536, 16)])
+@pytest.mark.parametrize("bits1,bits2", [(1, 4), (2, 4), (4, 4), (8, 1)])
+@pytest.mark.parametrize("nf", [1, 67])
+def test_codes_of_all_rows(engine, fft, shift, bits1, bits2, nf):
+    scan = make_scan(fft=fft, fs=512e6, bits1=bits1, bits2=bits2, lsb1=nf > 1, lsb2=nf > 1,
+                     shuffle="generic", band=(shift, 0, fft // 2 - shift, shift), delay=DELAY,
+                     products=oracle.PROD_PHASED | oracle.PROD_RAW)
+    check(engine, scan, nf, seed=fft + bits1)
