@@ -23,10 +23,10 @@ namespace fxc {
 constexpr uint32_t kTabPos = 4096, kTabLut = 4608, kTabEnd = kTabLut + 8192;
 
 // WHOLE, here and below: the kernel decodes every shuffle of whole samples from the
-// raw words as they are.  The kernels of FFT <= 8192 that hold a frame's words in
-// registers do (WHOLE = true): for them the rewriting costs an exchange through
-// shared memory and a barrier per frame (FFT 2048 8-bit ACF with pair-swapped
-// bits: 181 us with it, 167 without; phased FFT 8192, the same stations:
+// raw words as they are.  The correlation kernels of FFT <= 4096 and the phased kernels
+// of FFT <= 8192 do (WHOLE = true): the rewriting costs them an exchange through
+// shared memory and a barrier per frame (FFT 2048 8-bit ACF with pair-swapped bits:
+// 181 us with it, 167 without; phased FFT 8192, the same stations:
 // 1257 -> 1204 us, 2-bit 974 -> 950; the test costs the identity at FFT 1024 1 us of
 // 140).  The other kernels (WHOLE = false) rewrite the words of every shuffle but
 // the identity: there the flag cost the generic shuffles 2.5 % (FFT 8192, 20,000
