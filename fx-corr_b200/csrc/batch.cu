@@ -208,6 +208,7 @@ fxc_status grow(fxc_batch* b, fxc_batch::Arena& A, uint64_t arena_bytes, uint64_
 struct Entry {
   uint32_t idx;  // position in the caller's arrays
   int group;
+  uint64_t per;  // frames per item
   BatchScan bs;
 };
 
@@ -419,9 +420,16 @@ fxc_status run_batch(fxc_batch* b, fxc_scan* const* scans, const uint8_t* const*
       BCK(cudaEventCreateWithFlags(&b->ev_join[g], cudaEventDisableTiming));
     }
   }
-  // table order: by group, then call order; items follow the same order
-  std::stable_sort(ents.begin(), ents.end(),
-                   [](const Entry& a, const Entry& c) { return a.group < c.group; });
+  // Table order: by group, then the longest items first, then call order; items
+  // follow the same order, so that a call does not end with long items that were
+  // taken last (FFT 4096, 16 sectors of 250-4000 frames: 850 us in call order, 645).
+  for (Entry& e : ents) {
+    const Shape& sh = b->shape[e.group];
+    e.per = item_len(sh, e.group, b->sms, e.bs.p.nf, sh.pinned || b->tuning[e.group]);
+  }
+  std::stable_sort(ents.begin(), ents.end(), [](const Entry& a, const Entry& c) {
+    return a.group != c.group ? a.group < c.group : a.per > c.per;
+  });
   BatchHeader hdr{};
   hdr.nscans = (uint32_t)ents.size();
   std::vector<BatchItem> items;
@@ -430,9 +438,7 @@ fxc_status run_batch(fxc_batch* b, fxc_scan* const* scans, const uint8_t* const*
     hdr.item0[g] = (uint32_t)items.size();
     for (Entry& e : ents) {
       if (e.group != g) continue;
-      const Shape& sh = b->shape[g];
-      const uint64_t n = e.bs.p.nf;
-      const uint64_t per = item_len(sh, g, b->sms, n, sh.pinned || b->tuning[g]);
+      const uint64_t n = e.bs.p.nf, per = e.per;
       const uint32_t nparts = (uint32_t)((n + per - 1) / per);
       const uint64_t h = e.bs.h;
       const uint64_t slot = phased_group(g) ? h : 4 * h;  // partial doubles per item

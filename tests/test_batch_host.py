@@ -1,0 +1,70 @@
+"""The host side of the batched sectors (batch.cu) on the CPU: the file is linked
+with a fake of the CUDA runtime (fake_cudart.cpp) and driven by
+batch_host_check.cu, which logs every launch with the launches before it and the
+work items of its group."""
+import shutil
+import subprocess
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parents[1]
+OK, EBUSY = 0, -6
+
+
+@pytest.fixture(scope="module")
+def batch(tmp_path_factory):
+    """batch(command, *sectors, budget, fail_at) -> parsed output of the driver."""
+    from fxc import build
+
+    tmp = tmp_path_factory.mktemp("batch_host")
+    inc = ["-I", str(ROOT / "include"), "-I", str(ROOT / "fx-corr_b200" / "csrc"),
+           "-I", str(ROOT / "tests")]
+    cxx = shutil.which("g++") or "g++"
+    subprocess.run([cxx, "-std=c++17", "-O1", "-I", str(Path(build.nvcc()).parents[1] / "include"),
+                    "-c", str(ROOT / "tests" / "fake_cudart.cpp"), "-o", str(tmp / "fake.o")],
+                   check=True)
+    subprocess.run([build.nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O1",
+                    "-cudart", "none", "--diag-suppress", "128", *inc,
+                    str(ROOT / "fx-corr_b200" / "csrc" / "batch.cu"),
+                    str(ROOT / "tests" / "batch_host_check.cu"), str(tmp / "fake.o"),
+                    "-o", str(tmp / "check")], check=True)
+
+    def call(command, *sectors, budget=0, fail_at=-1):
+        r = subprocess.run([str(tmp / "check"), command, str(budget), str(fail_at),
+                            *[":".join(map(str, s)) for s in sectors]],
+                           capture_output=True, text=True, check=True)
+        out = dict(launches=[])
+        for line in r.stdout.splitlines():
+            w = line.split()
+            if w[0] == "item":
+                out["launches"][-1]["items"].append(tuple(map(int, w[1:])))
+            elif w[0].isdigit():
+                out["launches"].append(dict(name=w[1], group=int(w[2]),
+                                            before=set(map(int, w[4:])), items=[]))
+            elif w[0] == "stream":
+                out["stream"] = set(map(int, w[1:]))
+            else:
+                out[w[0]] = int(w[1])
+        assert out["left"] == 0  # every reserved byte was given back
+        return out
+
+    return call
+
+
+def groups(out):
+    return {ln["group"]: ln["items"] for ln in out["launches"] if ln["group"] >= 0}
+
+
+def test_longest_items_first(batch):
+    """A group's items are taken in order: a call whose long sectors come last must
+    not end with their items."""
+    out = batch("items", (4096, 0, 100, 2), (4096, 0, 3000, 3), (4096, 0, 900, 4),
+                (16384, 1, 40, 3), (16384, 1, 500, 2))
+    assert out["status"] == OK
+    for items in groups(out).values():
+        lengths = {}
+        for scan, row, f0, f1, part, flush in items:
+            lengths.setdefault(scan, []).append(f1 - f0)
+        longest = [max(v) for v in lengths.values()]  # in ticket order
+        assert len(set(longest)) > 1 and longest == sorted(longest, reverse=True)
