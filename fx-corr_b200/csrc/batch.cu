@@ -3,8 +3,9 @@
 // A call describes each scan's sector (BatchScan: the scan's tables, frame
 // record buffer, raw words and output; correlation or phased products),
 // splits every sector into work items
-// of `item_frames` frames (at most one per persistent CTA), uploads the
-// tables in one copy and runs
+// of `item_frames` frames or a part of a short sector (item_len; whole short
+// sectors where the call has many, whole_sectors), uploads the tables in one copy
+// and runs
 //   batch_frame_info_kernel  the FP64 delay records of every frame,
 //   one persistent kernel per FFT length present (tickets over its items), side
 //   by side,
@@ -17,9 +18,12 @@
 
 #include <algorithm>
 #include <chrono>
+#include <cmath>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <mutex>
+#include <queue>
 #include <random>
 #include <string>
 #include <vector>
@@ -214,25 +218,69 @@ struct Entry {
 
 // Frames per item of a sector: the group's item size, enlarged so that a
 // sector has at most one item per resident CTA and, unless the caller set it,
-// reduced to a part of a short sector (but at least 2^15 samples per station),
-// rounded to whole CTA iterations.  A call takes at least as long as its
-// longest item: 128 frames of FFT 4096 phased are 1.8 ms on one CTA while the
-// rest of the GPU has run out of items.  An item costs 2-4 us beyond its frames
-// (tables, first copy) and writes 16 N bytes of partials, which the reduction
-// reads.  24 sectors of 2^21 samples, FFT 1024 / 4096 / 16384, correlation and
-// phased: 4820 us a call with 128-frame items one group after another, 736 us
-// with 16 items a sector and the groups side by side, 583 with 24, 519 with 32;
-// 64 sectors of FFT 8192, 125-2000 frames: 2766 us with 64-frame items, 2776
-// with 16, 2753 with 24, 2792 with 32 (the partials).  So 24 for correlation
-// and, four times smaller partials, 32 for phased sectors.  Only the sector's
-// own length counts, so that its sums do not depend on what else is in the call.
+// reduced to a part of a short sector, rounded to whole CTA iterations.  A call
+// takes at least as long as its longest item: 128 frames of FFT 4096 phased are
+// 1.8 ms on one CTA while the rest of the GPU has run out of items.  24 sectors of
+// 2^21 samples, FFT 1024 / 4096 / 16384, correlation and phased: 4820 us a call
+// with 128-frame items one group after another, 736 us with 16 items a sector and
+// the groups side by side, 583 with 24, 519 with 32; 64 sectors of FFT 8192,
+// 125-2000 frames: 2766 us with 64-frame items, 2776 with 16, 2753 with 24, 2792
+// with 32 (the partials).  So 24 for correlation and, four times smaller partials,
+// 32 for phased sectors, of at least 2^15 samples per station: 24 sectors of
+// 2^17 samples 130 us a call, 220 with at least 2^16, 367 with 2^17.  The two-row
+// kernel has two items, one a row, and takes 2^16: 64 sectors of 16-62 frames 486 us
+// with 2^15, 405 with 2^16.  Only the sector's own length counts, so that its sums do
+// not depend on what else is in the call.
 uint64_t item_len(const Shape& sh, int g, int sms, uint64_t nf, bool exact) {
   const uint64_t maxn = (uint64_t)std::max(1, sms * sh.ctas);
   uint64_t per = sh.item_frames;
   const uint64_t parts = phased_group(g) ? 32 : 24;
-  if (!exact) per = std::min(per, std::max<uint64_t>((nf + parts - 1) / parts, 32768 / kGroupN[g]));
+  const uint64_t least = (g == BG_16384 ? 65536 : 32768) / kGroupN[g];
+  if (!exact) per = std::min(per, std::max<uint64_t>((nf + parts - 1) / parts, least));
   if ((nf + per - 1) / per > maxn) per = (nf + maxn - 1) / maxn;
   return align_up(per, (uint64_t)sh.fpc);
+}
+
+// Whether a correlation group's short sectors run whole, one item each.  Such a
+// sector's items have one f32 run each (at most 32 frames, kRun).  As one item it
+// keeps the runs, flushed to f64 at the same frames and so added in the same order:
+// the sums are the same bit for bit, and what else is in the call may decide.  An
+// item costs about 1.5 frames beyond its own (ticket, tables, first copies, and
+// its partials, which the reduction reads again), a flush within an item 0.1; whole
+// sectors fill the CTAs less evenly, so they are dealt out here, the longest first,
+// as the tickets will.  1024 sectors of FFT 8192, 32-125 frames: 4600 us a call in
+// parts, 3590 whole, and a fifth of the partials; 256 of FFT 16384, 16-62 frames:
+// 1720 and 1190 us; 64 of them 400 and 480.  What stays in parts among many others
+// pays the items' cost: 1000 sectors of FFT 1024, 628 frames, 3430 us against 3290
+// with 128-frame items.  (Phased groups, with a quarter of the partials a frame,
+// stay in parts.)
+constexpr uint64_t kRun = 32;
+bool whole_sectors(const std::vector<Entry>& ents, int g, int ctas) {
+  double split = 0.0, shared = 0.0, longest = 0.0, sum = 0.0;  // frames
+  std::vector<double> whole;
+  for (const Entry& e : ents) {
+    if (e.group != g) continue;
+    const double n = (double)e.bs.p.nf, items = std::ceil(n / (double)e.per);
+    split += n + 1.5 * items;
+    longest = std::max(longest, (double)e.per);
+    if (e.per <= kRun) whole.push_back(n + 1.5 + 0.1 * items);
+    else shared += n + 1.5 * items;
+  }
+  for (double x : whole) sum += x;
+  split = std::max(longest, split / ctas + 0.25 * longest);
+  if (whole.empty() || (shared + sum) / ctas >= split) return false;
+  std::sort(whole.begin(), whole.end(), std::greater<double>());
+  std::priority_queue<double, std::vector<double>, std::greater<double>> load(
+      std::greater<double>(), std::vector<double>(ctas, shared / ctas));
+  double end = 0.0;
+  for (double x : whole) {
+    const double t = load.top() + x;
+    if (t >= split) return false;
+    load.pop();
+    load.push(t);
+    end = std::max(end, t);
+  }
+  return end < split;
 }
 
 fxc_status run_batch(fxc_batch* b, fxc_scan* const* scans, const uint8_t* const* r1,
@@ -426,6 +474,16 @@ fxc_status run_batch(fxc_batch* b, fxc_scan* const* scans, const uint8_t* const*
   for (Entry& e : ents) {
     const Shape& sh = b->shape[e.group];
     e.per = item_len(sh, e.group, b->sms, e.bs.p.nf, sh.pinned || b->tuning[e.group]);
+  }
+  for (int g = 0; g < kCorrGroups; ++g) {
+    const Shape& sh = b->shape[g];
+    if (!(mask & (1u << g)) || sh.pinned || b->tuning[g]) continue;
+    const bool whole = whole_sectors(ents, g, b->sms * sh.ctas / (g == BG_16384 ? 2 : 1));
+    for (Entry& e : ents) {
+      if (e.group != g) continue;
+      e.bs.p.flush_every = (uint32_t)(std::min(e.per, kRun) / sh.fpc);  // iterations
+      if (whole && e.per <= kRun) e.per = std::max(e.per, align_up(e.bs.p.nf, (uint64_t)sh.fpc));
+    }
   }
   std::stable_sort(ents.begin(), ents.end(), [](const Entry& a, const Entry& c) {
     return a.group != c.group ? a.group < c.group : a.per > c.per;

@@ -101,7 +101,6 @@ __device__ __forceinline__ bool small_span(const CorrParams& p, uint64_t it0, ui
   constexpr int T = FPC * T1;
   constexpr int H = N / 2 + 1;
   constexpr int BPT = (N / 2) / T;
-  constexpr int kFlush = 32 / FPC;  // 32 frames
   static_assert(BPT * T == N / 2 && BPT >= 2, "bins per thread");
   static_assert(Geom<N>::NPASS == 3, "the transform ends in the buffer it began in");
   FrameInfo* finfo = reinterpret_cast<FrameInfo*>(smem + L::FI);
@@ -164,9 +163,12 @@ __device__ __forceinline__ bool small_span(const CorrParams& p, uint64_t it0, ui
   // every bin of the warp in the overlap (bin N/2 apart)
   const bool whole = __all_sync(0xFFFFFFFFu, (inov & ((1u << BPT) - 1u)) == (1u << BPT) - 1u);
   const bool want_xcf = (p.products & 2u) != 0;
+  const uint32_t flush_every = p.flush_every;
   bool first_flush = true;
   uint32_t since_flush = 0;
 
+  // Each address is this thread's alone: the atomics are additions that nothing
+  // waits for, in order (corr_fold.cu).
   auto flush = [&]() {
     const bool want_acf = (p.products & 1u) != 0, ov_only = (p.products & 16u) != 0;
     const int colP = g0 ? 0 : 1, colS = g0 ? 1 : 0;  // output columns of the two ACFs
@@ -181,7 +183,8 @@ __device__ __forceinline__ bool small_span(const CorrParams& p, uint64_t it0, ui
         if (v == 0 ? !(want_acf && (!ov_only || in)) : (v == 1 ? !want_acf : !want_xcf)) x = 0.f;
         if (v == 3 && !g0) x = -x;  // grid 1: the conjugate was summed
         double* q = part + (size_t)(v == 0 ? colP : (v == 1 ? colS : v)) * H + bin;
-        *q = (first_flush ? 0.0 : *q) + (double)x;
+        if (first_flush) *q = 0.0 + (double)x;
+        else atomicAdd(q, (double)x);
         acc[i][v] = 0.f;
       }
     }
@@ -326,7 +329,7 @@ __device__ __forceinline__ bool small_span(const CorrParams& p, uint64_t it0, ui
         bin_acc(Z[N / 2], Z[N / 2], s, ramp(N / 2), acc[BPT]);
       }
     }
-    if (++since_flush >= kFlush) flush();
+    if (++since_flush >= flush_every) flush();
   }
   if (ok && (since_flush > 0 || first_flush)) flush();
   c.seq = seq0 + (uint32_t)(it1 - it0);

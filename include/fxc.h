@@ -283,8 +283,9 @@ FXC_API fxc_status fxc_server_destroy(fxc_server* sv);
  * batch runs one sector of each of many distinct scans in a few launches:
  * the frame records of every sector in one launch, every sector of one FFT
  * length in one persistent kernel (1-8 bit stations mixed; work items of up to
- * a few hundred frames, at least two dozen of a long sector, handed out to the
- * CTAs by an atomic ticket; the lengths' kernels side by side), and one
+ * a few hundred frames, at least two dozen of a long sector, whole sectors where
+ * there are many short ones, handed out to the CTAs by an atomic ticket; the
+ * lengths' kernels side by side), and one
  * fixed-order reduction for all.  With use_graphs the launches of each set of
  * FFT lengths are captured once in a CUDA graph and replayed.  The frames per
  * CTA iteration and frames per work item of each FFT length come from an
@@ -297,7 +298,7 @@ FXC_API fxc_status fxc_server_destroy(fxc_server* sv);
  * correlation and phased products, empty sectors) run through the per-scan
  * path on the same stream.  A sector's products equal fxc_sector_run_device's within the
  * library's FP32 tolerance (phased .raw frames byte for byte), and are
- * identical bit for bit whatever else shares the batch (the item split
+ * identical bit for bit whatever else shares the batch (the order of its sums
  * depends only on the sector's frame count and the batch's tuning). */
 typedef struct fxc_batch fxc_batch;
 

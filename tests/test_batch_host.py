@@ -68,3 +68,25 @@ def test_longest_items_first(batch):
             lengths.setdefault(scan, []).append(f1 - f0)
         longest = [max(v) for v in lengths.values()]  # in ticket order
         assert len(set(longest)) > 1 and longest == sorted(longest, reverse=True)
+
+
+def test_many_short_sectors_run_whole(batch):
+    """Where the sectors alone fill the GPU, a short one is one item with one partial
+    slot; its f32 runs end at the same frames as its items do where it is split."""
+    for fft, nf, few, many in ((1024, 400, 8, 2000), (4096, 150, 8, 1024), (8192, 75, 16, 512),
+                               (16384, 40, 8, 256)):
+        rows = 2 if fft == 16384 else 1
+        split = batch("items", (fft, 0, nf, few))
+        whole = batch("items", (fft, 0, nf, many))
+        assert split["status"] == whole["status"] == OK
+        (s_items,), (w_items,) = groups(split).values(), groups(whole).values()
+        assert len(w_items) == many * rows and len(s_items) > 2 * few * rows
+        assert all(f0 == 0 and f1 == nf for _, _, f0, f1, _, _ in w_items)
+        assert len({part for *_, part, _ in w_items}) == many  # rows share a slot
+        fpc = {1024: 4}.get(fft, 1)
+        lengths = {f1 - f0 for _, _, f0, f1, _, _ in s_items if f1 < nf}
+        assert lengths == {flush * fpc for *_, flush in w_items} and max(lengths) <= 32
+        assert whole["in_use"] < 0.6 * many / few * split["in_use"]
+    # sectors whose items have several runs stay split
+    (items,) = groups(batch("items", (8192, 0, 2000, 512))).values()
+    assert len(items) == 512 * 24

@@ -61,3 +61,46 @@ def test_short_sector_items(engine, fxc_lib, scale):
             got = dict(acf11=a[:h], acf22=a[h:2 * h], xcf=a[2 * h:4 * h].view(np.complex128))
             assert_sector_close(got, one, sc, f"fft {sc.fft} nf {nf}", nf=nf)
         s.close()
+
+
+@pytest.mark.parametrize("fft,nf,many", [(1024, 70, 2070), (2048, 100, 1182), (4096, 75, 591),
+                                         (8192, 33, 294), (8192, 101, 294), (16384, 21, 147)])
+def test_short_sector_alone_and_among_many(engine, fxc_lib, fft, nf, many):
+    """A short sector runs in parts where it is alone and whole among many (so many that
+    they fill the CTAs of 148 SMs evenly): the same sums bit for bit, ragged last run
+    included."""
+    import torch
+
+    scans = []
+    for k, (grid, shuffle, bits) in enumerate([(0, "generic", 2), (1, "identity", 2),
+                                               (0, "generic", 4)]):
+        sc = make_scan(fft=fft, fs=512e6, bits1=bits, bits2=2, grid=grid, shuffle=shuffle,
+                       band=(-8, 40, fft // 2, 32), delay=DELAY, seed=k)
+        r1, r2 = signal_raw(sc, nf, seed=fft + k, rho=0.3, delay_samples=2.6)
+        scans.append((sc, *(torch.from_numpy(np.ascontiguousarray(r)).cuda() for r in (r1, r2))))
+    opened = [[engine.open_scan(to_fxc(sc)) for sc, *_ in scans]
+              for _ in range(-(-many // len(scans)))]
+
+    def run(copies):
+        acc = [[torch.zeros(5 * (fft // 2 + 1), dtype=torch.float64, device="cuda")
+                for _ in scans] for _ in copies]
+        n = len(copies) * len(scans)
+        batch = fxc_lib.Batch(engine)
+        batch.run_device([s for c in copies for s in c], [d1 for _ in copies for _, d1, _ in scans],
+                         [d2 for _ in copies for _, _, d2 in scans], [nf] * n, [3] * n,
+                         [a for c in acc for a in c])
+        torch.cuda.synchronize()
+        batch.close()
+        return acc
+
+    alone, among = run(opened[:1])[0], run(opened)
+    for k, (sc, d1, d2) in enumerate(scans):
+        for c in among:
+            assert torch.equal(c[k], alone[k])
+        one = opened[0][k].sector_device(d1, d2, nf, first_frame=3)
+        a, h = alone[k].cpu().numpy(), fft // 2 + 1
+        got = dict(acf11=a[:h], acf22=a[h:2 * h], xcf=a[2 * h:4 * h].view(np.complex128))
+        assert_sector_close(got, one, sc, f"fft {fft} nf {nf}", nf=nf)
+    for c in opened:
+        for s in c:
+            s.close()
