@@ -213,10 +213,10 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kT, 1)
     for (int v = 0; v < 4; ++v) acc[i][v] = 0.f;
 
   // Every sum runs for every bin: out of the overlap the secondary spectrum is
-  // zero, and the products that were not asked for are left out here.  (Predicates
-  // per bin and product and the odd frames' sign on every secondary value: FFT 65536,
-  // 3001 frame pairs, 4-bit 2181 -> 2140 us; 32768 829 -> 809; 16384 with an odd band
-  // shift, 8001 frame pairs, 966 -> 951 us.)
+  // zero; those bins and the products that were not asked for are left out here.
+  // (Predicates per bin and product and the odd frames' sign on every secondary
+  // value: FFT 65536, 3001 frame pairs, 4-bit 2181 -> 2140 us; 32768 829 -> 809; 16384
+  // with an odd band shift, 8001 frame pairs, 966 -> 951 us.)
   auto flush = [&]() {
 #pragma unroll
     for (int i = 0; i <= kJ; ++i) {
@@ -228,7 +228,8 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kT, 1)
         const int col = v == 0 ? colP : (v == 1 ? colS : v);
         double* d = part + (size_t)col * H + bin;
         float x = acc[i][v];
-        if (v == 0 ? !(want_acf && (!ov_only || in)) : (v == 1 ? !want_acf : !want_xcf)) x = 0.f;
+        // (a zero secondary spectrum times an infinite or NaN primary bin is NaN)
+        if (v == 0 ? !(want_acf && (!ov_only || in)) : !(in && (v == 1 ? want_acf : want_xcf))) x = 0.f;
         if (v == 3 && !g0) x = -x;  // grid 1: the conjugate was summed
         *d = (first_flush ? 0.0 : *d) + (double)x;
         acc[i][v] = 0.f;

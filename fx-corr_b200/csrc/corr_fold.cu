@@ -21,11 +21,11 @@
 //     at the bin pair (j, N/2 - j); the secondary spectrum goes through the
 //     free ping-pong buffer to the thread that owns the band-shifted bin;
 //   * every sum runs for every bin: out of the overlap the secondary spectrum is
-//     zero and the flush leaves out what was not asked for; the odd frames' sign
-//     and the grid's conjugate are in the ramp.  Predicates per bin and product and
-//     the sign on the secondary spectrum cost 1.1k of 26.4k warp instructions per
-//     frame pair: FFT 8192, 40000 frame pairs 1371 -> 1315 us, FFT 16384 (20000)
-//     1711 -> 1669 us;
+//     zero and the flush leaves out those bins and what was not asked for; the odd
+//     frames' sign and the grid's conjugate are in the ramp.  Predicates per bin and
+//     product and the sign on the secondary spectrum cost 1.1k of 26.4k warp
+//     instructions per frame pair: FFT 8192, 40000 frame pairs 1371 -> 1315 us, FFT
+//     16384 (20000) 1711 -> 1669 us;
 //   * four barriers per frame pair: after the first pass, after each
 //     radix-16 pass, and between the two halves of the accumulation.  The
 //     frame record is double-buffered so no barrier closes an iteration.
@@ -216,7 +216,7 @@ __device__ __forceinline__ bool fold_span(const CorrParams& p, int row, uint64_t
   const int qoff = g0 ? sb : -sb;   // secondary bin = primary bin + qoff
   // Which of the thread's bins lie in the overlap (bit i: acc[i]).  Every sum
   // runs unconditionally: the secondary spectrum is zero out of the overlap, and
-  // the flush leaves out the products that were not asked for.
+  // the flush leaves out those bins and the products that were not asked for.
   uint32_t inov = 0;
 #pragma unroll
   for (int i = 0; i < kSlots; ++i) {
@@ -235,9 +235,13 @@ __device__ __forceinline__ bool fold_span(const CorrParams& p, int row, uint64_t
 
   // Each address is this thread's alone: the atomics are additions that nothing
   // waits for, in order.  Loading the partials to add to them held a CTA up for
-  // about 5 us (FFT 8192, 125000 frame pairs, a flush every 32: 4040 us against 3985).
+  // about 5 us (FFT 8192, 125000 frame pairs, a flush every 32: 4092 us against 3958).
   auto flush = [&]() {
     const bool want_acf = (p.products & 1u) != 0, ov_only = (p.products & 16u) != 0;
+    // Which sums are kept, by bin.  Out of the overlap a zero secondary spectrum times
+    // an infinite or NaN primary bin is NaN.
+    const uint32_t keepP = want_acf ? (ov_only ? inov : ~0u) : 0u;
+    const uint32_t keepS = want_acf ? inov : 0u, keepX = want_xcf ? inov : 0u;
 #pragma unroll
     for (int i = 0; i < kSlots; ++i) {
       if (i == kSlots - 1 && tid != 0) continue;
@@ -246,13 +250,12 @@ __device__ __forceinline__ bool fold_span(const CorrParams& p, int row, uint64_t
       const int bin = ROWS == 1 ? ((i == kSlots - 1) ? kN / 4 : ((i & 1) ? kN / 2 - j : j))
                                 : ((i == kSlots - 1) ? NF / 4
                                    : ((i & 1) ? NF / 2 - 2 * j - row : 2 * j + row));
-      const bool in = (inov >> i) & 1u;
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
         const int col = v == 0 ? colP : (v == 1 ? colS : v);
         double* q = part + (size_t)col * HF + bin;
         float x = acc[i][v];
-        if (v == 0 ? !(want_acf && (!ov_only || in)) : (v == 1 ? !want_acf : !want_xcf)) x = 0.f;
+        if (!(((v == 0 ? keepP : (v == 1 ? keepS : keepX)) >> i) & 1u)) x = 0.f;
         if (v == 3 && !g0) x = -x;  // grid 1: the conjugate was summed
         if (first_flush) *q = 0.0 + (double)x;
         else atomicAdd(q, (double)x);

@@ -257,14 +257,15 @@ __global__ void __cluster_dims__(C / 2, 1, 1) __launch_bounds__(kT, 1)
   float acc_h[4] = {0.f, 0.f, 0.f, 0.f};
 
   // Every sum runs for every bin: out of the overlap the secondary spectrum is
-  // zero, and the products that were not asked for are left out here.  (Predicates
-  // per bin and product, and the odd frames' sign on every secondary value: FFT
-  // 16384 odd shift, 8001 frame pairs 736 -> 711 us 1-bit, 786 -> 754 us 2-bit; 32768
-  // (6000) 1209 -> 1176; 65536 (3001) 1413 -> 1375 us.)
+  // zero; those bins and the products that were not asked for are left out here.
+  // (Predicates per bin and product, and the odd frames' sign on every secondary
+  // value: FFT 16384 odd shift, 8001 frame pairs 736 -> 711 us 1-bit, 786 -> 754 us
+  // 2-bit; 32768 (6000) 1209 -> 1176; 65536 (3001) 1413 -> 1375 us.)
   auto add_part = [&](int bin, int v, float x) {
     const int col = v == 0 ? colP : (v == 1 ? colS : v);
     const bool in = (unsigned)(bin - ovs) < (unsigned)ov;
-    if (v == 0 ? !(want_acf && (!ov_only || in)) : (v == 1 ? !want_acf : !want_xcf)) x = 0.f;
+    // (a zero secondary spectrum times an infinite or NaN primary bin is NaN)
+    if (v == 0 ? !(want_acf && (!ov_only || in)) : !(in && (v == 1 ? want_acf : want_xcf))) x = 0.f;
     if (v == 3 && !g0) x = -x;  // grid 1: the conjugate was summed
     double* d = part + (size_t)col * H + bin;
     *d = (first_flush ? 0.0 : *d) + (double)x;

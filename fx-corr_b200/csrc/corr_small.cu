@@ -19,8 +19,8 @@
 //   4. two-for-one split at the bin and at the band-shifted bin, |P|^2, |S|^2 and
 //      P conj(S) times the phase ramp into f32 registers, flushed every 32 frames
 //      to f64 partials.  All sums run unconditionally: out of the overlap the
-//      secondary spectrum is zero, and the flush leaves out what was not asked
-//      for.
+//      secondary spectrum is zero, and the flush leaves out those bins and what was
+//      not asked for.
 // Bound by instruction issue (65 % of the slots with 16 warps per SM; 1000 of 1660
 // instructions per thread and frame pair of FFT 4096 are the FFT's and the sums'
 // FP32).  Against the general form it replaces (words rewritten by LUT for every
@@ -180,7 +180,8 @@ __device__ __forceinline__ bool small_span(const CorrParams& p, uint64_t it0, ui
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
         float x = acc[i][v];
-        if (v == 0 ? !(want_acf && (!ov_only || in)) : (v == 1 ? !want_acf : !want_xcf)) x = 0.f;
+        // (a zero secondary spectrum times an infinite or NaN primary bin is NaN)
+        if (!(v < 2 ? want_acf : want_xcf) || (!in && (v > 0 || ov_only))) x = 0.f;
         if (v == 3 && !g0) x = -x;  // grid 1: the conjugate was summed
         double* q = part + (size_t)(v == 0 ? colP : (v == 1 ? colS : v)) * H + bin;
         if (first_flush) *q = 0.0 + (double)x;
