@@ -158,45 +158,46 @@ fxc_status set_shape(fxc_batch* b, int g, int fpc, uint32_t item_frames) {
 }
 
 // Grows the device arena / partials (waiting for the previous call's work,
-// whose graphs point at the old buffers) and the pinned staging.
+// whose graphs point at the old buffers) and the pinned staging.  Without room in
+// the engine's budget nothing has changed.
 fxc_status grow(fxc_batch* b, fxc_batch::Arena& A, uint64_t arena_bytes, uint64_t part_elems) {
-  if (arena_bytes > A.cap || part_elems > b->part_cap) {
+  const uint64_t arena_want = arena_bytes > A.cap ? std::max<uint64_t>(arena_bytes, 2 * A.cap) : 0;
+  const uint64_t part_want =
+      part_elems > b->part_cap ? std::max<uint64_t>(part_elems, b->part_cap + b->part_cap / 2) : 0;
+  if (arena_want || part_want) {
+    const fxc_status st = engine_reserve(b->eng, arena_want + part_want * 8);
+    if (st != FXC_OK) return st;
+    b->charged += arena_want + part_want * 8;
     BCK(cudaEventSynchronize(b->ev_done));
     drop_graphs(b);
   }
-  if (arena_bytes > A.cap) {
-    const uint64_t want = std::max<uint64_t>(arena_bytes, 2 * A.cap);
-    fxc_status st = engine_reserve(b->eng, want);
-    if (st != FXC_OK) return st;
+  auto give_back = [&](uint64_t bytes) {
+    engine_release(b->eng, bytes);
+    b->charged -= bytes;
+  };
+  if (arena_want) {
     cudaFree(A.d);
-    engine_release(b->eng, A.cap);
-    b->charged -= std::min(b->charged, A.cap);
+    give_back(A.cap);
     A.d = nullptr;
     A.cap = 0;
-    const cudaError_t e = cudaMalloc(&A.d, want);
+    const cudaError_t e = cudaMalloc(&A.d, arena_want);
     if (e != cudaSuccess) {
-      engine_release(b->eng, want);
+      give_back(arena_want + part_want * 8);
       BCK(e);
     }
-    A.cap = want;
-    b->charged += want;
+    A.cap = arena_want;
   }
-  if (part_elems > b->part_cap) {
-    const uint64_t want = std::max<uint64_t>(part_elems, b->part_cap + b->part_cap / 2);
-    fxc_status st = engine_reserve(b->eng, want * 8);
-    if (st != FXC_OK) return st;
+  if (part_want) {
     cudaFree(b->d_part);
-    engine_release(b->eng, b->part_cap * 8);
-    b->charged -= std::min(b->charged, b->part_cap * 8);
+    give_back(b->part_cap * 8);
     b->d_part = nullptr;
     b->part_cap = 0;
-    const cudaError_t e = cudaMalloc(&b->d_part, want * 8);
+    const cudaError_t e = cudaMalloc(&b->d_part, part_want * 8);
     if (e != cudaSuccess) {
-      engine_release(b->eng, want * 8);
+      give_back(part_want * 8);
       BCK(e);
     }
-    b->part_cap = want;
-    b->charged += want * 8;
+    b->part_cap = part_want;
   }
   if (arena_bytes > A.hcap) {
     BCK(cudaEventSynchronize(A.staged));
@@ -241,7 +242,7 @@ uint64_t item_len(const Shape& sh, int g, int sms, uint64_t nf, bool exact) {
   return align_up(per, (uint64_t)sh.fpc);
 }
 
-// Whether a correlation group's short sectors run whole, one item each.  Such a
+// Whether a group's short sectors run whole, one item each.  Such a
 // sector's items have one f32 run each (at most 32 frames, kRun).  As one item it
 // keeps the runs, flushed to f64 at the same frames and so added in the same order:
 // the sums are the same bit for bit, and what else is in the call may decide.  An
@@ -286,7 +287,7 @@ bool whole_sectors(const std::vector<Entry>& ents, int g, int ctas) {
 fxc_status run_batch(fxc_batch* b, fxc_scan* const* scans, const uint8_t* const* r1,
                      const uint8_t* const* r2, const uint64_t* nf, const uint64_t* first,
                      double* const* acc, uint8_t* const* raw_out, uint32_t count,
-                     cudaStream_t stream, bool allow_graph);
+                     cudaStream_t stream, bool allow_graph, bool tight = false);
 
 // Times every variant x item size of group g on a synthetic batch and keeps
 // the fastest.  The caller holds b->mu.
@@ -423,7 +424,7 @@ fxc_status autotune_locked(fxc_batch* b, int g) {
 fxc_status run_batch(fxc_batch* b, fxc_scan* const* scans, const uint8_t* const* r1,
                      const uint8_t* const* r2, const uint64_t* nf, const uint64_t* first,
                      double* const* acc, uint8_t* const* raw_out, uint32_t count,
-                     cudaStream_t stream, bool allow_graph) {
+                     cudaStream_t stream, bool allow_graph, bool tight) {
   std::vector<Entry> ents;
   std::vector<uint32_t> others;
   ents.reserve(count);
@@ -475,14 +476,18 @@ fxc_status run_batch(fxc_batch* b, fxc_scan* const* scans, const uint8_t* const*
     const Shape& sh = b->shape[e.group];
     e.per = item_len(sh, e.group, b->sms, e.bs.p.nf, sh.pinned || b->tuning[e.group]);
   }
-  for (int g = 0; g < kCorrGroups; ++g) {
+  for (int g = 0; g < kBatchGroups; ++g) {
     const Shape& sh = b->shape[g];
     if (!(mask & (1u << g)) || sh.pinned || b->tuning[g]) continue;
-    const bool whole = whole_sectors(ents, g, b->sms * sh.ctas / (g == BG_16384 ? 2 : 1));
+    const bool whole =
+        tight || (!phased_group(g) &&
+                  whole_sectors(ents, g, b->sms * sh.ctas / (g == BG_16384 ? 2 : 1)));
     for (Entry& e : ents) {
       if (e.group != g) continue;
-      e.bs.p.flush_every = (uint32_t)(std::min(e.per, kRun) / sh.fpc);  // iterations
+      // iterations
+      e.bs.p.flush_every = e.bs.pp.flush_every = (uint32_t)(std::min(e.per, kRun) / sh.fpc);
       if (whole && e.per <= kRun) e.per = std::max(e.per, align_up(e.bs.p.nf, (uint64_t)sh.fpc));
+      else if (tight) e.per = item_len(sh, g, b->sms, e.bs.p.nf, true);
     }
   }
   std::stable_sort(ents.begin(), ents.end(), [](const Entry& a, const Entry& c) {
@@ -519,6 +524,8 @@ fxc_status run_batch(fxc_batch* b, fxc_scan* const* scans, const uint8_t* const*
   hdr.nframes = fi;
   hdr.nbins = bins;
 
+  bool tuning = false;
+  for (bool t : b->tuning) tuning = tuning || t;
   BCK(cudaStreamWaitEvent(stream, b->ev_done, 0));
   if (!ents.empty()) {
     const uint64_t off_scans = align_up(sizeof(BatchHeader), 256);
@@ -528,6 +535,20 @@ fxc_status run_batch(fxc_batch* b, fxc_scan* const* scans, const uint8_t* const*
     b->next_arena ^= 1;
     fxc_batch::Arena& A = b->arena[ai];
     fxc_status st = grow(b, A, bytes, std::max<uint64_t>(part, 1));
+    if ((st == FXC_EBUSY || st == FXC_ENOMEM) && !tuning) {
+      // No room for the partials of every item: half the sectors at a time, with the
+      // same sums; one alone whole or, where its items have several runs, in items of
+      // the group's size.  A split sector has up to 24 times an unsplit one's partials.
+      auto half = [&](uint32_t k, uint32_t n, bool t) {
+        return run_batch(b, scans + k, r1 + k, r2 + k, nf + k, first + k, acc + k,
+                         raw_out ? raw_out + k : nullptr, n, stream, allow_graph, t);
+      };
+      if (count > 1) {
+        st = half(0, count / 2, false);
+        return st == FXC_OK ? half(count / 2, count - count / 2, false) : st;
+      }
+      if (!tight) return half(0, 1, true);
+    }
     if (st != FXC_OK) return st;
     BCK(cudaEventSynchronize(A.staged));  // the call before the previous one
     hdr.scans = reinterpret_cast<const BatchScan*>(A.d + off_scans);

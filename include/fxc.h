@@ -299,7 +299,10 @@ FXC_API fxc_status fxc_server_destroy(fxc_server* sv);
  * path on the same stream.  A sector's products equal fxc_sector_run_device's within the
  * library's FP32 tolerance (phased .raw frames byte for byte), and are
  * identical bit for bit whatever else shares the batch (the order of its sums
- * depends only on the sector's frame count and the batch's tuning). */
+ * depends only on the sector's frame count and the batch's tuning; a sector of
+ * more than 768 frames in an engine without room for its partials alone is the
+ * exception).  A call whose partials do not fit the engine's HBM budget runs
+ * fewer sectors at a time. */
 typedef struct fxc_batch fxc_batch;
 
 typedef struct fxc_batch_opts {

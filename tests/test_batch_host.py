@@ -90,3 +90,40 @@ def test_many_short_sectors_run_whole(batch):
     # sectors whose items have several runs stay split
     (items,) = groups(batch("items", (8192, 0, 2000, 512))).values()
     assert len(items) == 512 * 24
+
+
+@pytest.mark.parametrize("sector,count,budget", [
+    ((8192, 0, 100), 10, 1_600_000),     # a slot of 131 KB a sector and the tables
+    ((8192, 0, 100), 40, 6_000_000),
+    ((16384, 0, 100), 30, 10_000_000),
+    ((1024, 0, 300), 500, 10_000_000),
+    ((8192, 1, 64), 64, 2_500_000),
+    ((4096, 0, 2000), 1, 1_500_000),     # one sector, items of several runs
+    ((8192, 0, 100), 1, 200_000)])
+def test_no_room_for_every_item(batch, sector, count, budget):
+    """A call whose sectors' partials would fit unsplit is taken: fewer sectors at a
+    time or, one alone, fewer items, its runs the same wherever an item has one."""
+    out = batch("items", (*sector, count), budget=budget)
+    assert out["status"] == OK and out["in_use"] <= budget
+    fft, phased, nf = sector
+    free = groups(batch("items", (*sector, 1)))
+    fpc = {1024: 4}.get(fft, 1)
+    one_run = max(f1 - f0 for items in free.values() for _, _, f0, f1, _, _ in items) <= 32
+    seen = 0
+    for ln in out["launches"]:
+        frames = {}
+        for scan, row, f0, f1, part, flush in ln["items"]:
+            frames.setdefault((scan, row), []).append((f0, f1))
+            if one_run:
+                assert f1 - f0 <= flush * fpc or (f0, f1) == (0, nf)
+                assert flush == next(iter(free.values()))[0][-1]
+        for (scan, row), f in frames.items():  # every frame once
+            assert [a for a, _ in sorted(f)] == [0] + [b for _, b in sorted(f)][:-1]
+            assert max(b for _, b in f) == nf
+            seen += row == 0
+    assert seen == count
+
+
+def test_budget_too_small_stays_refused(batch):
+    out = batch("items", (8192, 0, 100, 10), budget=100_000)
+    assert out["status"] == EBUSY and not out["launches"]

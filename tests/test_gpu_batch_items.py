@@ -104,3 +104,46 @@ def test_short_sector_alone_and_among_many(engine, fxc_lib, fft, nf, many):
     for c in opened:
         for s in c:
             s.close()
+
+
+def test_little_budget(engine, fxc_lib):
+    """An engine whose budget has room for its scans and half of a call's partials: the
+    call is taken, with the same sums bit for bit."""
+    import torch
+
+    sc = make_scan(fft=1024, fs=512e6, band=(-8, 40, 512, 32), delay=DELAY, shuffle="generic")
+    nf, n = 300, 24  # ten items, 10 x 16416 bytes of partials, a sector
+    r1, r2 = signal_raw(sc, nf, seed=5, rho=0.3, delay_samples=2.6)
+    d1, d2 = (torch.from_numpy(np.ascontiguousarray(r)).cuda() for r in (r1, r2))
+
+    def run(eng, scans):
+        acc = [torch.zeros(5 * 513, dtype=torch.float64, device="cuda") for _ in range(n)]
+        batch = fxc_lib.Batch(eng)
+        batch.run_device(scans, [d1] * n, [d2] * n, [nf] * n, [3 + k for k in range(n)], acc)
+        torch.cuda.synchronize()
+        batch.close()
+        return acc
+
+    def opened(budget):
+        eng = fxc_lib.Engine(0, hbm_budget_bytes=budget)
+        try:
+            return eng, [eng.open_scan(to_fxc(sc)) for _ in range(n)]
+        except fxc_lib.FxcError as e:
+            assert e.status == fxc_lib.EBUSY
+            eng.close()
+            return None
+
+    lo, hi = 1 << 20, 1 << 30  # too little for the scans, enough
+    while hi - lo > 1 << 18:
+        mid = (lo + hi) // 2
+        got = opened(mid)
+        lo, hi = (lo, mid) if got else (mid, hi)
+        if got:
+            got[0].close()
+    eng, scans = opened(hi + n * 10 * 16416 // 2)
+    ref_scans = [engine.open_scan(to_fxc(sc)) for _ in range(n)]
+    for a, b in zip(run(eng, scans), run(engine, ref_scans)):
+        assert torch.equal(a, b)
+    eng.close()
+    for s in ref_scans:
+        s.close()
