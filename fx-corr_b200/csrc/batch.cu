@@ -527,6 +527,14 @@ fxc_status run_batch(fxc_batch* b, fxc_scan* const* scans, const uint8_t* const*
   bool tuning = false;
   for (bool t : b->tuning) tuning = tuning || t;
   BCK(cudaStreamWaitEvent(stream, b->ev_done, 0));
+  // The next call waits for what this one has launched, also when it fails midway.
+  struct Done {
+    fxc_batch* b;
+    cudaStream_t s;
+    ~Done() {
+      if (b) cudaEventRecord(b->ev_done, s);
+    }
+  } done{b, stream};
   if (!ents.empty()) {
     const uint64_t off_scans = align_up(sizeof(BatchHeader), 256);
     const uint64_t off_items = off_scans + align_up(ents.size() * sizeof(BatchScan), 256);
@@ -578,21 +586,34 @@ fxc_status run_batch(fxc_batch* b, fxc_scan* const* scans, const uint8_t* const*
       // before it.  The slowest per frame first: phased, then by FFT length.
       const bool fork = (mask & (mask - 1u)) != 0;
       if (fork) BCK(cudaEventRecord(b->ev_fork, s));
-      for (int g = kBatchGroups - 1; g >= 0; --g) {
-        if (!(mask & (1u << g))) continue;
-        const Shape& sh = b->shape[g];
-        uint64_t grid = (uint64_t)b->sms * sh.ctas;
-        if (!full) grid = std::min<uint64_t>(grid, hdr.nitems[g]);
-        const cudaStream_t gs = fork ? b->side[g] : s;
-        if (fork) BCK(cudaStreamWaitEvent(gs, b->ev_fork, 0));
-        if (phased_group(g))
-          BCK(launch_phased_batch(kGroupN[g], a, g, (int)std::max<uint64_t>(grid, 1), gs));
-        else
-          BCK(launch_batch_group(g, sh.fpc, a, (int)std::max<uint64_t>(grid, 1), gs));
-        if (fork) BCK(cudaEventRecord(b->ev_join[g], gs));
+      uint32_t forked = 0;
+      auto run_groups = [&]() -> fxc_status {
+        for (int g = kBatchGroups - 1; g >= 0; --g) {
+          if (!(mask & (1u << g))) continue;
+          const Shape& sh = b->shape[g];
+          uint64_t grid = (uint64_t)b->sms * sh.ctas;
+          if (!full) grid = std::min<uint64_t>(grid, hdr.nitems[g]);
+          const cudaStream_t gs = fork ? b->side[g] : s;
+          if (fork) BCK(cudaStreamWaitEvent(gs, b->ev_fork, 0));
+          if (fork) forked |= 1u << g;
+          if (phased_group(g))
+            BCK(launch_phased_batch(kGroupN[g], a, g, (int)std::max<uint64_t>(grid, 1), gs));
+          else
+            BCK(launch_batch_group(g, sh.fpc, a, (int)std::max<uint64_t>(grid, 1), gs));
+        }
+        return FXC_OK;
+      };
+      fxc_status gst = run_groups();
+      // after an error too: what was launched comes before the stream's next work
+      for (int g = 0; g < kBatchGroups; ++g) {
+        if (!(forked & (1u << g))) continue;
+        cudaError_t e = cudaEventRecord(b->ev_join[g], b->side[g]);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(s, b->ev_join[g], 0);
+        if (e == cudaSuccess) continue;
+        if (!full) cudaStreamSynchronize(b->side[g]);
+        if (gst == FXC_OK) gst = internal_fail(FXC_ECUDA, cudaGetErrorString(e));
       }
-      for (int g = 0; fork && g < kBatchGroups; ++g)
-        if (mask & (1u << g)) BCK(cudaStreamWaitEvent(s, b->ev_join[g], 0));
+      if (gst != FXC_OK) return gst;
       const uint64_t rgrid = full ? (uint64_t)grid_aux
                                   : std::min<uint64_t>((uint64_t)grid_aux, (4 * hdr.nbins + 255) / 256);
       BCK(launch_batch_reduce(a, (int)std::max<uint64_t>(rgrid, 1), s));
@@ -629,6 +650,7 @@ fxc_status run_batch(fxc_batch* b, fxc_scan* const* scans, const uint8_t* const*
                                         raw_out ? raw_out[i] : nullptr, stream);
     if (st != FXC_OK) return st;
   }
+  done.b = nullptr;
   BCK(cudaEventRecord(b->ev_done, stream));
   return FXC_OK;
 }

@@ -127,3 +127,16 @@ def test_no_room_for_every_item(batch, sector, count, budget):
 def test_budget_too_small_stays_refused(batch):
     out = batch("items", (8192, 0, 100, 10), budget=100_000)
     assert out["status"] == EBUSY and not out["launches"]
+
+
+@pytest.mark.parametrize("fail_at", range(5))
+def test_launches_before_an_error_are_waited_for(batch, fail_at):
+    """Records, three groups on streams of their own, reduction: when one of them fails,
+    whatever was launched comes before the caller's next work on its stream and before
+    the next call, on another stream."""
+    out = batch("error", (1024, 0, 300, 3), (8192, 0, 100, 2), (8192, 1, 100, 1), fail_at=fail_at)
+    assert out["status"] not in (OK, EBUSY) and out["again"] == OK
+    launched = set(range(fail_at))
+    assert out["stream"] == launched
+    again = out["launches"][fail_at + 1:]
+    assert again[0]["name"] == "records" and all(launched <= ln["before"] for ln in again)
