@@ -406,6 +406,7 @@ fxc_status autotune_locked(fxc_batch* b, int g) {
     if (result != FXC_OK) break;
     result = set_shape(b, g, best.fpc, best.item_frames);
     b->shape[g].tuned = true;
+    b->shape[g].pinned = b->item_override != 0;  // no longer the caller's (fxc_batch_set_shape)
     b->shape[g].gsps = (double)kScans * frames * 2.0 * fft_len / (best_ms * 1e-3) / 1e9;
   } while (false);
   cleanup();

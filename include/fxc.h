@@ -308,7 +308,8 @@ typedef struct fxc_batch fxc_batch;
 typedef struct fxc_batch_opts {
   int32_t use_graphs;        /* capture and replay CUDA graphs */
   int32_t autotune;          /* tune an FFT length at its first batch */
-  uint32_t item_frames;      /* frames per work item; 0 = tuned or the default */
+  uint32_t item_frames;      /* frames per work item, of short sectors too; 0 = the
+                                tuned or default size, less for short sectors */
 } fxc_batch_opts;
 
 FXC_API fxc_status fxc_batch_create(fxc_engine* e, const fxc_batch_opts* opts, fxc_batch** out);
@@ -343,7 +344,7 @@ FXC_API fxc_status fxc_batch_shape(fxc_batch* b, uint32_t fft_len, int32_t* fpc,
                                    uint32_t* item_frames, int32_t* ctas_per_sm, double* gsps);
 /* Pins the shape of an FFT length: fpc a variant the length has (1024 and
  * 2048: 1, 2, 4; 4096: 1, 2; 8192 and 16384: 1), item_frames a positive
- * multiple of 32. */
+ * multiple of 32, kept for short sectors too until fxc_batch_autotune replaces it. */
 FXC_API fxc_status fxc_batch_set_shape(fxc_batch* b, uint32_t fft_len, int32_t fpc,
                                        uint32_t item_frames);
 /* Kernels the batch launched so far (graph replays count their kernels). */

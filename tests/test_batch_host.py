@@ -140,3 +140,10 @@ def test_launches_before_an_error_are_waited_for(batch, fail_at):
     assert out["stream"] == launched
     again = out["launches"][fail_at + 1:]
     assert again[0]["name"] == "records" and all(launched <= ln["before"] for ln in again)
+
+
+def test_autotune_after_set_shape_splits_as_untouched(batch):
+    """The tuner replaces a shape that the caller had pinned: short sectors are split by
+    their own length again, as in a batch whose shape nobody has set."""
+    pinned, free = (groups(batch(cmd, (8192, 0, 30, 1))) for cmd in ("pinned", "items"))
+    assert len(free[3]) > 1 and [i[2:4] for i in pinned[3]] == [i[2:4] for i in free[3]]
