@@ -476,6 +476,8 @@ fxc_status run_batch(fxc_batch* b, fxc_scan* const* scans, const uint8_t* const*
   for (Entry& e : ents) {
     const Shape& sh = b->shape[e.group];
     e.per = item_len(sh, e.group, b->sms, e.bs.p.nf, sh.pinned || b->tuning[e.group]);
+    // a run, in iterations of this shape (the scan's own kernel may have another)
+    e.bs.p.flush_every = e.bs.pp.flush_every = (uint32_t)(std::min(e.per, kRun) / sh.fpc);
   }
   for (int g = 0; g < kBatchGroups; ++g) {
     const Shape& sh = b->shape[g];
@@ -485,8 +487,6 @@ fxc_status run_batch(fxc_batch* b, fxc_scan* const* scans, const uint8_t* const*
                   whole_sectors(ents, g, b->sms * sh.ctas / (g == BG_16384 ? 2 : 1)));
     for (Entry& e : ents) {
       if (e.group != g) continue;
-      // iterations
-      e.bs.p.flush_every = e.bs.pp.flush_every = (uint32_t)(std::min(e.per, kRun) / sh.fpc);
       if (whole && e.per <= kRun) e.per = std::max(e.per, align_up(e.bs.p.nf, (uint64_t)sh.fpc));
       else if (tight) e.per = item_len(sh, g, b->sms, e.bs.p.nf, true);
     }

@@ -82,7 +82,7 @@ fxc_status batch_describe(fxc_scan* s, const uint8_t*, const uint8_t*, uint64_t 
   static const uint32_t len[] = {1024, 2048, 4096, 8192, 16384};
   BatchScan b{};
   b.p.nf = b.pp.nf = nf;
-  b.p.flush_every = b.pp.flush_every = 32;
+  b.p.flush_every = b.pp.flush_every = s->n < 4096 ? s->n / 128 : 32;  // 32 frames of its own kernel
   b.n = s->n;
   b.h = s->n / 2 + 1;
   b.phased = s->phased ? 1 : 0;
@@ -182,8 +182,9 @@ int main(int argc, char** argv) {
   cudaStream_t s[2];
   for (auto& x : s) cudaStreamCreateWithFlags(&x, 0);
   if (budget) g_engine.budget = budget;
-  if (cmd == "pinned") {  // a shape of the caller's, then the tuner's
+  if (cmd == "shape" || cmd == "pinned")  // a shape of the caller's
     if (fxc_batch_set_shape(b, c.scans[0]->n, 1, 64) != FXC_OK) return 3;
+  if (cmd == "pinned") {  // then the tuner's
     if (fxc_batch_autotune(b, c.scans[0]->n) != FXC_OK) return 3;
     g_log.clear();
   }

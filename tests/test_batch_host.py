@@ -147,3 +147,11 @@ def test_autotune_after_set_shape_splits_as_untouched(batch):
     their own length again, as in a batch whose shape nobody has set."""
     pinned, free = (groups(batch(cmd, (8192, 0, 30, 1))) for cmd in ("pinned", "items"))
     assert len(free[3]) > 1 and [i[2:4] for i in pinned[3]] == [i[2:4] for i in free[3]]
+
+
+@pytest.mark.parametrize("fft", [1024, 2048, 4096, 8192])
+def test_runs_of_a_pinned_shape(batch, fft):
+    """With one frame per iteration, whatever the scan's own kernel has, an f32 run is
+    32 iterations."""
+    (items,) = groups(batch("shape", (fft, 0, 300, 2))).values()
+    assert {(f0 % 64, flush) for _, _, f0, _, _, flush in items} == {(0, 32)}
