@@ -64,3 +64,30 @@ def test_far_beyond_the_levels_all_tie(engine, fft, bits):
                      w1=1e30, w2=1e30)
     r1, r2 = signal_raw(scan, 9, seed=fft, rho=0.4)
     assert not np.any(phased_raw(engine, scan, r1, r2, 9))
+
+
+@pytest.mark.parametrize("fft,bits", [
+    (1024, 2), (8192, 2), (2048, 4), (4096, 8), (16384, 2), (16384, 4), (16384, 8), (32768, 2),
+    (32768, 4), (65536, 2), (65536, 8)])
+def test_tables_in_any_order(engine, fft, bits):
+    """Levels in no order (sign and magnitude, two's complement) take the search, four
+    samples at a time: with station 1's codes renumbered the same way the samples are
+    the same, and so are the output's but for their numbers and ties."""
+    rng = np.random.Generator(np.random.PCG64(fft + bits))
+    up, nf = oracle.default_levels(bits), max(9, 200_000 // fft)
+    number = rng.permutation(1 << bits)  # new number of the old code
+    renumbered = [0.0] * (1 << bits)
+    for old, new in enumerate(number):
+        renumbered[new] = up[old]
+    byte = np.zeros(256, np.uint8)
+    for v in range(256):
+        for s in range(0, 8, bits):
+            byte[v] |= number[(v >> s) & ((1 << bits) - 1)] << s
+    scan = make_scan(fft=fft, fs=512e6, bits1=bits, bits2=bits, levels1=up, delay=DELAY,
+                     products=PROD, lsb1=True, lsb2=True, band=(8, 0, fft // 2 - 8, 8))
+    r1, r2 = signal_raw(scan, nf, seed=fft + bits, rho=0.4)
+    a = phased_raw(engine, scan, r1, r2, nf)
+    b = phased_raw(engine, dataclasses.replace(scan, levels1=renumbered), byte[r1], r2, nf)
+    differ = int(np.count_nonzero(byte[a] != b))
+    assert differ <= 3, (differ, a.size)
+    assert len(np.unique(a)) > 1
