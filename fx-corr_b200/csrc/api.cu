@@ -9,7 +9,6 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
-#include <limits>
 #include <atomic>
 #include <mutex>
 #include <string>
@@ -19,6 +18,7 @@
 #include "fxc.h"
 #include "fxc_internal.h"
 #include "fxc_kernels.h"
+#include "quant_table.h"
 
 using namespace fxc;
 
@@ -90,12 +90,6 @@ struct SectorSlot {
   bool busy = false;
 };
 
-// The re-quantiser's thresholds (fxc_device.cuh, quantise).
-struct QuantTable {
-  int32_t kind = QUANT_SEARCH;
-  float hi = 0.0f, step = 0.0f, offset = 0.0f;
-};
-
 struct fxc_scan {
   fxc_engine* eng = nullptr;
   fxc_scan_cfg cfg{};
@@ -160,60 +154,6 @@ void build_lut(const uint8_t sh[32], uint32_t* lut) {
     for (int v = 0; v < 256; ++v)
       if ((v >> bit) & 1) lut[byte * 256 + v] |= (1u << o);
   }
-}
-
-// Thresholds of the nearest-level rule (first index wins ties) for strictly
-// ascending levels: thr[i], i = 1..n-1, is the least f32 x whose rounded distance
-// to level i is below that to level i - 1.  Between two levels both rounded
-// distances are monotonic in x, so that is a step, found by bisection; and no
-// other level can be nearer or tie as long as the spacing does not vanish in the
-// rounding: levels no closer than 2^-20 of their range, |x| up to 2^20
-// spacings beyond them.  Other tables keep the search.
-QuantTable quant_thresholds(const float* lv, uint32_t n, bool ascending, float* thr) {
-  QuantTable q;
-  for (int i = 0; i < 257; ++i) thr[i] = std::numeric_limits<float>::infinity();
-  thr[0] = -thr[256];
-  if (!ascending || n < 2) return q;
-  double gap = 1e300;
-  for (uint32_t i = 1; i < n; ++i) gap = std::min(gap, (double)lv[i] - (double)lv[i - 1]);
-  const double top = std::max(std::fabs((double)lv[0]), std::fabs((double)lv[n - 1]));
-  if (!std::isfinite(top) || !(gap > 0x1p-100) || gap < top * 0x1p-20) return q;
-  // f32 values in order as integers
-  auto key = [](float x) {
-    int32_t b;
-    std::memcpy(&b, &x, 4);
-    return b < 0 ? (int64_t)INT32_MIN - b : (int64_t)b;
-  };
-  auto val = [](int64_t k) {
-    const int32_t b = k < 0 ? (int32_t)((int64_t)INT32_MIN - k) : (int32_t)k;
-    float x;
-    std::memcpy(&x, &b, 4);
-    return x;
-  };
-  for (uint32_t i = 1; i < n; ++i) {
-    int64_t lo = key(lv[i - 1]), hi = key(lv[i]);  // not past, past
-    while (hi - lo > 1) {
-      const int64_t m = lo + (hi - lo) / 2;
-      const float x = val(m);
-      const float below = std::fabs(x - lv[i - 1]), above = std::fabs(x - lv[i]);
-      if (above < below) hi = m;
-      else lo = m;
-    }
-    thr[i] = val(hi);
-  }
-  q.hi = (float)(gap * 0x1p+20);
-  if (n <= 4) {
-    q.kind = QUANT_COMPARE;
-    return q;
-  }
-  // a uniform table: the guess is right but next to a threshold
-  const double step = ((double)lv[n - 1] - (double)lv[0]) / (n - 1);
-  for (uint32_t i = 0; i < n; ++i)
-    if (std::fabs((double)lv[i] - ((double)lv[0] + i * step)) > 0.01 * step) return q;
-  q.kind = QUANT_STEP;
-  q.step = (float)(1.0 / step);
-  q.offset = (float)(0.5 - (double)lv[0] / step);
-  return q;
 }
 
 // Power of two nearest 1/RMS of a level table.  Both stations share one

@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "quant_table.h"
+
 namespace fxc {
 
 // ------------------------------------------------------------ parameters
@@ -706,7 +708,6 @@ __device__ __forceinline__ uint32_t nearest_level(float x, const float* __restri
 // by one level at most, and the two thresholds around it.  The general search
 // takes about 8 instructions per level; this 6 in all, or 12.  Values beyond
 // `hi` (where the distances round to ties) and NaN take the general search.
-enum : int32_t { QUANT_SEARCH = 0, QUANT_COMPARE = 1, QUANT_STEP = 2 };
 struct Quantiser {
   const float* ql;   // levels, then from 256 the thresholds
   int32_t n, monotonic, kind;
