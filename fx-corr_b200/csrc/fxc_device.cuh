@@ -745,7 +745,7 @@ static __device__ __noinline__ uint32_t nearest_four(float4 x, const float* ql, 
   }
   return best[0] | best[1] << 8 | best[2] << 16 | best[3] << 24;
 }
-// K (2, 4 or 8) samples at a time, one test of the thresholds' range for all.  COMPARE, STEP: the
+// K (4 or 8) samples at a time, one test of the thresholds' range for all.  COMPARE, STEP: the
 // kinds of table that the caller can meet, any other takes the search (`thr`: the
 // thresholds; t = thr[1..3]).
 template <bool COMPARE, bool STEP, int K>
@@ -770,10 +770,9 @@ __device__ __forceinline__ void quantise_many(const float (&x)[K], const Quantis
 #pragma unroll
     for (int k = 0; k < K; k += 4) {
       const uint32_t four =
-          nearest_four(make_float4(x[k], x[k + 1], x[K > 2 ? k + 2 : k], x[K > 2 ? k + 3 : k]), q.ql,
-                       q.n, q.monotonic);
+          nearest_four(make_float4(x[k], x[k + 1], x[k + 2], x[k + 3]), q.ql, q.n, q.monotonic);
 #pragma unroll
-      for (int j = 0; j < 4 && k + j < K; ++j) c[k + j] = (four >> (8 * j)) & 255u;
+      for (int j = 0; j < 4; ++j) c[k + j] = (four >> (8 * j)) & 255u;
     }
   }
 }

@@ -17,9 +17,9 @@
 //                         each frame group (<= 32 frames), then f64 per-group partials
 //                         reduced by reduce_partials_kernel.
 //   phased_global_kernel  per-bin phased synthesis (src/main.rs:2222-2365) and the
-//                         Hermitian-extended inverse input; rows_fft_complex_kernel<C>
-//                         (C <= 4) or dif_kernel + cfft_kernel its FFT; quant_global_kernel
-//                         the re-quantised .raw frames (src/utils.rs:378-410).
+//                         Hermitian-extended inverse input; rows_fft_complex_kernel<4>
+//                         or dif_kernel<8> + cfft_kernel its FFT; quant_global_kernel the
+//                         re-quantised .raw frames (src/utils.rs:378-410).  C = 4, 8.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -831,19 +831,16 @@ static int grid_for(uint64_t work, int threads, int sms) {
   return (int)(g < (uint64_t)sms * 8 ? (g ? g : 1) : (uint64_t)sms * 8);
 }
 
-// DIF over C columns (buf0 -> buf1), then the M-point row FFTs in place on buf1.
+// DIF over C columns (buf0 -> buf1), then the M-point row FFTs in place on buf1
+// (eight rows, FFT 65536).
 static cudaError_t row_ffts(const LargeParams& p, uint64_t nb, float2* buf1, int sms,
                            cudaStream_t s);
 
 static cudaError_t large_fft_core(const LargeParams& p, uint64_t nb, const float2* buf0,
                                   float2* buf1, int sms, cudaStream_t s) {
   const uint64_t work = nb * kLargeM;
-  switch (p.c) {
-    case 2: dif_kernel<2><<<grid_for(work, 256, sms), 256, 0, s>>>(buf0, buf1, nb, p.tw); break;
-    case 4: dif_kernel<4><<<grid_for(work, 256, sms), 256, 0, s>>>(buf0, buf1, nb, p.tw); break;
-    case 8: dif_kernel<8><<<grid_for(work, 256, sms), 256, 0, s>>>(buf0, buf1, nb, p.tw); break;
-    default: return cudaErrorInvalidValue;
-  }
+  if (p.c != 8) return cudaErrorInvalidValue;
+  dif_kernel<8><<<grid_for(work, 256, sms), 256, 0, s>>>(buf0, buf1, nb, p.tw);
   return row_ffts(p, nb, buf1, sms, s);
 }
 
@@ -897,30 +894,16 @@ cudaError_t launch_rows_fft(const LargeParams& p, uint64_t f0, uint64_t nb, floa
   return cudaGetLastError();
 }
 
-// The DIF step and the row FFTs of a complex input in global memory (x -> y).
+// The DIF step and the row FFTs of a complex input in global memory (x -> y; four
+// rows, FFT 32768).
 cudaError_t launch_rows_fft_complex(const LargeParams& p, uint64_t nb, const float2* x, float2* y,
                                     int sms, cudaStream_t s) {
   const uint32_t smem = 2 * kRwBuf;
   const unsigned grid = (unsigned)std::min<uint64_t>(nb * (uint64_t)p.c, (uint64_t)sms);
-  cudaError_t e;
-  switch (p.c) {
-    case 2:
-      e = cudaFuncSetAttribute(rows_fft_complex_kernel<2>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e == cudaSuccess) rows_fft_complex_kernel<2><<<grid, 512, smem, s>>>(x, y, nb, p.tw);
-      break;
-    case 4:
-      e = cudaFuncSetAttribute(rows_fft_complex_kernel<4>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e == cudaSuccess) rows_fft_complex_kernel<4><<<grid, 512, smem, s>>>(x, y, nb, p.tw);
-      break;
-    case 8:
-      e = cudaFuncSetAttribute(rows_fft_complex_kernel<8>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e == cudaSuccess) rows_fft_complex_kernel<8><<<grid, 512, smem, s>>>(x, y, nb, p.tw);
-      break;
-    default: return cudaErrorInvalidValue;
-  }
+  if (p.c != 4) return cudaErrorInvalidValue;
+  const cudaError_t e = cudaFuncSetAttribute(
+      rows_fft_complex_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) rows_fft_complex_kernel<4><<<grid, 512, smem, s>>>(x, y, nb, p.tw);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }
@@ -976,12 +959,12 @@ cudaError_t launch_large_phased(const LargeParams& p, const PhasedParams& pp, fl
   phased_global_kernel<<<grid, 256, 0, s>>>(p, pp, buf1, f0, nb, first_batch, part, buf0);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || !pp.want_raw) return e;
-  e = p.c <= 4 ? launch_rows_fft_complex(p, nb, buf0, buf1, sms, s)
+  // FFT 32768 and 65536: the phased products of FFT 16384 are the two-row kernel's
+  e = p.c == 4 ? launch_rows_fft_complex(p, nb, buf0, buf1, sms, s)
                : large_fft_core(p, nb, buf0, buf1, sms, s);
   if (e != cudaSuccess) return e;
   const int ctas = grid_for(nb * (uint64_t)kLargeM, 256, sms);
   switch (p.c) {
-    case 2: quant_global_kernel<2><<<ctas, 256, 0, s>>>(pp, buf1, f0, nb); break;
     case 4: quant_global_kernel<4><<<ctas, 256, 0, s>>>(pp, buf1, f0, nb); break;
     case 8: quant_global_kernel<8><<<ctas, 256, 0, s>>>(pp, buf1, f0, nb); break;
     default: return cudaErrorInvalidValue;
