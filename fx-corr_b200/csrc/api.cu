@@ -517,7 +517,7 @@ fxc_status run_corr_stage(fxc_scan* s, const uint8_t* r1, const uint8_t* r2, uin
                                corr_cluster_size(s->n));
     CK(launch_corr_cluster(s->n, p, nblk, st));
   } else {
-    CK(launch_corr(s->n, MODE_CORR, p, grid, st));
+    CK(launch_corr(s->n, p, grid, st));
   }
   if (ev) CK(cudaEventRecord(ev->second, st));
   const double u1 = 1.0 / s->scale[0], u2 = 1.0 / s->scale[1];
@@ -1068,7 +1068,7 @@ fxc_status fxc_decode_device(fxc_scan* s, const uint8_t* d_raw1, const uint8_t* 
     CK(launch_fold_decode(p, grid, (cudaStream_t)stream));
     return FXC_OK;
   }
-  CK(launch_corr(s->n, MODE_DECODE, p, corr_grid(s, nf), (cudaStream_t)stream));
+  CK(launch_row_decode(s->n, p, s->eng->sm_count, (cudaStream_t)stream));
   return FXC_OK;
 }
 
@@ -1097,7 +1097,7 @@ fxc_status fxc_spectra_device(fxc_scan* s, const uint8_t* d_raw1, const uint8_t*
   CorrParams p = corr_params(s, d_raw1, d_raw2, nf, first_frame);
   p.out_a = d_s1;
   p.out_b = d_s2;
-  CK(launch_corr(s->n, MODE_SPECTRA, p, corr_grid(s, nf), (cudaStream_t)stream));
+  CK(launch_spectra(s->n, p, corr_grid(s, nf), (cudaStream_t)stream));
   return FXC_OK;
 }
 

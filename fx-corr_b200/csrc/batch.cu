@@ -52,7 +52,7 @@ constexpr uint32_t kGroupN[kBatchGroups] = {1024, 2048, 4096, 8192, 16384,
 // groups have one variant each (the single-scan phased kernel's)
 const std::vector<int> kGroupFpc[kBatchGroups] = {{1, 2, 4}, {1, 2, 4}, {1, 2}, {1}, {1},
                                                   {4}, {2}, {1}, {1}, {1}};
-// single-scan defaults: the frames per iteration of corr_kernel / phased_kernel
+// single-scan defaults: the frames per iteration of the scan's own kernels
 constexpr int kDefaultFpc[kBatchGroups] = {4, 2, 1, 1, 1, 4, 2, 1, 1, 1};
 
 bool phased_group(int g) { return g >= kCorrGroups; }

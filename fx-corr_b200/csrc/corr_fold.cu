@@ -1,9 +1,8 @@
 // corr_fold.cu — the FFT-8192 correlation kernel (the full-rate path).
 //
-// Same contract as corr_kernel<8192, 1, MODE_CORR> (src/main.rs:2491-2568
-// per frame pair, partials reduced by reduce_partials_kernel), arranged to
-// spend as few shared-memory wavefronts and barriers per frame pair as the
-// data flow allows:
+// src/main.rs:2491-2568 per frame pair, one CTA a frame pair, partials [4][H] per
+// CTA reduced by reduce_partials_kernel, arranged to spend as few shared-memory
+// wavefronts and barriers per frame pair as the data flow allows:
 //   * decode straight from the staged .raw words: each thread's 16 samples of
 //     a station sit at one bit position of 16 words (the frame stride N/16 is
 //     a whole number of words), so a sample costs a word load, a rotate and a

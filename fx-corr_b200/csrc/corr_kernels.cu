@@ -5,8 +5,8 @@
 // 48-byte FrameInfo records; batch_frame_info_kernel does so for every sector of
 // a batch.
 //
-// corr_kernel is the stage entry points' kernel (FFT <= 8192): decode + integer
-// shift (MODE_DECODE), or the spectra of both stations (MODE_SPECTRA).  One CTA
+// spectra_kernel is the spectra stage's kernel (FFT <= 8192): both stations'
+// spectra of every frame, by a decode of its own.  One CTA
 // processes a contiguous run of frame pairs: FrameInfo and packed words arrive
 // by cp.async.bulk tracked by an mbarrier, two stages deep; 32-bit word shuffle,
 // b-bit codes -> f32 levels, LSB->USB flip of odd samples (src/utils.rs:215-376),
@@ -25,7 +25,7 @@
 
 namespace fxc {
 
-// Per-CTA setup of corr_kernel: mbarriers, error flag, twiddle chains.
+// Per-CTA setup of spectra_kernel: mbarriers, error flag, twiddle chains.
 template <int N, int FPC>
 __device__ __forceinline__ void corr_cta_init(const SmemLayout& L, uint8_t* smem, Twiddles<N>& tw) {
   constexpr int T1 = N / 16;
@@ -50,7 +50,7 @@ __device__ __forceinline__ void corr_cta_drain(const SmemLayout& L, uint8_t* sme
 
 // Iterations [it0, it1) (FPC frame pairs each) of the sector described by p into
 // p.out_a, p.out_b.
-template <int N, int FPC, int MODE>
+template <int N, int FPC>
 __device__ __forceinline__ void stage_span(const CorrParams& p, uint64_t it0, uint64_t it1,
                                            uint8_t* smem, const SmemLayout& L,
                                            const Twiddles<N>& tw) {
@@ -128,25 +128,6 @@ __device__ __forceinline__ void stage_span(const CorrParams& p, uint64_t it0, ui
     const PackedStation pb{w2 + g * (bpf2 / 4), lv + 256, (uint32_t)p.st[1].bits,
                            (1u << p.st[1].bits) - 1u, p.st[1].lsb ? 1 : 0, s2};
 
-    if constexpr (MODE == MODE_DECODE) {
-      if (valid) {
-        float* o1 = p.out_a + frame_local * N;
-        float* o2 = p.out_b + frame_local * N;
-        const float u1 = 1.0f / p.st[0].scale, u2 = 1.0f / p.st[1].scale;  // exact
-        for (int n = t; n < N; n += T1) {
-          const int m1 = n - s1, m2 = n - s2;
-          o1[n] = ((unsigned)m1 < (unsigned)N) ? packed_sample(pa, m1) * u1 : 0.f;
-          o2[n] = ((unsigned)m2 < (unsigned)N) ? packed_sample(pb, m2) * u2 : 0.f;
-        }
-      }
-      __syncthreads();
-      if (tid == 0 && it + kStages < it1) {
-        fence_proxy_async();
-        issue(it + kStages);
-      }
-      continue;
-    }
-
     float2* za = bufA + g * Geom<N>::CSTRIDE;
     float2* zb = bufB + g * Geom<N>::CSTRIDE;
     first_pass_packed<N>(pa, pb, za, t);
@@ -159,26 +140,23 @@ __device__ __forceinline__ void stage_span(const CorrParams& p, uint64_t it0, ui
     }
     __syncthreads();
 
-    if constexpr (MODE == MODE_SPECTRA) {
-      if (valid) {
-        float2* o1 = reinterpret_cast<float2*>(p.out_a) + frame_local * H;
-        float2* o2 = reinterpret_cast<float2*>(p.out_b) + frame_local * H;
-        const float u1 = 0.5f / p.st[0].scale, u2 = 0.5f / p.st[1].scale;  // exact
-        for (int k = t; k < H; k += T1) {
-          const float2 a = Z0[k], b = Z0[(N - k) & (N - 1)];
-          o1[k] = make_float2(u1 * (a.x + b.x), u1 * (a.y - b.y));
-          o2[k] = make_float2(u2 * (a.y + b.y), -u2 * (a.x - b.x));
-        }
+    if (valid) {
+      float2* o1 = reinterpret_cast<float2*>(p.out_a) + frame_local * H;
+      float2* o2 = reinterpret_cast<float2*>(p.out_b) + frame_local * H;
+      const float u1 = 0.5f / p.st[0].scale, u2 = 0.5f / p.st[1].scale;  // exact
+      for (int k = t; k < H; k += T1) {
+        const float2 a = Z0[k], b = Z0[(N - k) & (N - 1)];
+        o1[k] = make_float2(u1 * (a.x + b.x), u1 * (a.y - b.y));
+        o2[k] = make_float2(u2 * (a.y + b.y), -u2 * (a.x - b.x));
       }
-      __syncthreads();
-      continue;
     }
+    __syncthreads();
   }
 }
 
-template <int N, int FPC, int MODE>
+template <int N, int FPC>
 __global__ void __launch_bounds__(FPC * N / 16, (N >= 8192 ? 1 : 2))
-corr_kernel(const CorrParams p) {
+spectra_kernel(const CorrParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
   const SmemLayout L = smem_layout<N, FPC>(p.stage_bytes);
   Twiddles<N> tw;
@@ -187,7 +165,7 @@ corr_kernel(const CorrParams p) {
   const uint64_t iters = (p.nf + FPC - 1) / FPC;
   const uint64_t it0 = (blockIdx.x * iters) / gridDim.x;
   const uint64_t it1 = ((blockIdx.x + 1) * iters) / gridDim.x;
-  stage_span<N, FPC, MODE>(p, it0, it1, smem, L, tw);
+  stage_span<N, FPC>(p, it0, it1, smem, L, tw);
   corr_cta_drain(L, smem);
 }
 
@@ -388,10 +366,10 @@ __global__ void batch_reduce_kernel(const BatchArgs a) {
 
 // ------------------------------------------------------------- launchers
 
-template <int N, int FPC, int MODE>
+template <int N, int FPC>
 static cudaError_t launch_one(const CorrParams& p, int grid, cudaStream_t stream) {
   const SmemLayout L = smem_layout<N, FPC>(p.stage_bytes);
-  auto kern = corr_kernel<N, FPC, MODE>;
+  auto kern = spectra_kernel<N, FPC>;
   // the limit is shared by every host thread: always the largest layout
   // (8-bit stations), never lowered under a concurrent launch
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -401,34 +379,27 @@ static cudaError_t launch_one(const CorrParams& p, int grid, cudaStream_t stream
   return cudaGetLastError();
 }
 
-template <int MODE>
-static cudaError_t launch_mode(uint32_t n, const CorrParams& p, int grid, cudaStream_t s) {
-  if constexpr (MODE == MODE_CORR) {
-    // FFT 16384 as two 8192-point rows; odd band shifts take other kernels
-    if (n == 8192) return launch_corr_fold(p, grid, s);
-    if (n == 16384) return launch_corr_fold2(p, grid, s);
-    return launch_corr_small(n, p, grid, s);
-  } else {
-    switch (n) {
-      case 1024: return launch_one<1024, 4, MODE>(p, grid, s);
-      case 2048: return launch_one<2048, 2, MODE>(p, grid, s);
-      case 4096: return launch_one<4096, 1, MODE>(p, grid, s);
-      case 8192: return launch_one<8192, 1, MODE>(p, grid, s);
-      default: return cudaErrorInvalidValue;  // the four-step path
-    }
-  }
-}
-
 int corr_frames_per_cta_iter(uint32_t n) {
   return n == 1024 ? 4 : (n == 2048 ? 2 : 1);
 }
 
 int corr_ctas_per_sm(uint32_t n) { return n >= 8192 ? 1 : 2; }
 
-cudaError_t launch_corr(uint32_t n, int mode, const CorrParams& p, int grid, cudaStream_t s) {
-  if (mode == MODE_CORR) return launch_mode<MODE_CORR>(n, p, grid, s);
-  if (mode == MODE_SPECTRA) return launch_mode<MODE_SPECTRA>(n, p, grid, s);
-  return launch_mode<MODE_DECODE>(n, p, grid, s);
+cudaError_t launch_corr(uint32_t n, const CorrParams& p, int grid, cudaStream_t s) {
+  // FFT 16384 as two 8192-point rows; odd band shifts take other kernels
+  if (n == 8192) return launch_corr_fold(p, grid, s);
+  if (n == 16384) return launch_corr_fold2(p, grid, s);
+  return launch_corr_small(n, p, grid, s);
+}
+
+cudaError_t launch_spectra(uint32_t n, const CorrParams& p, int grid, cudaStream_t s) {
+  switch (n) {
+    case 1024: return launch_one<1024, 4>(p, grid, s);
+    case 2048: return launch_one<2048, 2>(p, grid, s);
+    case 4096: return launch_one<4096, 1>(p, grid, s);
+    case 8192: return launch_one<8192, 1>(p, grid, s);
+    default: return cudaErrorInvalidValue;  // the four-step path
+  }
 }
 
 // ------------------------------------------------------- batched launchers

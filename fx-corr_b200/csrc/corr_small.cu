@@ -41,7 +41,7 @@ namespace fxc {
 namespace {
 
 // Shared memory: decode tables [0, 4352), frame records (double-buffered), mbarriers,
-// flag and batch ticket up to 4608 + ..., byte LUTs, the two buffers, the stages.
+// flag and batch ticket, byte LUTs, the two buffers, the stages.
 template <int N, int FPC>
 struct SmallLayout {
   static constexpr uint32_t FI = kTabPos + 256;  // 2 FPC records
@@ -384,7 +384,70 @@ corr_small_batch_kernel(const BatchArgs a, int grp) {
   small_cta_drain<N, FPC>(smem);
 }
 
+// Decode + integer shift of FPC frame pairs a CTA iteration, by the correlation and
+// phased kernels' own tables and inputs (fold::row_station), written out as f32
+// samples (src/utils.rs:126-376).
+template <int N, int FPC>
+__global__ void __launch_bounds__(FPC * N / 16) row_decode_kernel(const CorrParams p) {
+  constexpr int T1 = N / 16, T = FPC * T1;
+  extern __shared__ __align__(128) uint8_t smem[];
+  const int tid = threadIdx.x, g = tid / T1, t = tid % T1;
+  const bool g0 = p.grid == 0;
+  const StationParams& sp = p.st[g0 ? 0 : 1];
+  const StationParams& ss = p.st[g0 ? 1 : 0];
+  const bool preP = rewritten(sp), preS = rewritten(ss);
+  const uint32_t* pos = reinterpret_cast<const uint32_t*>(smem + kTabPos);
+  uint32_t* lut = reinterpret_cast<uint32_t*>(smem + kTabLut);
+  uint32_t* wP = reinterpret_cast<uint32_t*>(smem + kTabEnd);
+  uint32_t* wS = wP + FPC * (sp.bpf / 4);
+  build_decode_tables_at<true>(sp, ss, preP, preS, smem, lut, tid, T);
+  const bool splitP = split_2bit<true>(sp), splitS = split_2bit<true>(ss);
+  float* outP = g0 ? p.out_a : p.out_b;
+  float* outS = g0 ? p.out_b : p.out_a;
+  const float uP = 1.0f / sp.scale, uS = 1.0f / ss.scale;  // powers of two: exact
+  for (uint64_t f0 = (uint64_t)blockIdx.x * FPC; f0 < p.nf; f0 += (uint64_t)gridDim.x * FPC) {
+    const uint32_t nv = (uint32_t)(p.nf - f0 < (uint64_t)FPC ? p.nf - f0 : (uint64_t)FPC);
+    __syncthreads();  // tables built / previous frames' words consumed
+    const uint4* gP = reinterpret_cast<const uint4*>(sp.raw + f0 * sp.bpf);
+    const uint4* gS = reinterpret_cast<const uint4*>(ss.raw + f0 * ss.bpf);
+    for (uint32_t i = tid; i < nv * sp.bpf / 16; i += T) reinterpret_cast<uint4*>(wP)[i] = gP[i];
+    for (uint32_t i = tid; i < nv * ss.bpf / 16; i += T) reinterpret_cast<uint4*>(wS)[i] = gS[i];
+    __syncthreads();
+    if (preP || preS) {
+      preshuffle_slot(wP, nv * sp.bpf / 4, preP ? sp.shkind : SH_IDENTITY, lut, wS, nv * ss.bpf / 4,
+                      preS ? ss.shkind : SH_IDENTITY, lut + 1024, tid, T);
+      __syncthreads();
+    }
+    if (g >= (int)nv) continue;
+    const FrameInfo fi = p.finfo[f0 + g];
+    const int sP = g0 ? fi.s1 : fi.s2, sS = g0 ? fi.s2 : fi.s1;
+    const int mP = t - sP, mS = t - sS;
+    const uint32_t tbP = (uint32_t)((mP & (sp.lsb ? 1 : 0)) << (sp.bits + 2));
+    const uint32_t tbS = 2048u + (uint32_t)((mS & (ss.lsb ? 1 : 0)) << (ss.bits + 2));
+    float2 v[16];
+    fold::row_station<N, false>(sp.bits, splitP, wP + g * (sp.bpf / 4), smem, sP,
+                                pos[mP & ((32 / sp.bits) - 1)], tbP, v, t);
+    fold::row_station<N, true>(ss.bits, splitS, wS + g * (ss.bpf / 4), smem, sS,
+                               pos[32 + (mS & ((32 / ss.bits) - 1))], tbS, v, t);
+    float* oP = outP + (f0 + g) * N + t;
+    float* oS = outS + (f0 + g) * N + t;
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+      oP[r * T1] = v[r].x * uP;
+      oS[r * T1] = v[r].y * uS;
+    }
+  }
+}
+
 namespace {
+
+template <int N, int FPC>
+cudaError_t decode_one(const CorrParams& p, int sms, cudaStream_t s) {
+  const uint64_t iters = (p.nf + FPC - 1) / FPC;
+  const int grid = (int)(iters < (uint64_t)sms * 6 ? iters : (uint64_t)sms * 6);
+  row_decode_kernel<N, FPC><<<grid, FPC * N / 16, kTabEnd + 2u * FPC * N, s>>>(p);
+  return cudaGetLastError();
+}
 
 template <int N, int FPC>
 cudaError_t launch_one(const CorrParams& p, int grid, cudaStream_t s) {
@@ -451,6 +514,15 @@ cudaError_t launch_corr_small(uint32_t n, const CorrParams& p, int grid, cudaStr
     case 1024: return launch_one<1024, 4>(p, grid, s);
     case 2048: return launch_one<2048, 2>(p, grid, s);
     case 4096: return launch_one<4096, 1>(p, grid, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+cudaError_t launch_row_decode(uint32_t n, const CorrParams& p, int sms, cudaStream_t s) {
+  switch (n) {
+    case 1024: return decode_one<1024, 4>(p, sms, s);
+    case 2048: return decode_one<2048, 2>(p, sms, s);
+    case 4096: return decode_one<4096, 1>(p, sms, s);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -1,6 +1,5 @@
 // decode_tables.cuh — the shared-memory decode tables of the kernels that
-// decode straight from staged .raw words (the FFT-8192/16384 fold kernels, the
-// large-FFT staged kernels and the cluster kernel).
+// decode straight from staged .raw words (all but the spectra stage's).
 //
 // Layout, in bytes from the start of dynamic shared memory:
 //   [0, 4096)      levels: station a at 0, station b at 2048 (2^b f32 each,

@@ -1,6 +1,7 @@
-// fold_decode.cuh — the decode of the FFT-8192 / 16384 fold kernels: a
-// thread's 16 first-pass inputs of one station straight from the staged .raw
-// words (corr_fold.cu, phased_pair.cu).
+// fold_decode.cuh — a thread's 16 first-pass inputs of one station straight from
+// the staged .raw words: fold_inputs for one or two rows of 8192 points
+// (corr_fold.cu, phased_pair.cu), row_inputs for a frame of one row (corr_small.cu, FFT
+// 1024..4096; phased_kernels.cu, FFT 1024..8192).
 #pragma once
 
 #include <stdint.h>
@@ -109,7 +110,7 @@ __device__ __forceinline__ void fold_station(int bits, bool split, const uint32_
   }
 }
 
-// The same for a frame of one row of N points (N/16 threads; FFT 1024..4096):
+// The same for a frame of one row of N points (N/16 threads; FFT 1024..8192):
 // samples x[t + r N/16 - shift], r < 16.  The zero fill is checked for a half of
 // them only where the frame's shift reaches into it.
 template <int N, int BITS, bool IMAG, bool SPLIT>

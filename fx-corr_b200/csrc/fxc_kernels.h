@@ -32,8 +32,6 @@ inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, unsigned bloc
   return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
 }
 
-enum { MODE_CORR = 0, MODE_SPECTRA = 1, MODE_DECODE = 2 };
-
 struct CorrParams {
   StationParams st[2];
   DelayParams dl;
@@ -44,8 +42,8 @@ struct CorrParams {
   uint32_t flush_every;  // iterations between f32 -> f64 flushes
   double df_hz;
   const FrameInfo* finfo; // per-frame records of the sector (frame_info_kernel)
-  double* partials;      // MODE_CORR: [grid][4][H] f64
-  float* out_a;          // MODE_SPECTRA: S1 [nf][H] complex; MODE_DECODE: x1 [nf][N]
+  double* partials;      // correlation: [grid][4][H] f64
+  float* out_a;          // spectra: S1 [nf][H] complex; decode: x1 [nf][N]
   float* out_b;          // S2 / x2
   uint32_t* err;         // device error word (ERR_*)
   uint32_t wait_polls;   // polls before a staging wait gives up (0: kWaitPolls)
@@ -90,25 +88,28 @@ struct PhasedParams {
 
 int corr_frames_per_cta_iter(uint32_t n);
 int corr_ctas_per_sm(uint32_t n);
-cudaError_t launch_corr(uint32_t n, int mode, const CorrParams& p, int grid, cudaStream_t s);
-// FFT 1024..4096 correlation (MODE_CORR; corr_small.cu), corr_frames_per_cta_iter
+cudaError_t launch_corr(uint32_t n, const CorrParams& p, int grid, cudaStream_t s);
+// Both stations' spectra of every frame, FFT <= 8192
+cudaError_t launch_spectra(uint32_t n, const CorrParams& p, int grid, cudaStream_t s);
+// FFT 1024..4096 correlation (corr_small.cu), corr_frames_per_cta_iter
 // frame pairs per CTA iteration; its batched form by variant (batch_prepare etc.)
 cudaError_t launch_corr_small(uint32_t n, const CorrParams& p, int grid, cudaStream_t s);
 cudaError_t small_batch_prepare(int g, int fpc);
 int small_batch_ctas_per_sm(int g, int fpc);
 struct BatchArgs;
 cudaError_t launch_small_batch(int g, int fpc, const BatchArgs& a, int grid, cudaStream_t s);
-// FFT-8192 correlation (MODE_CORR), one frame pair per CTA iteration (corr_fold.cu)
+// FFT-8192 correlation, one frame pair per CTA iteration (corr_fold.cu)
 cudaError_t launch_corr_fold(const CorrParams& p, int grid, cudaStream_t s);
-// FFT-8192 decode + integer shift through the correlation kernel's own decode
-// path (fold_inputs), written out as f32 samples (MODE_DECODE semantics)
+// Decode + integer shift through the kernels' own decode paths (fold_inputs: FFT
+// 8192; row_inputs: 1024..4096), written out as f32 samples
 cudaError_t launch_fold_decode(const CorrParams& p, int grid, cudaStream_t s);
+cudaError_t launch_row_decode(uint32_t n, const CorrParams& p, int sms, cudaStream_t s);
 // FFT-16384 correlation as two 8192-point rows (corr_fold.cu); needs an even
 // band shift (a row holds the bins of one parity)
 bool corr_fold2_supported(const CorrParams& p);
 cudaError_t launch_corr_fold2(const CorrParams& p, int grid, cudaStream_t s);
 uint32_t fold_smem_bytes(uint32_t stage_bytes);
-// FFT 16384 / 32768 / 65536 correlation (MODE_CORR) by clusters of C = N / 8192
+// FFT 16384 / 32768 / 65536 correlation by clusters of C = N / 8192
 // CTAs exchanging through distributed shared memory (corr_cluster.cu): every
 // band shift and bit depth; partials [clusters][4][H].
 int corr_cluster_size(uint32_t n);      // C, 0 when N has no cluster kernel

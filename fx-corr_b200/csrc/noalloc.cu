@@ -225,7 +225,7 @@ extern "C" fxc_status fxc_sector_run_device_noalloc(const fxc_scan_cfg* cfg,
   const uint64_t fit = (kScratchBytes - kOffPartials) / (4ull * h * sizeof(double));
   const uint64_t grid = std::max<uint64_t>(
       1, std::min<uint64_t>({iters, (uint64_t)sms * corr_ctas_per_sm(n), fit}));
-  NA_CK(launch_corr(n, MODE_CORR, p, (int)grid, s));
+  NA_CK(launch_corr(n, p, (int)grid, s));
   const double u1 = 1.0 / scale[0], u2 = 1.0 / scale[1];
   NA_CK(launch_reduce(part, (int)grid, (int)h, 0.25 * u1 * u1, 0.25 * u2 * u2, 0.25 * u1 * u2,
                       d_acc, s));

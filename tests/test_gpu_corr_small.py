@@ -80,3 +80,34 @@ def test_bands_and_products(engine, fft, grid, products):
         scan = make_scan(fft=fft, fs=fs, grid=grid, band=band, products=products,
                          delay=delays(fs, 11, 4))
         check(engine, scan, 10, fft + grid, f"grid {grid} band {band} products {products}")
+
+
+@pytest.mark.parametrize("fft", [1024, 2048, 4096])
+@pytest.mark.parametrize("grid", [0, 1])
+@pytest.mark.parametrize("bits1,bits2,shuffle", [
+    (1, 4, "generic"), (2, 8, "pairswap"), (4, 2, "sample2"), (8, 4, "generic"),
+    (4, 8, "identity"), (2, 2, "generic")])
+def test_decode_bit_exact(engine, fft, grid, bits1, bits2, shuffle):
+    """The kernels' own decode, through the decode stage: rewritten words and raw ones,
+    integer shifts of every size, whichever station is the primary; frame counts that
+    leave a CTA iteration half empty."""
+    fs, nf = 32e6, 39
+    delay = dict(net_d1_base=-1.3 * fft / fs, total_rate1_base=2.7 / 40, net_d2_base=5.0 / fs,
+                 total_rate2_base=-0.05)
+    scan = make_scan(fft=fft, fs=fs, bits1=bits1, bits2=bits2, shuffle=shuffle, lsb1=True, grid=grid,
+                     delay=delay, seed=fft + bits1)
+    rng = np.random.Generator(np.random.PCG64(fft + bits2))
+    raws = [rng.integers(0, 256, nf * scan.bpf(b), dtype=np.uint8) for b in (bits1, bits2)]
+    s = engine.open_scan(to_fxc(scan))
+    got = s.decode(dev(raws[0]), dev(raws[1]), nf, first_frame=3)
+    s.check()
+    ents = oracle.c_delay_entries(scan, 3, nf)
+    for x, raw, bits, sh, lv, lsb, key in zip(
+            got, raws, (bits1, bits2), (scan.shuffle1, scan.shuffle2),
+            (scan.levels1, scan.levels2), (True, False), ("int1", "int2")):
+        x, bpf = x.cpu().numpy(), scan.bpf(bits)
+        for i in range(nf):
+            e = oracle.c_decode(raw[i * bpf:(i + 1) * bpf], fft, bits, sh, lv, lsb)
+            np.testing.assert_array_equal(x[i], oracle.c_shift(e, ents[key][i]))
+    assert min(ents["int1"]) <= -fft and max(ents["int1"]) >= fft
+    s.close()
