@@ -111,3 +111,37 @@ def test_decode_bit_exact(engine, fft, grid, bits1, bits2, shuffle):
             np.testing.assert_array_equal(x[i], oracle.c_shift(e, ents[key][i]))
     assert min(ents["int1"]) <= -fft and max(ents["int1"]) >= fft
     s.close()
+
+
+@pytest.mark.parametrize("fft,fpc", [(1024, 1), (1024, 2), (1024, 4), (2048, 1), (2048, 2),
+                                     (2048, 4), (4096, 1), (4096, 2)])
+def test_many_iterations(engine, fxc_lib, fft, fpc):
+    """CTAs with dozens of iterations (a batch's items of 96 frames and of the 13 left):
+    buffers that take turns, two copies in flight while words are rewritten in place,
+    several flushes and a ragged last run."""
+    import torch
+
+    nf, fs, half = 109, 512e6, fft // 2
+    scans = []
+    for k, (bits, shuffle, grid, band) in enumerate([
+            (4, "generic", 0, (0, 0, half + 1, 0)), (8, "generic", 1, (-7, 7, half, 0)),
+            (2, "generic", 0, (5, 100, half - 90, 105)), (1, "identity", 1, (0, 33, half, 33)),
+            (8, "pairswap", 0, (3, 0, half - 7, 3))]):
+        scan = make_scan(fft=fft, fs=fs, bits1=bits, bits2=bits, shuffle=shuffle, grid=grid, band=band,
+                         lsb1=k % 2 == 0, delay=delays(fs, 11 + 40 * k, 4 - 9 * k), seed=k)
+        scans.append((scan, *signal_raw(scan, nf, seed=fft + k, rho=0.3, delay_samples=2.6)))
+    opened = [engine.open_scan(to_fxc(sc)) for sc, *_ in scans]
+    acc = [torch.zeros(5 * (half + 1), dtype=torch.float64, device="cuda") for _ in scans]
+    batch = fxc_lib.Batch(engine)
+    batch.set_shape(fft, fpc, 96)
+    batch.run_device(opened, [dev(r1) for _, r1, _ in scans], [dev(r2) for *_, r2 in scans],
+                     [nf] * len(scans), [3] * len(scans), acc)
+    torch.cuda.synchronize()
+    for (sc, r1, r2), s, a in zip(scans, opened, acc):
+        s.check()
+        a, h = a.cpu().numpy(), half + 1
+        got = dict(acf11=a[:h], acf22=a[h:2 * h], xcf=a[2 * h:4 * h].view(np.complex128))
+        ref = oracle.fp64_sector_corr(sc, r1, r2, nf, first_frame=3)
+        assert_sector_close(got, ref, sc, f"{fft} {fpc} {sc.bits1} bits", nf=nf, ref_acf=ref)
+        s.close()
+    batch.close()

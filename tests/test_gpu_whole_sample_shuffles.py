@@ -68,3 +68,9 @@ def test_same_samples_same_products(engine, fft, bits, kind):
             assert np.array_equal(got[k], ref[k]), (products, shift, k)
         if products == PHASED:  # ant1's shuffle applied to the output words
             assert np.array_equal(got["raw"], shuffled(ref["raw"], sh1))
+
+
+@pytest.mark.parametrize("bits", [2, 4, 8])
+@pytest.mark.parametrize("kind", ["pairswap", "fields", "both", "torn"])
+def test_same_samples_same_products_2048(engine, bits, kind):
+    test_same_samples_same_products(engine, 2048, bits, kind)
