@@ -81,11 +81,11 @@ def test_short_sector_alone_and_among_many(engine, fxc_lib, fft, nf, many):
     opened = [[engine.open_scan(to_fxc(sc)) for sc, *_ in scans]
               for _ in range(-(-many // len(scans)))]
 
-    def run(copies):
+    def run(copies, graphs):
         acc = [[torch.zeros(5 * (fft // 2 + 1), dtype=torch.float64, device="cuda")
                 for _ in scans] for _ in copies]
         n = len(copies) * len(scans)
-        batch = fxc_lib.Batch(engine)
+        batch = fxc_lib.Batch(engine, use_graphs=graphs)
         batch.run_device([s for c in copies for s in c], [d1 for _ in copies for _, d1, _ in scans],
                          [d2 for _ in copies for _, _, d2 in scans], [nf] * n, [3] * n,
                          [a for c in acc for a in c])
@@ -93,7 +93,7 @@ def test_short_sector_alone_and_among_many(engine, fxc_lib, fft, nf, many):
         batch.close()
         return acc
 
-    alone, among = run(opened[:1])[0], run(opened)
+    alone, among = run(opened[:1], False)[0], run(opened, False) + run(opened, True)
     for k, (sc, d1, d2) in enumerate(scans):
         for c in among:
             assert torch.equal(c[k], alone[k])
