@@ -226,7 +226,7 @@ struct Entry {
 // with 128-frame items one group after another, 736 us with 16 items a sector and
 // the groups side by side, 583 with 24, 519 with 32; 64 sectors of FFT 8192,
 // 125-2000 frames: 2766 us with 64-frame items, 2776 with 16, 2753 with 24, 2792
-// with 32 (the partials).  So 24 for correlation and, four times smaller partials,
+// with 32 (the partials; all in call order: 2370 with 24, the longest first).  So 24 for correlation and, four times smaller partials,
 // 32 for phased sectors, of at least 2^15 samples per station: 24 sectors of
 // 2^17 samples 130 us a call, 220 with at least 2^16, 367 with 2^17.  The two-row
 // kernel has two items, one a row, and takes 2^16: 64 sectors of 16-62 frames 486 us

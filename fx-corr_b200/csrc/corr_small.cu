@@ -18,17 +18,17 @@
 //      three barriers in all;
 //   4. two-for-one split at the bin and at the band-shifted bin, |P|^2, |S|^2 and
 //      P conj(S) times the phase ramp into f32 registers, flushed every 32 frames
-//      to f64 partials.  All sums run unconditionally: out of the overlap the
+//      (p.flush_every iterations) to f64 partials.  All sums run unconditionally: out of the overlap the
 //      secondary spectrum is zero, and the flush leaves out those bins and what was
 //      not asked for.
-// Bound by instruction issue (65 % of the slots with 16 warps per SM; 1000 of 1660
+// Bound by instruction issue (66 % of the slots with 16 warps per SM; 1000 of 1660
 // instructions per thread and frame pair of FFT 4096 are the FFT's and the sums'
-// FP32).  Against the general form it replaces (words rewritten by LUT for every
+// FP32).  Against the general form it replaced (words rewritten by LUT for every
 // shuffle, a check and a sign per sample, grid selects and product predicates per
-// bin, five barriers), sector calls of 31250 frame pairs, 2-bit, no band shift:
-// FFT 1024 173 -> 141 us, 2048 291 -> 256, 4096 566 -> 502; 8-bit auto-spectra of FFT
-// 2048 (20011), pairs of bits swapped, 204 -> 167; 4-bit against 2-bit cross-spectra
-// of FFT 4096 (12207), LSB, shifted band 256 -> 237 us.
+// bin, five barriers, partials loaded to add to them), sector calls of 31250 frame
+// pairs, 2-bit, no band shift: FFT 1024 173 -> 141 us, 2048 291 -> 248, 4096 566 -> 488;
+// 8-bit auto-spectra of FFT 2048 (20011), pairs of bits swapped, 204 -> 164; 4-bit
+// against 2-bit cross-spectra of FFT 4096 (12207), LSB, shifted band 256 -> 228 us.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
