@@ -226,12 +226,13 @@ struct Entry {
 // with 128-frame items one group after another, 736 us with 16 items a sector and
 // the groups side by side, 583 with 24, 519 with 32; 64 sectors of FFT 8192,
 // 125-2000 frames: 2766 us with 64-frame items, 2776 with 16, 2753 with 24, 2792
-// with 32 (the partials; all in call order: 2370 with 24, the longest first).  So 24 for correlation and, four times smaller partials,
-// 32 for phased sectors, of at least 2^15 samples per station: 24 sectors of
-// 2^17 samples 130 us a call, 220 with at least 2^16, 367 with 2^17.  The two-row
-// kernel has two items, one a row, and takes 2^16: 64 sectors of 16-62 frames 486 us
-// with 2^15, 405 with 2^16.  Only the sector's own length counts, so that its sums do
-// not depend on what else is in the call.
+// with 32 (the partials; all in call order: with the longest first 2370 with 24).
+// So 24 for correlation and, four times smaller partials, 32 for phased sectors, of
+// at least 2^15 samples per station: 24 sectors of 2^17 samples 130 us a call, 220
+// with at least 2^16, 367 with 2^17.  The two-row kernel has two items, one a row, and
+// takes 2^16: 64 sectors of 16-62 frames 486 us with 2^15, 405 with 2^16.  Only the
+// sector's own length counts, so that its sums do not depend on what else is in the
+// call.
 uint64_t item_len(const Shape& sh, int g, int sms, uint64_t nf, bool exact) {
   const uint64_t maxn = (uint64_t)std::max(1, sms * sh.ctas);
   uint64_t per = sh.item_frames;
@@ -242,19 +243,19 @@ uint64_t item_len(const Shape& sh, int g, int sms, uint64_t nf, bool exact) {
   return align_up(per, (uint64_t)sh.fpc);
 }
 
-// Whether a group's short sectors run whole, one item each.  Such a
-// sector's items have one f32 run each (at most 32 frames, kRun).  As one item it
-// keeps the runs, flushed to f64 at the same frames and so added in the same order:
-// the sums are the same bit for bit, and what else is in the call may decide.  An
-// item costs about 1.5 frames beyond its own (ticket, tables, first copies, and
-// its partials, which the reduction reads again), a flush within an item 0.1; whole
-// sectors fill the CTAs less evenly, so they are dealt out here, the longest first,
-// as the tickets will.  1024 sectors of FFT 8192, 32-125 frames: 4600 us a call in
-// parts, 3590 whole, and a fifth of the partials; 256 of FFT 16384, 16-62 frames:
-// 1720 and 1190 us; 64 of them 400 and 480.  What stays in parts among many others
-// pays the items' cost: 1000 sectors of FFT 1024, 628 frames, 3430 us against 3290
-// with 128-frame items.  (Phased groups, with a quarter of the partials a frame,
-// stay in parts.)
+// Whether a group's short sectors run whole, one item each.  Such a sector's items
+// have one f32 run each (at most 32 frames, kRun).  As one item it keeps the runs,
+// flushed to f64 at the same frames and so added in the same order: the sums are
+// the same bit for bit, and what else is in the call may decide.  An item costs
+// about 1.5 frames beyond its own (ticket, tables, first copies, and its partials,
+// which the reduction reads again), a flush within an item 0.1; whole sectors fill
+// the CTAs less evenly, so they are dealt out here, the longest first, as the
+// tickets will.  1024 sectors of FFT 8192, 32-125 frames: 4600 us a call in parts,
+// 3590 whole, and a fifth of the partials; 256 of FFT 16384, 16-62 frames: 1720 and
+// 1190 us; 64 of them 400 and 480.  What stays in parts among many others pays the
+// items' cost: 1000 sectors of FFT 1024, 628 frames, 3430 us against 3290 with
+// 128-frame items.  (Phased groups, with a quarter of the partials a frame, stay in
+// parts.)
 constexpr uint64_t kRun = 32;
 bool whole_sectors(const std::vector<Entry>& ents, int g, int ctas) {
   double split = 0.0, shared = 0.0, longest = 0.0, sum = 0.0;  // frames

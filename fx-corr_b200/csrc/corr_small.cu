@@ -18,9 +18,9 @@
 //      three barriers in all;
 //   4. two-for-one split at the bin and at the band-shifted bin, |P|^2, |S|^2 and
 //      P conj(S) times the phase ramp into f32 registers, flushed every 32 frames
-//      (p.flush_every iterations) to f64 partials.  All sums run unconditionally: out of the overlap the
-//      secondary spectrum is zero, and the flush leaves out those bins and what was
-//      not asked for.
+//      (p.flush_every iterations) to f64 partials.  All sums run unconditionally:
+//      out of the overlap the secondary spectrum is zero, and the flush leaves out
+//      those bins and what was not asked for.
 // Bound by instruction issue (66 % of the slots with 16 warps per SM; 1000 of 1660
 // instructions per thread and frame pair of FFT 4096 are the FFT's and the sums'
 // FP32).  Against the general form it replaced (words rewritten by LUT for every
