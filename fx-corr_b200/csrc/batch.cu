@@ -252,10 +252,8 @@ uint64_t item_len(const Shape& sh, int g, int sms, uint64_t nf, bool exact) {
 // the CTAs less evenly, so they are dealt out here, the longest first, as the
 // tickets will.  1024 sectors of FFT 8192, 32-125 frames: 4600 us a call in parts,
 // 3590 whole, and a fifth of the partials; 256 of FFT 16384, 16-62 frames: 1720 and
-// 1190 us; 64 of them 400 and 480.  What stays in parts among many others pays the
-// items' cost: 1000 sectors of FFT 1024, 628 frames, 3430 us against 3290 with
-// 128-frame items.  (Phased groups, with a quarter of the partials a frame, stay in
-// parts.)
+// 1190 us; 64 of them 400 and 480.  (Phased groups, with a quarter of the partials a
+// frame, stay in parts.)
 constexpr uint64_t kRun = 32;
 bool whole_sectors(const std::vector<Entry>& ents, int g, int ctas) {
   double split = 0.0, shared = 0.0, longest = 0.0, sum = 0.0;  // frames
@@ -283,6 +281,19 @@ bool whole_sectors(const std::vector<Entry>& ents, int g, int ctas) {
     end = std::max(end, t);
   }
   return end < split;
+}
+
+// f32 runs (kRun) that an item of the FFT 1024..4096 kernel takes in a row, each into a
+// partial slot of its own as if it were an item: the ticket, the tables and the
+// first copies are paid once, the sums stay the same.  As many as leave every CTA
+// eight items: 1000 sectors of FFT 1024, 628 frames, 3460 us a call with one run an
+// item, 3245 with four; but 256 of 256-1000 frames 877 with one and 950 with four.
+uint32_t item_runs(const std::vector<Entry>& ents, int g, int ctas) {
+  if (g > BG_4096) return 1;
+  uint64_t runs = 0;
+  for (const Entry& e : ents)
+    if (e.group == g && e.per <= kRun) runs += (e.bs.p.nf + e.per - 1) / e.per;
+  return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(4, runs / (8 * (uint64_t)ctas)));
 }
 
 fxc_status run_batch(fxc_batch* b, fxc_scan* const* scans, const uint8_t* const* r1,
@@ -501,6 +512,9 @@ fxc_status run_batch(fxc_batch* b, fxc_scan* const* scans, const uint8_t* const*
   uint64_t fi = 0, bins = 0, part = 0;
   for (int g = 0; g < kBatchGroups; ++g) {
     hdr.item0[g] = (uint32_t)items.size();
+    const Shape& sh = b->shape[g];
+    const bool ours = (mask & (1u << g)) && !sh.pinned && !b->tuning[g];
+    const uint32_t runs_per_item = ours ? item_runs(ents, g, b->sms * sh.ctas) : 1;
     for (Entry& e : ents) {
       if (e.group != g) continue;
       const uint64_t n = e.bs.p.nf, per = e.per;
@@ -512,10 +526,11 @@ fxc_status run_batch(fxc_batch* b, fxc_scan* const* scans, const uint8_t* const*
       e.bs.fi0 = fi;
       e.bs.bin0 = bins;
       const uint32_t si = (uint32_t)(&e - ents.data());
-      for (uint32_t k = 0; k < nparts; ++k) {
-        const uint64_t f0 = k * per, f1 = std::min(n, f0 + per);
-        for (uint32_t row = 0; row < (g == BG_16384 ? 2u : 1u); ++row)
-          items.push_back(BatchItem{si, row, f0, f1, part + (uint64_t)k * slot});
+      const uint32_t m = per <= kRun ? runs_per_item : 1;
+      for (uint32_t k = 0; k < nparts; k += m) {
+        const uint64_t f0 = k * per, f1 = std::min(n, f0 + m * per);
+        for (uint16_t row = 0; row < (g == BG_16384 ? 2 : 1); ++row)
+          items.push_back(BatchItem{si, row, (uint16_t)(m > 1), f0, f1, part + (uint64_t)k * slot});
       }
       part += (uint64_t)nparts * slot;
       fi += n;

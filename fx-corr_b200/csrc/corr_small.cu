@@ -90,11 +90,11 @@ __device__ __forceinline__ void small_cta_drain(uint8_t* smem) {
 }
 
 // Iterations [it0, it1) (FPC frame pairs each, frames below fend) of the sector
-// described by p, into the f64 partials at part ([4][H]).  Returns false when a
-// bounded wait gave up (the CTA must stop).
+// described by p, into the f64 partials at part ([4][H]; slots: one for every flush).
+// Returns false when a bounded wait gave up (the CTA must stop).
 template <int N, int FPC>
 __device__ __forceinline__ bool small_span(const CorrParams& p, uint64_t it0, uint64_t it1,
-                                           uint64_t fend, double* part, uint8_t* smem,
+                                           uint64_t fend, double* part, bool slots, uint8_t* smem,
                                            uint32_t raw_bytes, SmallCta<N>& c) {
   using L = SmallLayout<N, FPC>;
   constexpr int T1 = N / 16;
@@ -184,13 +184,14 @@ __device__ __forceinline__ bool small_span(const CorrParams& p, uint64_t it0, ui
         if (!(v < 2 ? want_acf : want_xcf) || (!in && (v > 0 || ov_only))) x = 0.f;
         if (v == 3 && !g0) x = -x;  // grid 1: the conjugate was summed
         double* q = part + (size_t)(v == 0 ? colP : (v == 1 ? colS : v)) * H + bin;
-        if (first_flush) *q = 0.0 + (double)x;
+        if (first_flush || slots) *q = 0.0 + (double)x;
         else atomicAdd(q, (double)x);
         acc[i][v] = 0.f;
       }
     }
     first_flush = false;
     since_flush = 0;
+    if (slots) part += 4 * H;
   };
 
   bool ok = true;
@@ -351,8 +352,8 @@ corr_small_kernel(const __grid_constant__ CorrParams p) {
   const uint64_t iters = (p.nf + FPC - 1) / FPC;
   const uint64_t it0 = (blockIdx.x * iters) / gridDim.x;
   const uint64_t it1 = ((blockIdx.x + 1) * iters) / gridDim.x;
-  small_span<N, FPC>(p, it0, it1, p.nf, p.partials + (size_t)blockIdx.x * 4 * H, smem,
-                     p.stage_bytes, c);
+  small_span<N, FPC>(p, it0, it1, p.nf, p.partials + (size_t)blockIdx.x * 4 * H, false,
+                     smem, p.stage_bytes, c);
   small_cta_drain<N, FPC>(smem);
 }
 
@@ -378,7 +379,7 @@ corr_small_batch_kernel(const BatchArgs a, int grp) {
     if (k >= n_items) break;
     const BatchItem w = items[k];
     if (!small_span<N, FPC>(scans[w.scan].p, w.f0 / FPC, (w.f1 + FPC - 1) / FPC, w.f1,
-                            a.partials + w.part, smem, 2u * FPC * N, c))
+                            a.partials + w.part, w.slots != 0, smem, 2u * FPC * N, c))
       break;
   }
   small_cta_drain<N, FPC>(smem);

@@ -173,7 +173,9 @@ enum {
 // Frames [f0, f1) of the sector of scan `scan` (for the two-row kernel, the
 // bins of parity `row`), accumulated into partials + part ([4][H] f64).
 struct BatchItem {
-  uint32_t scan, row;
+  uint32_t scan;
+  uint16_t row;
+  uint16_t slots;  // FFT 1024..4096: every f32 run into a slot of its own, from `part` on
   uint64_t f0, f1;
   uint64_t part;
 };

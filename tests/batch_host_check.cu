@@ -150,9 +150,9 @@ void print_log(bool items) {
     for (int x : l.before) std::printf(" %d", x);
     if (items)
       for (size_t i = 0; i < l.items.size(); ++i)
-        std::printf("\n  item %u %u %llu %llu %llu %u", l.items[i].scan, l.items[i].row,
+        std::printf("\n  item %u %u %llu %llu %llu %u %u", l.items[i].scan, l.items[i].row,
                     (unsigned long long)l.items[i].f0, (unsigned long long)l.items[i].f1,
-                    (unsigned long long)l.items[i].part, l.flush[i]);
+                    (unsigned long long)l.items[i].part, l.items[i].slots, l.flush[i]);
     std::printf("\n");
   }
 }

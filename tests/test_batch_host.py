@@ -64,7 +64,7 @@ def test_longest_items_first(batch):
     assert out["status"] == OK
     for items in groups(out).values():
         lengths = {}
-        for scan, row, f0, f1, part, flush in items:
+        for scan, row, f0, f1, part, slots, flush in items:
             lengths.setdefault(scan, []).append(f1 - f0)
         longest = [max(v) for v in lengths.values()]  # in ticket order
         assert len(set(longest)) > 1 and longest == sorted(longest, reverse=True)
@@ -81,10 +81,10 @@ def test_many_short_sectors_run_whole(batch):
         assert split["status"] == whole["status"] == OK
         (s_items,), (w_items,) = groups(split).values(), groups(whole).values()
         assert len(w_items) == many * rows and len(s_items) > 2 * few * rows
-        assert all(f0 == 0 and f1 == nf for _, _, f0, f1, _, _ in w_items)
-        assert len({part for *_, part, _ in w_items}) == many  # rows share a slot
+        assert all(f0 == 0 and f1 == nf and not slots for _, _, f0, f1, _, slots, _ in w_items)
+        assert len({part for *_, part, _, _ in w_items}) == many  # rows share a slot
         fpc = {1024: 4}.get(fft, 1)
-        lengths = {f1 - f0 for _, _, f0, f1, _, _ in s_items if f1 < nf}
+        lengths = {f1 - f0 for _, _, f0, f1, *_ in s_items if f1 < nf}
         assert lengths == {flush * fpc for *_, flush in w_items} and max(lengths) <= 32
         assert whole["in_use"] < 0.6 * many / few * split["in_use"]
     # sectors whose items have several runs stay split
@@ -108,14 +108,14 @@ def test_no_room_for_every_item(batch, sector, count, budget):
     fft, phased, nf = sector
     free = groups(batch("items", (*sector, 1)))
     fpc = {1024: 4}.get(fft, 1)
-    one_run = max(f1 - f0 for items in free.values() for _, _, f0, f1, _, _ in items) <= 32
+    one_run = max(f1 - f0 for items in free.values() for _, _, f0, f1, *_ in items) <= 32
     seen = 0
     for ln in out["launches"]:
         frames = {}
-        for scan, row, f0, f1, part, flush in ln["items"]:
+        for scan, row, f0, f1, part, slots, flush in ln["items"]:
             frames.setdefault((scan, row), []).append((f0, f1))
             if one_run:
-                assert f1 - f0 <= flush * fpc or (f0, f1) == (0, nf)
+                assert slots or f1 - f0 <= flush * fpc or (f0, f1) == (0, nf)
                 assert flush == next(iter(free.values()))[0][-1]
         for (scan, row), f in frames.items():  # every frame once
             assert [a for a, _ in sorted(f)] == [0] + [b for _, b in sorted(f)][:-1]
@@ -154,4 +154,24 @@ def test_runs_of_a_pinned_shape(batch, fft):
     """With one frame per iteration, whatever the scan's own kernel has, an f32 run is
     32 iterations."""
     (items,) = groups(batch("shape", (fft, 0, 300, 2))).values()
-    assert {(f0 % 64, flush) for _, _, f0, _, _, flush in items} == {(0, 32)}
+    assert {(f0 % 64, slots, flush) for _, _, f0, _, _, slots, flush in items} == {(0, 0, 32)}
+
+
+def test_several_runs_an_item(batch):
+    """Where the runs of FFT 1024..4096 are many, an item takes up to four in a row, each
+    with the slot it has as an item of its own."""
+    for fft, nf, many in ((1024, 300, 891), (2048, 130, 900), (4096, 150, 350)):
+        (few,) = groups(batch("items", (fft, 0, nf, 1))).values()
+        (items,) = groups(batch("items", (fft, 0, nf, many))).values()
+        h = fft // 2 + 1
+        run = few[0][3] - few[0][2]
+        assert len(few) < len(items) < many * len(few)
+        slots = {}
+        for scan, row, f0, f1, part, own, flush in items:
+            assert own and f0 % run == 0 and f1 - f0 <= 4 * run and flush == few[0][-1]
+            for k in range(-(-(f1 - f0) // run)):
+                slots.setdefault(scan, []).append((f0 + k * run, part + k * 4 * h))
+        assert len(slots) == many
+        for v in slots.values():  # the slots that single-run items have, in frame order
+            base = min(p for _, p in v)
+            assert sorted(v) == [(k * run, base + k * 4 * h) for k in range(len(few))]

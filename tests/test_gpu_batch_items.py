@@ -64,11 +64,12 @@ def test_short_sector_items(engine, fxc_lib, scale):
 
 
 @pytest.mark.parametrize("fft,nf,many", [(1024, 70, 2070), (2048, 100, 1182), (4096, 75, 591),
-                                         (8192, 33, 294), (8192, 101, 294), (16384, 21, 147)])
+                                         (8192, 33, 294), (8192, 101, 294), (16384, 21, 147),
+                                         (1024, 300, 891), (2048, 130, 900), (4096, 150, 350)])
 def test_short_sector_alone_and_among_many(engine, fxc_lib, fft, nf, many):
     """A short sector runs in parts where it is alone and whole among many (so many that
-    they fill the CTAs of 148 SMs evenly): the same sums bit for bit, ragged last run
-    included."""
+    they fill the CTAs of 148 SMs evenly), or, where they do not, in items of several
+    runs: the same sums bit for bit, ragged last run included."""
     import torch
 
     scans = []
